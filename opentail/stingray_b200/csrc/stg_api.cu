@@ -14,6 +14,7 @@
 #include "stg_flat.cuh"
 #include "stg_handle.h"
 #include "stg_launch.h"
+#include "stg_row.cuh"
 #include "stg_types.h"
 
 using namespace stg;
@@ -260,9 +261,9 @@ int make_plan(StgHandle h, const StgSampleBatch *b, int mode, bool shard, int gl
     for (int r = 0; r < rows; r++)
         if (pl.rows[r].n_chunks == 0) pl.items.push_back({r, -1});
     pl.n_row_items = (int)pl.items.size();
-    // The full-vocabulary rows join the flat step when every one of them can: no top-k on this path
-    // (it only arises together with a logit bias), a vocabulary the segment-parallel sum emulation
-    // covers, and room in the workspace.
+    // The full-vocabulary rows are done by clusters (stg_row.cu) when every one of them can: no top-k on this
+    // path (it only arises together with a logit bias), a vocabulary the tile summaries cover, and room in
+    // the workspace.
     pl.flat_full = full_ok && pl.n_row_items > 0 && pl.n_row_items <= h->full_cap && V <= kSub * kMaxSubTiles;
     for (int i = 0; i < pl.n_row_items && pl.flat_full; i++) {
         const RowPlan &rp = pl.rows[pl.items[i].row];
@@ -395,7 +396,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
                          ((b->mem_flags & STG_MEM_HOST_LOGITS) || ((uintptr_t)b->logits % need0) == 0);
     const bool flat_ok = mode == 0 && x.shard_mode != 2 && aligned && !getenv("STG_NO_FLAT") &&
                          !(x.shard_mode == 1 && getenv("STG_NO_FLAT_SHARD"));
-    const bool full_ok = (mode == 0 || mode == 2) && x.shard_mode == 0 && aligned && !getenv("STG_NO_FLAT") && !getenv("STG_NO_FLAT_FULL");
+    const bool full_ok = x.shard_mode == 0 && !getenv("STG_NO_FLAT") && !getenv("STG_NO_FLAT_FULL");
     // The plan depends on the batch description only (never on the logits): a decode loop that
     // repeats a description byte for byte reuses the plan of the previous call as it is.
     std::vector<unsigned char> &key = h->plan_key_scratch;
@@ -545,23 +546,16 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         return STG_OK;
     }
     // Row items are the full-vocabulary rows (and greedy rows with penalties), chunk items the rows
-    // of the top-k path and plain greedy rows.  In the flat form (stg_flat.cuh) ONE streaming kernel
-    // reads every row of both kinds from HBM; after it the per-row finish of the chunked rows runs on
-    // a side stream beside the phases of the full rows.  Rows the flat form does not take run in the
-    // two persistent kernels of the first design, again side by side.
+    // of the top-k path and plain greedy rows.  The former run as clusters of CTAs (stg_row.cu), the latter in
+    // the flat form (stg_flat.cuh), side by side; what neither takes runs in the two persistent kernels of
+    // the first design.
     const int n_rows_items = pl.n_row_items, n_chunk_items = (int)pl.items.size() - pl.n_row_items;
     cudaError_t e = cudaSuccess;
     const bool both = n_rows_items > 0 && n_chunk_items > 0;
     int launches = 0;
     int row_grid = 0;
     FlatRow *fr = (FlatRow *)h->flat_rows.p;
-    FullWs ws;
-    memset(&ws, 0, sizeof(ws));
-    ws.rows = (FullRow *)h->fw_rows.p; ws.e = (float *)h->fw_e.p; ws.e_stride = h->escratch_stride;
-    ws.ov_id = (int32_t *)h->fw_ov_id.p; ws.ov_adj = (float *)h->fw_ov_adj.p; ws.ew = (Emul2Work *)h->fw_ew.p;
-    ws.hist = (unsigned long long *)h->fw_hist.p; ws.bstart = (uint32_t *)h->fw_bstart.p;
-    ws.bin_exp = (unsigned char *)h->fw_binexp.p; ws.flag_bits = (uint32_t *)h->fw_flagbits.p;
-    ws.cursor = (uint32_t *)h->fw_cursor.p; ws.keys = (uint32_t *)h->fw_keys.p; ws.key_stride = h->key_stride;
+    const RowWs rw{(float *)h->fw_e.p, h->escratch_stride, (int32_t *)h->fw_redo.p};
     const bool flat_chunks = pl.flat && n_chunk_items > 0, flat_full = pl.flat_full && n_rows_items > 0;
     auto launch_rows_kernel = [&](bool redo_only, cudaStream_t on) {
         SampleArgs r = a;
@@ -569,7 +563,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         r.item_base = 0;
         r.work_counter = (uint32_t *)h->work_counter.p + 1;
         r.work_base = h->work_base_rows;
-        if (redo_only) { r.redo_flags = &ws.rows[0].redo; r.redo_stride = (int32_t)(sizeof(FullRow) / 4); r.static_items = 1; }
+        if (redo_only) { r.redo_flags = rw.redo; r.redo_stride = 1; r.static_items = 1; }
         row_grid = std::min(n_rows_items, h->sm_count);
         cudaError_t er = launch_sample_rows(r, row_grid, on);
         if (er == cudaSuccess) { if (!redo_only) h->work_base_rows += (uint32_t)n_rows_items + (uint32_t)row_grid; launches++; }
@@ -595,35 +589,9 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         h->kt.mark("greedy_step", stream);
         return;
     }
-    if (flat_chunks || flat_full) {
-        if (flat_chunks && !flat_full) { e = launch_flat_prep(c, fr, stream); launches++; h->kt.mark("flat_prep", stream); }
-        if (e == cudaSuccess && flat_full) { e = launch_full_prep(a, ws, flat_chunks ? fr : nullptr, stream); launches++; h->kt.mark("full_prep", stream); }
-        // The HBM pass: the full-vocabulary rows (first in the item list) by the general kernel, the
-        // others by a kernel of their own that needs fewer registers and keeps more warps resident.
-        static const bool one_stream_pass = getenv("STG_ONE_STREAM_PASS") != nullptr;
-        if (one_stream_pass) {
-            if (e == cudaSuccess) { e = launch_flat_stream(a, fr, ws, stream); launches++; h->kt.mark("flat_stream", stream); }
-        } else if (flat_full && flat_chunks) {
-            // both kinds: the full rows' pass on the caller's stream, where their phases follow at once; the
-            // others' pass on the side stream beside the first of those phases (the exp pass is bound by
-            // arithmetic, this one by HBM, and the full rows' chain is the longer one)
-            static const bool serial_passes = getenv("STG_SERIAL_PASSES") != nullptr;
-            cudaStream_t cs = serial_passes ? stream : h->aux_stream;
-            SampleArgs af = a;
-            af.n_items = n_rows_items;
-            if (e == cudaSuccess && !serial_passes) e = cudaEventRecord(h->ev_fork, stream);
-            if (e == cudaSuccess && !serial_passes) e = cudaStreamWaitEvent(h->aux_stream, h->ev_fork, 0);
-            if (e == cudaSuccess) { e = launch_flat_stream(af, fr, ws, stream); launches++; h->kt.mark("flat_stream_full_rows", stream); }
-            if (e == cudaSuccess) { e = launch_flat_stream_chunks(c, fr, cs); launches++; if (serial_passes) h->kt.mark("flat_stream_chunks", stream); }
-        } else if (flat_full) {
-            if (e == cudaSuccess) { e = launch_flat_stream(a, fr, ws, stream); launches++; h->kt.mark("flat_stream", stream); }
-        } else {
-            if (e == cudaSuccess) { e = launch_flat_stream_chunks(c, fr, stream); launches++; h->kt.mark("flat_stream_chunks", stream); }
-        }
-    }
-    const bool flat_rows = flat_full && n_rows_items > 0;
-    const bool fork = both || flat_rows;  // the redo pass of the flat full rows runs on the side stream too
-    if (e == cudaSuccess && fork) {
+    // both kinds of rows: the chunked ones on the side stream
+    const bool fork = both;
+    if (fork) {
         e = cudaEventRecord(h->ev_fork, stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(h->aux_stream, h->ev_fork, 0);
     }
@@ -632,26 +600,30 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         if (e != cudaSuccess || n_chunk_items == 0) return;
         cudaStream_t cs = fork ? h->aux_stream : stream;
         if (flat_chunks) {
-            // beside the full rows' one-SM-per-row kernels the finish must not take every SM
-            const int sms = flat_rows ? std::max(8, h->sm_count - std::min(n_rows_items, h->sm_count) - 4) : h->sm_count;
+            e = launch_flat_prep(c, fr, cs);
+            launches++;
+            if (!fork) h->kt.mark("flat_prep", cs);
+            if (e == cudaSuccess) { e = launch_flat_stream_chunks(c, fr, cs); launches++; }
+            if (!fork) h->kt.mark("flat_stream_chunks", cs);
+            if (e != cudaSuccess) return;
+            const int sms = h->sm_count;
             c.item_base = n_rows_items;  // diagnostic stamps: behind the full rows' slots
             static const bool no_small = getenv("STG_NO_SMALL_FINISH") != nullptr;
             // Smaller CTAs, several per SM, shorten the finish as long as all rows are in flight at once: the
             // phases of a row are short and barrier-separated, so a 1024-thread CTA leaves most of its SM
             // idle, but per row the smaller forms do more work (measured on 2048 rows: 577 us with 256
             // threads against 304 us with 1024).  So: 512 threads, two per SM, up to 2 rows per SM; 256
-            // threads, four per SM, up to 4 rows per SM (not beside the one-SM CTAs of full rows, which
-            // need whole SMs to come free); beyond that one full-size CTA per row.  The smaller forms also
+            // threads, four per SM, up to 4 rows per SM; beyond that one full-size CTA per row.  The smaller forms also
             // need their shorter buffers to hold a row's N best and one batch of its list.
             constexpr int kHalfCap = 6912, kQuarterCap = 3456;  // 2 x 110,592 B, 4 x 55,296 B (+ static) fit an SM
             if (!no_small && n_chunk_items <= 2 * sms && pl.max_sel + 2048 + 512 <= kHalfCap) {
                 c.finish_cap = kHalfCap;
                 e = launch_flat_finish_half(c, fr, n_chunk_items, cs);
-            } else if (!no_small && !flat_rows && n_chunk_items <= 4 * sms && pl.max_sel + 1024 + 512 <= kQuarterCap) {
+            } else if (!no_small && n_chunk_items <= 4 * sms && pl.max_sel + 1024 + 512 <= kQuarterCap) {
                 c.finish_cap = kQuarterCap;
                 e = launch_flat_finish_quarter(c, fr, n_chunk_items, cs);
             } else {
-                e = launch_flat_finish(c, fr, std::min(n_chunk_items, flat_rows ? sms : n_chunk_items), pl.smem, cs);
+                e = launch_flat_finish(c, fr, n_chunk_items, pl.smem, cs);
             }
             if (e == cudaSuccess) launches++;
             if (!fork) h->kt.mark("flat_finish", cs);
@@ -663,26 +635,17 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
             if (e == cudaSuccess) { h->work_base += (uint32_t)n_chunk_items + (uint32_t)grid; launches++; }
         }
     };
-    if (flat_rows) {
-        // Main stream: the phases of the full rows (their plan and scatter kernels on a stream of their
-        // own beside the walk).  Side stream: the finish of the chunked rows - held back until the scatter
-        // pass is through, because its one-SM CTAs would otherwise sit on the SMs that pass needs while
-        // the walk holds the others, whereas the cut that follows leaves two thirds of the GPU idle -
-        // and behind it, once the last kernel that can give a row up (the draw's partial sums) is through,
-        // the row kernel for exactly the rows the flat form gave up (every other CTA of it leaves at
-        // once), beside the draw.
-        if (!flat_chunks) launch_chunked();
-        const FullSide side{h->plan_stream, h->ev_exp, h->ev_scatter, pl.n_full_without_top_p > 0, pl.n_full_with_top_p > 0};
-        if (e == cudaSuccess) e = launch_full_rest(a, ws, a.items, n_rows_items, &launches, &h->kt, stream, 0, side);
-        if (flat_chunks) {
-            if (e == cudaSuccess && side.any_with_top_p) e = cudaStreamWaitEvent(h->aux_stream, h->ev_scatter, 0);
-            launch_chunked();
-        }
-        if (e == cudaSuccess) e = launch_full_rest(a, ws, a.items, n_rows_items, &launches, &h->kt, stream, 1, side);
-        if (e == cudaSuccess) e = cudaEventRecord(h->ev_cut, stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->aux_stream, h->ev_cut, 0);
-        if (e == cudaSuccess) e = launch_rows_kernel(true, h->aux_stream);
-        if (e == cudaSuccess) e = launch_full_rest(a, ws, a.items, n_rows_items, &launches, &h->kt, stream, 2, side);
+    if (flat_full) {
+        // the full rows by one cluster of CTAs each (stg_row.cu), then the row kernel for exactly the rows that gave up
+        // (every other CTA of it leaves at once)
+        SampleArgs af = a;
+        af.n_items = n_rows_items;
+        e = launch_row_clusters(af, rw, mode == 2 && x.want_argmax, stream);
+        launches++;
+        h->kt.mark("row_clusters", stream);
+        launch_chunked();
+        if (e == cudaSuccess) e = launch_rows_kernel(true, stream);
+        h->kt.mark("row_redo", stream);
     } else {
         if (e == cudaSuccess && n_rows_items > 0) {
             e = launch_rows_kernel(false, stream);
@@ -790,8 +753,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
 // every device buffer a handle owns
 std::vector<DevBuf *> all_buffers(StgHandle h)
 {
-    return {&h->plan_dev, &h->flat_rows, &h->fw_rows, &h->fw_e, &h->fw_keys, &h->fw_ov_id, &h->fw_ov_adj, &h->fw_ew, &h->fw_hist,
-            &h->fw_bstart, &h->fw_binexp, &h->fw_flagbits, &h->fw_cursor, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
+    return {&h->plan_dev, &h->flat_rows, &h->fw_redo, &h->fw_rows, &h->fw_e, &h->fw_ew, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
             &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
             &h->st_mask, &h->st_logits, &h->o_tokens, &h->o_probs, &h->o_flags, &h->o_topk_ids, &h->o_topk_vals, &h->o_topk_probs,
             &h->o_pairs, &h->ticks, &h->ring_ids, &h->ring_len_dev, &h->mc_words, &h->mc_slots, &h->sp_draft, &h->sp_uniforms,
@@ -836,7 +798,7 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
     const size_t R = (size_t)cfg->max_rows, V = (size_t)cfg->max_vocab;
     const size_t sel_max = std::max<size_t>(1, (size_t)cfg->max_top_k + cfg->max_history);
     h->cand_entries = R * std::max<size_t>({8 * sel_max, sel_max + (size_t)kFlatSlack, (size_t)64});
-    h->escratch_stride = (int64_t)round_up(V + 8, 64);
+    h->escratch_stride = (int64_t)round_up(V + 8, kSub);  // whole tiles (stg_row.cu)
     h->key_stride = (int64_t)round_up(V + 8, 64);
     h->plan_bytes_cap = round_up(R * sizeof(RowPlan), 256) + round_up((R * 65) * sizeof(WorkItem), 256) +
                         round_up(R * kPowTab * sizeof(float), 256) + 1024;
@@ -848,21 +810,15 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
     A(h->tickets, R * 4);
     A(h->flat_rows, R * sizeof(FlatRow));
     {
-        // full-vocabulary rows of the flat step (FullWs): per row the exp values and the candidate keys
-        // (4 bytes per token each), the histogram and its plan, the override list, the sub-tile summaries
+        // full-vocabulary rows: per row its exp values (stg_row.cu); for the speculative draws the sub-tile summaries
         h->full_cap = (int)std::min<size_t>(R, 1024);
         const size_t F = (size_t)h->full_cap;
-        A(h->fw_rows, F * sizeof(FullRow));
+        A(h->fw_redo, F * 4);
         A(h->fw_e, F * (size_t)h->escratch_stride * 4);
-        A(h->fw_keys, F * (size_t)h->key_stride * 4);
-        A(h->fw_ov_id, F * kMaxOverride * 4);
-        A(h->fw_ov_adj, F * kMaxOverride * 4);
-        A(h->fw_ew, F * sizeof(Emul2Work));
-        A(h->fw_hist, F * kHistBins * 8);
-        A(h->fw_bstart, F * kHistBins * 4);
-        A(h->fw_binexp, F * kHistBins);
-        A(h->fw_flagbits, F * (kHistBins / 32) * 4);
-        A(h->fw_cursor, F * kHistBins * 4);
+        if (cfg->max_spec_draft > 0) {
+            A(h->fw_rows, F * sizeof(FullRow));
+            A(h->fw_ew, F * sizeof(Emul2Work));
+        }
     }
     A(h->work_counter, 256);
     A(h->escratch, (size_t)h->sm_count * h->escratch_stride * 4);
@@ -916,10 +872,6 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_order, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_cut, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_exp, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_scatter, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&h->plan_stream, cudaStreamNonBlocking, hi);
         if (e != cudaSuccess) rc = cuda_fail(nullptr, e, "side stream");
     }
     for (int i = 0; i < 4 && rc == STG_OK; i++) {
@@ -955,10 +907,6 @@ int stg_destroy(StgHandle h)
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
     if (h->ev_order) cudaEventDestroy(h->ev_order);
-    if (h->ev_cut) cudaEventDestroy(h->ev_cut);
-    if (h->ev_exp) cudaEventDestroy(h->ev_exp);
-    if (h->ev_scatter) cudaEventDestroy(h->ev_scatter);
-    if (h->plan_stream) cudaStreamDestroy(h->plan_stream);
     if (h->aux_stream) cudaStreamDestroy(h->aux_stream);
     delete h;
     return STG_OK;

@@ -122,7 +122,7 @@ __device__ __forceinline__ void lane_composite(const float x[8], int eb, int &a0
 __device__ __forceinline__ int exp_of_double(double v)
 {
     if (!(v > 0.0)) return 1;
-    int e = ilogb(v) + 127;
+    const int e = ((__double2hiint(v) >> 20) & 2047) - 1023 + 127;  // floor(log2 v) + 127; subnormals clamp below
     return e < 1 ? 1 : (e > 254 ? 254 : e);
 }
 

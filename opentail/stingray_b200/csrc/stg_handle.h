@@ -79,8 +79,8 @@ struct StgSampler_ {
     const stg::WorkItem *d_items = nullptr;
     const float *d_pow = nullptr;
     stg::DevBuf flat_rows;               // FlatRow per row (stg_flat.cuh)
-    // full-vocabulary rows of the flat step: FullWs arrays for up to full_cap rows
-    stg::DevBuf fw_rows, fw_e, fw_ov_id, fw_ov_adj, fw_ew, fw_hist, fw_bstart, fw_binexp, fw_flagbits, fw_cursor, fw_keys;
+    // full-vocabulary rows: RowWs (stg_row.cuh) and FullWs (stg_flat.cuh) arrays for up to full_cap rows
+    stg::DevBuf fw_redo, fw_rows, fw_e, fw_ew;
     int full_cap = 0;
     stg::DevBuf cand, cand_count, tickets, work_counter, escratch, keyscratch, listscratch, dists;
     stg::DevBuf st_hist, st_bias_ids, st_bias_vals, st_uniforms, st_mask, st_logits;
@@ -92,9 +92,8 @@ struct StgSampler_ {
     int64_t escratch_stride = 0, key_stride = 0;
     size_t cand_entries = 0;
     uint32_t work_base = 0, work_base_rows = 0;
-    cudaStream_t aux_stream = nullptr;   // lowest priority: the chunked rows' finish runs here, beside the full rows' phases
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_cut = nullptr, ev_exp = nullptr, ev_scatter = nullptr;
-    cudaStream_t plan_stream = nullptr;  // the plan and scatter kernels of the full rows, beside the walk
+    cudaStream_t aux_stream = nullptr;   // lowest priority: the chunked rows run here, beside the full rows
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_order = nullptr;      // orders a call behind the previous call's work when the stream changes
     cudaStream_t last_stream = nullptr;
     bool last_stream_valid = false;
@@ -135,6 +134,7 @@ struct BatchExtra {
     int shard_mode = 0;           // 1: export each row's local candidates to the exchange buffer
     int vocab_offset = 0;
     int global_vocab = 0;         // 0: same as the batch's vocab
+    bool want_argmax = false;     // mode 2: the arg-max of the raw rows goes with the descriptors
 };
 int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *stream);
 int stage_in(StgHandle h, const void *src, size_t bytes, bool on_host, DevBuf &stage, cudaStream_t stream,

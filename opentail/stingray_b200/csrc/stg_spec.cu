@@ -141,6 +141,7 @@ int stg_spec_verify(StgHandle h, const StgSpecBatch *b, void *stream_)
         BatchExtra x;
         x.mode = 2;
         x.dists_out = which == 0 ? tdist : ddist;
+        x.want_argmax = b->mode == 1;  // the looser accept rule compares against it
         int rc = run_batch(h, &sb, x, stream);
         if (rc) return rc;
     }
