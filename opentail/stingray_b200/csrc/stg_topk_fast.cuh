@@ -5,8 +5,7 @@
 // also runs the softmax, the filters and the draw of Sampler.cs:296-349.  The radix selection it stands in
 // for crosses two block barriers per digit and ranks ties against the whole list: on 96 rows of bf16 logits
 // (which tie in droves) with 256-token histories the finish took 70 us and takes 27, a lone row's step of
-// 151,936 logits went from 25 to 19 us.  Bound: latency of a few dozen dependent shuffles, and fetching
-// instructions: the stages run in loops, as a CTA runs through this once.
+// 151,936 logits went from 25 to 19 us.  Bound: latency of a few dozen dependent shuffles.
 //
 // The row's order is (penalised value descending, raw order among equals).  Keys hold the penalised value, a
 // bit that says a penalty lowered it - its raw logit was higher than those of its equals that none did, so it
@@ -29,38 +28,40 @@ struct FastShared {
 
 __device__ __forceinline__ int fast_idx(u64 k) { return (int)(0x7FFFFFFFu - ((uint32_t)k & 0x7FFFFFFFu)); }
 
-// steps j0 .. 1 of stage k of a bitonic sort (descending) of 32 * KPL keys; key i is r[i / 32] of lane i % 32
+// steps j0 .. 1 of stage k of a bitonic sort (descending) of 32 * KPL keys; key i is r[i / 32] of lane i % 32.
+// Unrolled: in loops the same steps made a lone row's step 21.5 us instead of 18.8.
 template <int KPL>
 __device__ __forceinline__ void warp_steps(u64 (&r)[KPL], int k, int j0)
 {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int dj = KPL / 2; dj > 0; dj >>= 1) {
-        if (dj * 32 > j0) continue;
+    for (int j = 16 * KPL; j > 0; j >>= 1) {
+        if (j > j0) continue;
+        if (j >= 32) {
+            const int dj = j / 32;
 #pragma unroll
-        for (int q = 0; q < KPL; q++) {
-            if ((q & dj) == 0) {
-                const bool desc = ((q * 32 + lane) & k) == 0;
-                const u64 x = r[q], y = r[q | dj];
-                if ((x < y) == desc) { r[q] = y; r[q | dj] = x; }
+            for (int q = 0; q < KPL; q++) {
+                if ((q & dj) == 0) {
+                    const bool desc = ((q * 32 + lane) & k) == 0;
+                    const u64 x = r[q], y = r[q | dj];
+                    if ((x < y) == desc) { r[q] = y; r[q | dj] = x; }
+                }
             }
-        }
-    }
-#pragma unroll 1
-    for (int j = min(j0, 16); j > 0; j >>= 1) {
-        const bool lower = (lane & j) == 0;
+        } else {
+            const bool lower = (lane & j) == 0;
 #pragma unroll
-        for (int q = 0; q < KPL; q++) {
-            const bool desc = ((q * 32 + lane) & k) == 0;
-            const u64 o = __shfl_xor_sync(0xFFFFFFFFu, r[q], j);
-            if ((o > r[q]) == (lower == desc)) r[q] = o;  // keys are distinct, or zeros that pad
+            for (int q = 0; q < KPL; q++) {
+                const bool desc = ((q * 32 + lane) & k) == 0;
+                const u64 o = __shfl_xor_sync(0xFFFFFFFFu, r[q], j);
+                r[q] = (lower == desc) ? (r[q] > o ? r[q] : o) : (r[q] < o ? r[q] : o);
+            }
         }
     }
 }
 template <int KPL>
 __device__ __forceinline__ void warp_sort(u64 (&r)[KPL])
 {
-#pragma unroll 1
+#pragma unroll
     for (int k = 2; k <= 32 * KPL; k <<= 1) warp_steps<KPL>(r, k == 32 * KPL ? 1 << 30 : k, k >> 1);
 }
 // r = the best keys of r and of another descending list given reversed: rev[q] holds key 32 * KPL - 1 - (32 q + lane)
@@ -73,7 +74,7 @@ __device__ __forceinline__ void warp_best(u64 (&r)[KPL], const u64 (&rev)[KPL])
 }
 
 // o[i] = fl(o[i - 1] + x[i]) from 0 for i < m (a multiple of 8); one warp, returns the last
-static __device__ __noinline__ float warp_prefix_serial(const float *x, float *o, int m)
+__device__ __forceinline__ float warp_prefix_serial(const float *x, float *o, int m)
 {
     const int lane = threadIdx.x & 31;
     float acc = 0.f;
@@ -95,7 +96,7 @@ static __device__ __noinline__ float warp_prefix_serial(const float *x, float *o
 
 // What is left of the row for one warp: softmax over the k ordered candidates, min-p, top-p, the draw
 // (Sampler.cs:296-349; every fp32 operation as in finish_topk_draw).  vals / ids [k] are in `fs`.
-static __device__ __noinline__ void fast_draw(FastShared &fs, const RowPlan &rp, float uniform, FinishOut *out)
+__device__ __forceinline__ void fast_draw(FastShared &fs, const RowPlan &rp, float uniform, FinishOut *out)
 {
     const int lane = threadIdx.x & 31, k = rp.top_k, k8 = (k + 7) & ~7;
     const float inv_t = rp.temperature == 1.0f ? 1.0f : __fdiv_rn(1.0f, rp.temperature);
@@ -164,7 +165,7 @@ __device__ __forceinline__ bool fast_eligible(const RowPlan &rp, int cnt, size_t
 }
 
 // occurrences in the history | inside the window << 16
-static __device__ __noinline__ unsigned fast_occurrences(const int *hkey, const unsigned *hcnt, int hmask, int id)
+__device__ __forceinline__ unsigned fast_occurrences(const int *hkey, const unsigned *hcnt, int hmask, int id)
 {
     int h = (int)(((unsigned)id * 2654435761u) >> 7) & hmask;
 #pragma unroll 1
@@ -176,7 +177,7 @@ static __device__ __noinline__ unsigned fast_occurrences(const int *hkey, const 
     }
 }
 // the key of a candidate with the penalties applied (Sampler.cs:263-287)
-static __device__ __noinline__ u64 fast_penalise(u64 key, const int *hkey, const unsigned *hcnt, int hmask, const RowPlan &rp, const float *pow_tab)
+__device__ __forceinline__ u64 fast_penalise(u64 key, const int *hkey, const unsigned *hcnt, int hmask, const RowPlan &rp, const float *pow_tab)
 {
     if (key == 0ull) return key;
     key &= 0xFFFFFFFF7FFFFFFFull;
@@ -212,8 +213,7 @@ __device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, i
 #pragma unroll
     for (int q = 0; q < KPL; q++) {
         const int i = warp * K2 + q * 32 + lane;
-        nx[q] = i < cnt ? __ldcg(list + i) : 0ull;  // in flight while the history is hashed
-        r[q] = 0ull;
+        r[q] = i < cnt ? __ldcg(list + i) : 0ull;  // in flight while the history is hashed
     }
     if (tid == 0) fs.fail = 0;
     if (pen) {
@@ -236,8 +236,18 @@ __device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, i
         __syncthreads();
     }
     const int lists = (cnt + K2 - 1) / K2;
+    if (pen) {
+#pragma unroll
+        for (int q = 0; q < KPL; q++) r[q] = fast_penalise(r[q], hkey, hcnt, hslots - 1, rp, pow_tab);
+    }
+    warp_sort<KPL>(r);
 #pragma unroll 1
-    for (int l = warp; l < lists; l += W) {
+    for (int l = warp + W; l < lists; l += W) {
+#pragma unroll
+        for (int q = 0; q < KPL; q++) {
+            const int i = l * K2 + q * 32 + lane;
+            nx[q] = i < cnt ? __ldcg(list + i) : 0ull;
+        }
         if (pen) {
 #pragma unroll
             for (int q = 0; q < KPL; q++) nx[q] = fast_penalise(nx[q], hkey, hcnt, hslots - 1, rp, pow_tab);
@@ -247,11 +257,6 @@ __device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, i
 #pragma unroll
         for (int q = 0; q < KPL; q++) rev[q] = __shfl_xor_sync(0xFFFFFFFFu, nx[KPL - 1 - q], 31);
         warp_best<KPL>(r, rev);
-#pragma unroll
-        for (int q = 0; q < KPL; q++) {
-            const int i = (l + W) * K2 + q * 32 + lane;
-            nx[q] = i < cnt ? __ldcg(list + i) : 0ull;
-        }
     }
 #pragma unroll 1
     for (int w = W / 2; w > 0; w >>= 1) {
