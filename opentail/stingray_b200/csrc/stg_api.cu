@@ -282,9 +282,9 @@ int make_plan(StgHandle h, const StgSampleBatch *b, int mode, bool shard, int gl
 }
 
 // Uploads the plan unless it is byte-identical to the one already resident on the device.
-int upload_plan(StgHandle h, const Plan &pl, cudaStream_t stream, const RowPlan **d_rows,
-                const WorkItem **d_items, const float **d_pow)
+int upload_plan(StgHandle h, PlanSlot &ps, cudaStream_t stream)
 {
+    const Plan &pl = ps.plan;
     const size_t b_rows = round_up(pl.rows.size() * sizeof(RowPlan), 256);
     const size_t b_items = round_up(pl.items.size() * sizeof(WorkItem), 256);
     const size_t b_pow = round_up(pl.pow_tab.size() * sizeof(float), 256);
@@ -294,11 +294,11 @@ int upload_plan(StgHandle h, const Plan &pl, cudaStream_t stream, const RowPlan 
     memcpy(bytes.data(), pl.rows.data(), pl.rows.size() * sizeof(RowPlan));
     memcpy(bytes.data() + b_rows, pl.items.data(), pl.items.size() * sizeof(WorkItem));
     if (!pl.pow_tab.empty()) memcpy(bytes.data() + b_rows + b_items, pl.pow_tab.data(), pl.pow_tab.size() * sizeof(float));
-    unsigned char *dev = (unsigned char *)h->plan_dev.p;
-    *d_rows = (const RowPlan *)dev;
-    *d_items = (const WorkItem *)(dev + b_rows);
-    *d_pow = pl.pow_tab.empty() ? nullptr : (const float *)(dev + b_rows + b_items);
-    if (bytes == h->plan_cache) return STG_OK;
+    unsigned char *dev = (unsigned char *)ps.dev.p;
+    ps.d_rows = (const RowPlan *)dev;
+    ps.d_items = (const WorkItem *)(dev + b_rows);
+    ps.d_pow = pl.pow_tab.empty() ? nullptr : (const float *)(dev + b_rows + b_items);
+    if (bytes == ps.cache) return STG_OK;
     const int slot = h->plan_slot;
     h->plan_slot = (slot + 1) & 3;
     CK(cudaEventSynchronize(h->plan_ev[slot]));
@@ -306,7 +306,7 @@ int upload_plan(StgHandle h, const Plan &pl, cudaStream_t stream, const RowPlan 
     memcpy(pin, bytes.data(), total);
     CK(cudaMemcpyAsync(dev, pin, total, cudaMemcpyHostToDevice, stream));
     CK(cudaEventRecord(h->plan_ev[slot], stream));
-    h->plan_cache.swap(bytes);
+    ps.cache.swap(bytes);
     h->stats.plan_uploads++;
     return STG_OK;
 }
@@ -413,20 +413,21 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     } else if (b->history_offsets) put(b->history_offsets, (size_t)(rows + 1) * 4);
     if (b->bias_offsets) put(b->bias_offsets, (size_t)(rows + 1) * 4);
     if (b->row_uses_mask) put(b->row_uses_mask, (size_t)rows);
-    Plan &pl = h->plan;
-    if (!h->plan_valid || key != h->plan_key) {
-        h->plan_valid = false;
+    PlanSlot &ps = h->plans[x.plan_slot];
+    Plan &pl = ps.plan;
+    if (!ps.valid || key != ps.key) {
+        ps.valid = false;
         pl = Plan();
         rc = make_plan(h, b, mode, x.shard_mode != 0, x.global_vocab, flat_ok, full_ok, pl);
         if (rc) return rc;
         if (pl.smem > h->smem_optin || kRowArenaBytes > h->smem_optin) return fail(h, STG_ERR_CAPACITY, "shared memory needed exceeds the device limit");
-        rc = upload_plan(h, pl, stream, &h->d_rows, &h->d_items, &h->d_pow);
+        rc = upload_plan(h, ps, stream);
         if (rc) return rc;
-        h->plan_key = key;
-        h->plan_valid = true;
-        h->plan_version++;
+        ps.key = key;
+        ps.valid = true;
+        ps.version = ++h->plan_version;
     }
-    const RowPlan *d_rows = h->d_rows; const WorkItem *d_items = h->d_items; const float *d_pow = h->d_pow;
+    const RowPlan *d_rows = ps.d_rows; const WorkItem *d_items = ps.d_items; const float *d_pow = ps.d_pow;
 
     SampleArgs a;
     memset(&a, 0, sizeof(a));
@@ -666,7 +667,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         !h->kt.on && a.phase_ticks == nullptr) {
         std::vector<unsigned char> &gk = h->plan_key_scratch;  // free again: the plan key has been compared
         gk.assign((const unsigned char *)&a, (const unsigned char *)&a + sizeof(a));
-        const uint64_t extra[3] = {h->plan_version, (uint64_t)(uintptr_t)stream, (uint64_t)mode};
+        const uint64_t extra[3] = {ps.version, (uint64_t)(uintptr_t)stream, (uint64_t)mode};
         gk.insert(gk.end(), (const unsigned char *)extra, (const unsigned char *)extra + sizeof(extra));
         uint64_t hash = 1469598103934665603ull;
         for (unsigned char ch : gk) hash = (hash ^ ch) * 1099511628211ull;
@@ -753,7 +754,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
 // every device buffer a handle owns
 std::vector<DevBuf *> all_buffers(StgHandle h)
 {
-    return {&h->plan_dev, &h->flat_rows, &h->fw_redo, &h->fw_rows, &h->fw_e, &h->fw_ew, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
+    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
             &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
             &h->st_mask, &h->st_logits, &h->o_tokens, &h->o_probs, &h->o_flags, &h->o_topk_ids, &h->o_topk_vals, &h->o_topk_probs,
             &h->o_pairs, &h->ticks, &h->ring_ids, &h->ring_len_dev, &h->mc_words, &h->mc_slots, &h->sp_draft, &h->sp_uniforms,
@@ -804,21 +805,18 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
                         round_up(R * kPowTab * sizeof(float), 256) + 1024;
     int rc = STG_OK;
     auto A = [&](DevBuf &b, size_t bytes) { if (rc == STG_OK) rc = dev_alloc(h, b, bytes); };
-    A(h->plan_dev, h->plan_bytes_cap);
+    A(h->plans[0].dev, h->plan_bytes_cap);
+    if (cfg->max_spec_draft > 0) A(h->plans[1].dev, h->plan_bytes_cap);
     A(h->cand, h->cand_entries * 8);
     A(h->cand_count, R * 64 * 4);
     A(h->tickets, R * 4);
     A(h->flat_rows, R * sizeof(FlatRow));
     {
-        // full-vocabulary rows: per row its exp values (stg_row.cu); for the speculative draws the sub-tile summaries
+        // full-vocabulary rows: per row its exp values (stg_row.cu)
         h->full_cap = (int)std::min<size_t>(R, 1024);
         const size_t F = (size_t)h->full_cap;
         A(h->fw_redo, F * 4);
         A(h->fw_e, F * (size_t)h->escratch_stride * 4);
-        if (cfg->max_spec_draft > 0) {
-            A(h->fw_rows, F * sizeof(FullRow));
-            A(h->fw_ew, F * sizeof(Emul2Work));
-        }
     }
     A(h->work_counter, 256);
     A(h->escratch, (size_t)h->sm_count * h->escratch_stride * 4);
@@ -859,7 +857,7 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
         A(h->sp_draft, R * L * 4); A(h->sp_uniforms, R * (L + 2) * 8);
         A(h->sp_accepted, R * 4); A(h->sp_correction, R * 4); A(h->sp_aprobs, R * L * 4); A(h->sp_flags, R * 4);
         A(h->dists, R * (2 * L + 1) * sizeof(RowDist));
-        A(h->sp_rowstats, R * 20);  // flat verification: 16 bytes of control and a fall-back flag per sequence
+        A(h->sp_rowstats, R * 4);  // a fall-back flag per sequence
     }
     if (rc == STG_OK) {
         e = cudaHostAlloc((void **)&h->plan_host, h->plan_bytes_cap * 4, cudaHostAllocDefault);

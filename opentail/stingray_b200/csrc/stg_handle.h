@@ -42,6 +42,19 @@ struct Plan {
     int n_full_with_top_p = 0;     // ... and on
 };
 
+// The plan of the last step of a kind, as long as the batch description stays the same
+struct PlanSlot {
+    DevBuf dev;                           // RowPlan[], WorkItem[], pow table
+    std::vector<unsigned char> cache;     // bytes of the plan last uploaded
+    Plan plan;
+    std::vector<unsigned char> key;       // the batch description it was built for
+    bool valid = false;
+    uint64_t version = 0;                 // of StgSampler_::plan_version
+    const RowPlan *d_rows = nullptr;      // where the plan lives on the device
+    const WorkItem *d_items = nullptr;
+    const float *d_pow = nullptr;
+};
+
 }  // namespace stg
 
 struct StgSampler_ {
@@ -67,20 +80,14 @@ struct StgSampler_ {
     int lookback_drill = 0;              // STG_LOOKBACK_DRILL=1 or 2 at creation: see SampleArgs::lookback_drill
 
     // workspace (allocated once at creation)
-    stg::DevBuf plan_dev;                // RowPlan[], WorkItem[], pow table
+    stg::PlanSlot plans[2];              // [1]: the draft rows of a speculative step, whose plan is another one than the target rows'
     unsigned char *plan_host = nullptr;  // pinned mirror ring
     cudaEvent_t plan_ev[4]{};
     int plan_slot = 0;
-    std::vector<unsigned char> plan_cache;  // bytes of the plan last uploaded
-    stg::Plan plan;                          // the plan of the last step ...
-    std::vector<unsigned char> plan_key, plan_key_scratch;  // ... and the batch description it was built for
-    bool plan_valid = false;
-    const stg::RowPlan *d_rows = nullptr;    // where that plan lives on the device
-    const stg::WorkItem *d_items = nullptr;
-    const float *d_pow = nullptr;
+    std::vector<unsigned char> plan_key_scratch;
     stg::DevBuf flat_rows;               // FlatRow per row (stg_flat.cuh)
-    // full-vocabulary rows: RowWs (stg_row.cuh) and FullWs (stg_flat.cuh) arrays for up to full_cap rows
-    stg::DevBuf fw_redo, fw_rows, fw_e, fw_ew;
+    // full-vocabulary rows: RowWs arrays (stg_row.cuh) for up to full_cap rows
+    stg::DevBuf fw_redo, fw_e;
     int full_cap = 0;
     stg::DevBuf cand, cand_count, tickets, work_counter, escratch, keyscratch, listscratch, dists;
     stg::DevBuf st_hist, st_bias_ids, st_bias_vals, st_uniforms, st_mask, st_logits;
@@ -134,6 +141,7 @@ struct BatchExtra {
     int shard_mode = 0;           // 1: export each row's local candidates to the exchange buffer
     int vocab_offset = 0;
     int global_vocab = 0;         // 0: same as the batch's vocab
+    int plan_slot = 0;            // StgSampler_::plans
     bool want_argmax = false;     // mode 2: the arg-max of the raw rows goes with the descriptors
 };
 int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *stream);

@@ -32,6 +32,7 @@
 #include "stg_launch.h"
 #include "stg_row.cuh"
 #include "stg_rowdist.cuh"
+#include "stg_spec_prov.cuh"
 #include "stg_walk.cuh"
 
 namespace cg = cooperative_groups;
@@ -1505,19 +1506,174 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     }
 }
 
+// ---- speculative verification: accept chain and draw -------------------------------------------------------
+// What k_spec_finish (stg_spec_kernels.cu) does with one CTA per sequence, by a cluster per sequence: the accept
+// chain by a warp of every CTA (the draft positions side by side), then the values the draw runs over - the
+// target row's final probabilities (bonus draw, looser rule) or the residual max(p - q, 0), recomputed from
+// the logits - to the sequence's scratch row, and the walk of stg_walk.cuh; for the residual first to its sum, then
+// to u * sum.  As three kernels, one of them a CTA per sequence, a lone sequence took 110 us.  Sequences
+// that need a rare fall-back (an empty residual, a walk off the end) are left to k_spec_finish.
+template <bool BF16>
+__global__ void __launch_bounds__(kRT, 2) k_spec_row(const __grid_constant__ SpecArgs a, const RowWs ws, int32_t *fallback)
+{
+    extern __shared__ __align__(128) unsigned char dyn[];
+    __shared__ RowSh sh;
+    __shared__ int s_acc, s_bad;
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int s = blockIdx.x / C;
+    const int L = a.n_draft, n = a.vocab, nsub = (n + kSub - 1) / kSub;
+    const int per = (nsub + C - 1) / C;
+    const int t0 = min(rank * per, nsub), t1 = min(t0 + per, nsub);
+    WalkArea *wa = (WalkArea *)dyn;
+    WalkArea *dst = rank == 0 ? wa : (WalkArea *)cl.map_shared_rank((unsigned char *)wa, 0);
+    float *e = ws.e + (size_t)s * ws.e_stride;
+    const int esz = BF16 ? 2 : 4;
+    const RowDist *td = a.tdist + (int64_t)s * (L + 1);
+    const RowDist *dd = a.ddist ? a.ddist + (int64_t)s * L : nullptr;
+    const char *trows = (const char *)a.target + (int64_t)s * (L + 1) * n * esz;
+    const char *drows = a.draft ? (const char *)a.draft + (int64_t)s * L * n * esz : nullptr;
+    const double *u = a.uniforms + (int64_t)s * (L + 2);
+    const bool greedy = (td[0].flags & kDistOneHot) != 0;
+    if (warp == 0) {
+        bool ok = true, bad = false;
+        float shown = 0.f;
+        if (lane < L) {
+            const int i = lane;
+            const int tok = a.draft_tokens[(int64_t)s * L + i];
+            if ((unsigned)tok >= (unsigned)n) {
+                // a draft token outside the vocabulary (the reference's pDist[tokens[i]] throws,
+                // SpeculativeDecoder.cs:534): never read, rejected, and reported in the flags
+                ok = false;
+                bad = true;
+            } else if (greedy) {
+                ok = (tok == td[i].tie_idx_max);  // SpeculativeDecoder.Step, SpeculativeDecoder.cs:400-405
+                shown = ok ? 1.f : 0.f;
+            } else {
+                const float px = eval_point<BF16>(LogitRow{trows + (int64_t)i * n * esz, a.target_cap}, tok, td[i]);
+                if (a.mode == 0) {
+                    const float qx = eval_point<BF16>(LogitRow{drows + (int64_t)i * n * esz, a.draft_cap}, tok, dd[i]);
+                    const float r = qx > 0.f ? fminf(1.f, __fdiv_rn(px, qx)) : (px > 0.f ? 1.f : 0.f);
+                    ok = u[i] < (double)r;
+                    shown = r;
+                } else {
+                    ok = px >= a.p_min || tok == td[i].argmax;
+                    shown = px;
+                }
+            }
+        }
+        const unsigned rej = __ballot_sync(0xFFFFFFFFu, lane < L && !ok);
+        const int acc = rej ? __ffs(rej) - 1 : L;
+        const bool bad_draft = acc < L && __shfl_sync(0xFFFFFFFFu, bad ? 1 : 0, min(acc, 31)) != 0;
+        if (rank == 0) {
+            // positions after the first rejection are not tested
+            if (a.accept_probs && lane < L) a.accept_probs[(int64_t)s * L + lane] = lane <= acc ? shown : 0.f;
+            if (lane == 0) {
+                fallback[s] = 0;
+                a.accepted[s] = acc;
+                if (greedy) {
+                    a.correction[s] = td[acc].tie_idx_max;
+                    if (a.seq_flags) a.seq_flags[s] = bad_draft ? (1u << 9) : 0u;
+                }
+            }
+        }
+        if (lane == 0) { s_acc = acc; s_bad = bad_draft ? 1 : 0; }
+    }
+    if (greedy) return;
+    __syncthreads();
+    const int acc = s_acc;
+    const bool residual = !(acc == L || a.mode == 1);
+    {
+        const bool al = a.vec == 4;
+        const RowDist tdr = td[acc];
+        const LogitRow prow{trows + (int64_t)acc * n * esz, a.target_cap};
+        const ProvRow<BF16> pp{SrcLogits<BF16>{prow, nullptr, al, tdr.inv_t, tdr.inv_t != 1.0f}, tdr};
+        auto tile = [&](int t, const float (&x)[8]) {
+            store_e(e, t * kSub + lane * 8, x);
+            float sum = 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) sum += x[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
+            if (lane == 0) sh.tile_sum[t - t0] = sum;
+        };
+        if (residual) {
+            const RowDist dq = dd[acc];
+            const LogitRow qrow{drows + (int64_t)acc * n * esz, a.draft_cap};
+            const ProvRow<BF16> qq{SrcLogits<BF16>{qrow, nullptr, al, dq.inv_t, dq.inv_t != 1.0f}, dq};
+            const ProvResidual<BF16> rr{pp, qq};
+#pragma unroll 1
+            for (int t = t0 + warp; t < t1; t += kRW) {
+                float x[8];
+                rr.load(t * kSub + lane * 8, n, x);  // zeros beyond the row
+                tile(t, x);
+            }
+        } else {
+#pragma unroll 1
+            for (int t = t0 + warp; t < t1; t += kRW) {
+                float x[8];
+                pp.load(t * kSub + lane * 8, n, x);
+                tile(t, x);
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        double v = 0.0;
+        for (int t = lane; t < t1 - t0; t += 32) v += (double)sh.tile_sum[t];
+        v = warp_sum_d(v);
+        if (lane < C) cl.map_shared_rank(&sh, lane)->tot[0][rank] = v;
+    }
+    cl.sync();
+    double base = 0.0, all = 0.0;
+    for (int r = 0; r < C; r++) {
+        if (r == rank) base = all;
+        all += sh.tot[0][r];
+    }
+    const float u0 = __double2float_rn(u[L]);
+    auto get = [&](int t, float x[8]) { load_e(e, t * kSub + lane * 8, x); };
+    // the target of a residual is u times its sum: where it should lie is known well enough
+    summarise(sh, wa, dst, get, t0, t1, base, sh.tot[0][rank], all, 1.0, residual ? (double)u0 * all : (double)u0);
+    cl.sync();
+    if (rank != 0 || warp != 0) return;
+    float target = u0;
+    if (residual) {
+        // ResampleResidual (Sampler.cs:587-618): the sum of the residual, then the draw to u * sum
+        const float sum = row_walk(wa, get, n, nsub, 0.f, false).s;
+        if (!(sum > 0.f)) {  // nothing left of p - q (or NaN): the draw from p with the spare uniform
+            if (lane == 0) fallback[s] = 1;
+            return;
+        }
+        target = __fmul_rn(u0, sum);
+    }
+    const WalkOut o = row_walk(wa, get, n, nsub, target, true);
+    if (lane == 0) {
+        uint32_t fl = s_bad ? (1u << 9) : 0u;
+        int corr = o.hit;
+        if (corr < 0) {
+            if (residual) { fallback[s] = 1; return; }  // the rounding fall-back of the residual draw
+            corr = n - 1;
+            fl |= 1u << 5;
+        }
+        a.correction[s] = corr;
+        if (a.seq_flags) a.seq_flags[s] = fl;
+    }
+}
+
 }  // namespace
 
-cudaError_t launch_row_clusters(const SampleArgs &a, const RowWs &ws, bool want_argmax, cudaStream_t stream)
+// Launches `rows` clusters as large as the rows leave room for, one wave: a lone row is spread over 16 CTAs, several
+// hundred rows get one each (two CTAs fit an SM).  A CTA has at least one tile per warp.
+template <class... Params, class... Args>
+static cudaError_t launch_clusters(void (*fn)(Params...), size_t smem, int rows, int vocab, cudaStream_t stream, const Args &...args)
 {
-    void (*fn)(const SampleArgs, const RowWs, int) = a.dtype == 1 ? k_row<true> : k_row<false>;
-    cudaError_t e = ensure_dynamic_smem((const void *)fn, kRowSmem);
+    cudaError_t e = ensure_dynamic_smem((const void *)fn, smem);
     if (e != cudaSuccess) return e;
-    // Clusters as large as the rows leave room for, one wave: a lone row is spread over 16 CTAs, several
-    // hundred rows get one each (two CTAs fit an SM).  A CTA has at least one tile per warp.
-    const int nsub = (a.vocab + kSub - 1) / kSub;
+    const int nsub = (vocab + kSub - 1) / kSub;
     struct Fit { int n[5]; };
     static std::mutex mu;
-    static std::map<std::pair<int, int>, Fit> fits;
+    static std::map<std::pair<const void *, int>, Fit> fits;
     int dev = 0;
     e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -1525,14 +1681,14 @@ cudaError_t launch_row_clusters(const SampleArgs &a, const RowWs &ws, bool want_
     at.id = cudaLaunchAttributeClusterDimension;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kRT);
-    cfg.dynamicSmemBytes = kRowSmem;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     Fit fit;
     {
         std::lock_guard<std::mutex> lock(mu);
-        auto it = fits.find({dev, a.dtype});
+        auto it = fits.find({(const void *)fn, dev});
         if (it == fits.end()) {
             e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e != cudaSuccess) return e;
@@ -1542,17 +1698,27 @@ cudaError_t launch_row_clusters(const SampleArgs &a, const RowWs &ws, bool want_
                 e = cudaOccupancyMaxActiveClusters(&fit.n[k], fn, &cfg);
                 if (e != cudaSuccess) { cudaGetLastError(); fit.n[k] = 0; }
             }
-            fits[{dev, a.dtype}] = fit;
+            fits[{(const void *)fn, dev}] = fit;
         } else {
             fit = it->second;
         }
     }
     int k = 0;
     for (int j = 4; j > 0; j--)
-        if (fit.n[j] >= a.n_items && (1 << j) * kRW <= nsub) { k = j; break; }
+        if (fit.n[j] >= rows && (1 << j) * kRW <= nsub) { k = j; break; }
     at.val.clusterDim = {1u << k, 1, 1};
-    cfg.gridDim = dim3((unsigned)a.n_items << k);
-    return cudaLaunchKernelEx(&cfg, fn, a, ws, want_argmax ? 1 : 0);
+    cfg.gridDim = dim3((unsigned)rows << k);
+    return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+cudaError_t launch_row_clusters(const SampleArgs &a, const RowWs &ws, bool want_argmax, cudaStream_t stream)
+{
+    return launch_clusters(a.dtype == 1 ? k_row<true> : k_row<false>, kRowSmem, a.n_items, a.vocab, stream, a, ws, want_argmax ? 1 : 0);
+}
+
+cudaError_t launch_spec_rows(const SpecArgs &a, const RowWs &ws, int32_t *fallback, cudaStream_t stream)
+{
+    return launch_clusters(a.dtype == 1 ? k_spec_row<true> : k_spec_row<false>, sizeof(WalkArea), a.n_seq, a.vocab, stream, a, ws, fallback);
 }
 
 }  // namespace stg

@@ -23,4 +23,9 @@ struct RowWs {
 // want_argmax: descriptor mode (a.mode == 2) needs the arg-max of the raw row as well.
 cudaError_t launch_row_clusters(const SampleArgs &a, const RowWs &ws, bool want_argmax, cudaStream_t stream);
 
+// speculative verification behind the descriptor passes: accept chain and draw of every sequence (at most 32 draft
+// tokens); fallback[s] becomes 1 where k_spec_finish has to redo sequence s
+struct SpecArgs;
+cudaError_t launch_spec_rows(const SpecArgs &a, const RowWs &ws, int32_t *fallback, cudaStream_t stream);
+
 }  // namespace stg
