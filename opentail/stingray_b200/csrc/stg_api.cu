@@ -556,7 +556,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     int launches = 0;
     int row_grid = 0;
     FlatRow *fr = (FlatRow *)h->flat_rows.p;
-    const RowWs rw{(float *)h->fw_e.p, h->escratch_stride, (int32_t *)h->fw_redo.p};
+    const RowWs rw{(float *)h->fw_e.p, (int32_t *)h->fw_ids.p, h->escratch_stride, (int32_t *)h->fw_redo.p};
     const bool flat_chunks = pl.flat && n_chunk_items > 0, flat_full = pl.flat_full && n_rows_items > 0;
     auto launch_rows_kernel = [&](bool redo_only, cudaStream_t on) {
         SampleArgs r = a;
@@ -754,7 +754,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
 // every device buffer a handle owns
 std::vector<DevBuf *> all_buffers(StgHandle h)
 {
-    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
+    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->fw_ids, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
             &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
             &h->st_mask, &h->st_logits, &h->o_tokens, &h->o_probs, &h->o_flags, &h->o_topk_ids, &h->o_topk_vals, &h->o_topk_probs,
             &h->o_pairs, &h->ticks, &h->ring_ids, &h->ring_len_dev, &h->mc_words, &h->mc_slots, &h->sp_draft, &h->sp_uniforms,
@@ -817,6 +817,7 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
         const size_t F = (size_t)h->full_cap;
         A(h->fw_redo, F * 4);
         A(h->fw_e, F * (size_t)h->escratch_stride * 4);
+        A(h->fw_ids, F * (size_t)h->escratch_stride * 4);
     }
     A(h->work_counter, 256);
     A(h->escratch, (size_t)h->sm_count * h->escratch_stride * 4);

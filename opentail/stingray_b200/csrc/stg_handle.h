@@ -87,7 +87,7 @@ struct StgSampler_ {
     std::vector<unsigned char> plan_key_scratch;
     stg::DevBuf flat_rows;               // FlatRow per row (stg_flat.cuh)
     // full-vocabulary rows: RowWs arrays (stg_row.cuh) for up to full_cap rows
-    stg::DevBuf fw_redo, fw_e;
+    stg::DevBuf fw_redo, fw_e, fw_ids;
     int full_cap = 0;
     stg::DevBuf cand, cand_count, tickets, work_counter, escratch, keyscratch, listscratch, dists;
     stg::DevBuf st_hist, st_bias_ids, st_bias_vals, st_uniforms, st_mask, st_logits;

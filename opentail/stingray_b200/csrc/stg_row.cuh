@@ -15,6 +15,7 @@ constexpr int kRowMaxCluster = 16;   // CTAs of a cluster at most (above 8 is an
 // device workspace of the full-vocabulary rows of a step, indexed by RowPlan::flat_full
 struct RowWs {
     float *e;            // [n, e_stride] exp values (L2-resident between the phases), rows padded to whole tiles of 256
+    int32_t *ids;        // [n, e_stride] tokens of a row that was closed up to what its mask allows
     int64_t e_stride;
     int32_t *redo;       // [n] 1: the row kernel of the first design has to redo the row
 };

@@ -174,7 +174,7 @@ int stg_spec_verify(StgHandle h, const StgSpecBatch *b, void *stream_)
     cudaError_t e = cudaSuccess;
     static const bool no_flat_spec = getenv("STG_NO_FLAT_SPEC") != nullptr;
     if (!no_flat_spec && !getenv("STG_NO_FLAT") && S <= h->full_cap && L <= 32 && V <= kSub * kMaxSubTiles && h->sp_rowstats.p) {
-        const RowWs rw{(float *)h->fw_e.p, h->escratch_stride, (int32_t *)h->fw_redo.p};
+        const RowWs rw{(float *)h->fw_e.p, (int32_t *)h->fw_ids.p, h->escratch_stride, (int32_t *)h->fw_redo.p};
         int32_t *fallback = (int32_t *)h->sp_rowstats.p;
         e = launch_spec_rows(a, rw, fallback, stream);
         if (e != cudaSuccess) return cuda_fail(h, e, "speculative verification launch");
