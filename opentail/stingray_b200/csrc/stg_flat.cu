@@ -1,5 +1,4 @@
-// Kernels of the flat form of a sampling step (see stg_flat.cuh): prep, the HBM streaming pass, and
-// the per-row finish of the top-k path.
+// Kernels of the flat form of a sampling step (see stg_flat.cuh): prep and the per-row finish of the top-k path.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -14,9 +13,7 @@
 namespace stg {
 
 // ---- k_flat_prep --------------------------------------------------------------------------------------
-// One 1024-thread CTA per row (flat_prep_row, stg_flat_prep.cuh).  Launched on its own only when the
-// step has no full-vocabulary rows in the flat form; otherwise k_full_prep, which has a CTA per row
-// anyway, does this for the rows that are not its own.
+// One 1024-thread CTA per row (flat_prep_row, stg_flat_prep.cuh).
 template <bool BF16, bool CAP>
 __global__ void __launch_bounds__(kThreads) k_flat_prep(const __grid_constant__ SampleArgs a, FlatRow *fr)
 {

@@ -1,4 +1,4 @@
-// What a row of the flat step needs before it can be streamed (shared by k_flat_prep and k_full_prep).
+// What a row of the flat step needs before it can be streamed (k_flat_prep).
 #pragma once
 #include <math_constants.h>
 

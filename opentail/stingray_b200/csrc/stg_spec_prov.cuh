@@ -1,6 +1,6 @@
 // Providers of speculative verification: a row's final probabilities recomputed from its logits and
-// its distribution descriptor, and the positive part of p - q (shared by stg_spec_kernels.cu and the
-// flat form in stg_flat_full.cu).
+// its distribution descriptor, and the positive part of p - q (shared by stg_spec_kernels.cu and
+// stg_row.cu).
 #pragma once
 #include "stg_rowdist.cuh"
 

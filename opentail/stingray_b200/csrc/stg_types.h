@@ -45,7 +45,7 @@ struct RowPlan {
     int32_t cand_off;   // first entry of this row's candidate scratch (entries of 8 bytes)
     int32_t use_mask, has_penalty, pow_off, slot;
     int32_t flat_groups; // flat step, top-k rows: groups of the sample whose maxima bound the filter (power of two)
-    int32_t flat_full;   // flat step: index of a full-vocabulary row in the step's FullWs, -1 otherwise
+    int32_t flat_full;   // flat step: index of a full-vocabulary row in the step's RowWs, -1 otherwise
     int32_t flat_rank;   // flat step, top-k rows: the bound is the sample's flat_rank-th largest logit (0: the groups' bound itself)
 };
 
@@ -125,7 +125,7 @@ struct SampleArgs {
     float softcap;                   // != 0: every logit is read as tanh(x / softcap) * softcap
     int32_t finish_cap;              // candidates per buffer of the half-size finish (stg_flat_finish_half.cu)
     int32_t static_items;            // row kernel: CTA b takes items b, b + grid, ... (no work counter: the launch can be replayed)
-    int32_t lookback_drill;          // STG_LOOKBACK_DRILL at stg_create: 1 makes the exp pass's look-back run out, 2 that of the draw's partial sums
+    int32_t lookback_drill;          // STG_LOOKBACK_DRILL at stg_create: k_row gives every row up before its sum (1) or at its draw (2)
     const int32_t *redo_flags;       // row kernel as the flat step's second chance: only rows whose flag
     int32_t redo_stride;             // redo_flags[flat_full * redo_stride] is set are run; null: every row item
 };
