@@ -3,18 +3,16 @@
 //
 //   k_flat_prep    one CTA per row   what a row needs before it can be streamed: the filter bound of
 //                                    a top-k row (an order statistic of its first 4096 logits), zeroed
-//                                    counters (done by k_full_prep when the step has full rows too)
-//   k_flat_stream, k_flat_stream_chunks
-//                  one small CTA per 16384-element piece of a row: the only kernels that read the
-//                  logits from HBM, each row once - the first over the full-vocabulary rows
-//                  (stg_flat.cu), the second over all others (stg_flat_chunks.cu: fewer registers,
-//                  more resident warps).  Greedy rows keep a running arg-max key (64-bit atomicMax),
-//                  top-k rows append every logit above the row's bound to the row's candidate list
-//                  (staged in shared memory, one global atomicAdd per CTA)
+//                                    counters
+//   k_flat_stream_chunks
+//                  one small CTA per piece of a row (stg_flat_chunks.cu).  Greedy rows keep a running
+//                  arg-max key (64-bit atomicMax), top-k rows append every logit above the row's bound
+//                  to the row's candidate list (staged in shared memory, one global atomicAdd per CTA)
 //   k_flat_finish  one CTA per row   candidates only: the exact top-N selection, penalties, softmax
 //                                    over k, min-p, top-p and the draw of SampleTopK
 //                                    (src/OpenTail.Stingray.Engine/Sampler.cs:216-357); built for 1024,
 //                                    512 and 256 threads (one, two, four CTAs per SM)
+//   k_row          one cluster of CTAs per full-vocabulary row (stg_row.cuh), beside the kernels above
 //   k_greedy_step  a step whose rows are all plain arg-max rows: the HBM pass with prep and finish
 //                  folded in, one launch (stg_flat_greedy.cu)
 //
@@ -34,12 +32,11 @@
 
 namespace stg {
 
-constexpr int kFlatThreads = 256;                  // threads of a k_flat_stream CTA
+constexpr int kFlatThreads = 256;                  // threads of a k_flat_stream_chunks CTA
 constexpr int kFlatPiece = 16384;                  // elements of a row one such CTA reads
-constexpr int kFlatSteps = kFlatPiece / 4096;      // steps of 4 sub-steps of 1024 elements each
 constexpr int kFlatSample = 4096;                  // leading elements of a row the bound is guessed from
 constexpr int kFlatSlack = 8192;                   // candidate capacity of a top-k row beyond N (the bound scatters: up to ~3x the expected count was seen)
-constexpr int kFlatStage = 1024;                   // candidates a k_flat_stream CTA collects in shared memory
+constexpr int kFlatStage = 1024;                   // candidates a k_flat_stream_chunks CTA collects in shared memory
 
 // per-row state of the flat step (device memory, 32 bytes)
 struct FlatRow {

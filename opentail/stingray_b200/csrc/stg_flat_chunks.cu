@@ -1,14 +1,12 @@
-// The HBM pass of the flat step over the rows that are not full-vocabulary rows (top-k path and plain
-// arg-max rows): the same work as those branches of k_flat_stream (stg_flat.cu), as a kernel of its
-// own.  Without the full-vocabulary branch (overrides, stores, two running keys) and without a second
-// register set for prefetched loads it needs 40 registers instead of 62, so more warps are resident to
-// cover the load latency - measured on the arg-max form of this loop (stg_flat_greedy.cu), that is
-// worth more than the prefetch.
+// The HBM pass of the flat step over the rows of the top-k path and plain arg-max rows.  40 registers and no second
+// register set for prefetched loads: the warps that fit besides cover the load latency - measured on the
+// arg-max form of this loop (stg_flat_greedy.cu), that is worth more than the prefetch.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
 
 #include "stg_flat.cuh"
+#include "stg_flat_load.cuh"
 #include "stg_launch.h"
 #include "stg_select.cuh"
 #include "stg_types.h"
@@ -19,53 +17,40 @@
 
 namespace stg {
 
-template <bool BF16>
-__device__ __forceinline__ void chunk_load4(const LogitRow rowp, const uint32_t *mrow, int i, int end, float v[4])
-{
-    if (i + 3 < end) {
-        load_vec4<BF16, true>(rowp, i, v);
-    } else {
-#pragma unroll
-        for (int e = 0; e < 4; e++) v[e] = (i + e < end) ? load_one<BF16>(rowp, i + e) : -CUDART_INF_F;
-    }
-    if (mrow != nullptr && i < end) {
-        const uint32_t bits = __ldg(mrow + (i >> 5)) >> (i & 31);
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-            if (!((bits >> e) & 1u)) v[e] = -CUDART_INF_F;
-    }
-}
-
-// grid (pieces of kFlatPiece elements, rows of a.items); 256 threads; in step s thread t reads elements
-// 4096 s + 1024 u + 4 t .. + 3 (u = 0..3) of the piece as four independent 16-byte loads
-template <bool BF16, bool CAP>
+// grid (pieces of STEPS * 4096 elements, rows of a.items); 256 threads; in round s thread t reads elements
+// 256 E (U s + u) + E t .. + E - 1 (u < U) of the piece as U independent 16-byte loads (E 4 of fp32, 8 of bf16:
+// a loop's step of 96 bf16 rows of 151,936 went from 86.9 to 84.6 us with those instead of 8-byte loads).
+// STEPS is 4 where that gives every SM two CTAs to hold, else 1: a lone row of 151,936 is ten pieces of 16,384,
+// each four dependent rounds of loads long, or 38 of 4096.
+template <bool BF16, bool CAP, int STEPS>
 __global__ void __launch_bounds__(kFlatThreads, STG_CHUNKS_MB) k_flat_stream_chunks(const __grid_constant__ SampleArgs a, FlatRow *fr)
 {
     const int row = __ldg(&a.items[blockIdx.y].row), tid = threadIdx.x, lane = tid & 31;
     const RowPlan *rpp = a.plans + row;
     if (__ldg(&rpp->n_chunks) == 0) return;  // not a row of this pass
-    const int begin = blockIdx.x * kFlatPiece;
-    const int end = min(a.vocab, begin + kFlatPiece);
+    const int begin = blockIdx.x * (STEPS * 4096);
+    const int end = min(a.vocab, begin + STEPS * 4096);
     if (begin >= end) return;
     const int esz = BF16 ? 2 : 4;
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, CAP ? a.softcap : 0.f};
     const uint32_t *mrow = (__ldg(&rpp->use_mask) && a.mask) ? a.mask + (int64_t)row * a.mask_stride : nullptr;
-    const int i0 = begin + tid * 4;
+    typedef FlatShare<BF16, STEPS> S;
+    const int i0 = begin + tid * S::E;
 
     if (__ldg(&rpp->path) == kPathGreedy) {
         __shared__ unsigned long long red[kFlatThreads / 32];
         float best = -CUDART_INF_F;
         int best_i = -1;
 #pragma unroll 1
-        for (int s = 0; s < kFlatSteps; s++) {
-            float cur[4][4];
+        for (int s = 0; s < S::R; s++) {
+            float cur[S::U][S::E];
 #pragma unroll
-            for (int u = 0; u < 4; u++) chunk_load4<BF16>(rowp, mrow, i0 + (s * 4 + u) * 1024, end, cur[u]);
+            for (int u = 0; u < S::U; u++) flat_load<BF16>(rowp, mrow, i0 + (s * S::U + u) * S::kStride, end, cur[u]);
 #pragma unroll
-            for (int u = 0; u < 4; u++)
+            for (int u = 0; u < S::U; u++)
 #pragma unroll
-                for (int e = 0; e < 4; e++)
-                    if (cur[u][e] > best) { best = cur[u][e]; best_i = i0 + (s * 4 + u) * 1024 + e; }
+                for (int e = 0; e < S::E; e++)
+                    if (cur[u][e] > best) { best = cur[u][e]; best_i = i0 + (s * S::U + u) * S::kStride + e; }
         }
         // a thread visits ascending indices, so it holds its lowest index of the value; the key
         // order (value, then lower index) settles ties between threads, pieces and CTAs
@@ -96,27 +81,27 @@ __global__ void __launch_bounds__(kFlatThreads, STG_CHUNKS_MB) k_flat_stream_chu
     const int cap = fr[row].cap;
     unsigned long long *cand = a.cand + __ldg(&rpp->cand_off);
     int *cnt_p = &fr[row].cnt;
-    // The sweep itself only notes which of the thread's 64 elements pass (one bit each): keeping the
+    // The sweep itself only notes which of the thread's elements pass (one bit each): keeping the
     // key construction and the appends out of the loop keeps it as tight as the arg-max loop.  The
     // few that pass (a fraction of a percent) are read again afterwards, from L2.
     unsigned long long passed = 0ull;
 #pragma unroll 1
-    for (int s = 0; s < kFlatSteps; s++) {
-        float cur[4][4];
+    for (int s = 0; s < S::R; s++) {
+        float cur[S::U][S::E];
 #pragma unroll
-        for (int u = 0; u < 4; u++) chunk_load4<BF16>(rowp, mrow, i0 + (s * 4 + u) * 1024, end, cur[u]);
+        for (int u = 0; u < S::U; u++) flat_load<BF16>(rowp, mrow, i0 + (s * S::U + u) * S::kStride, end, cur[u]);
         unsigned pass = 0u;
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+        for (int u = 0; u < S::U; u++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) pass |= (cur[u][e] > tau) ? (1u << (u * 4 + e)) : 0u;  // out of range and masked read -inf
-        passed |= (unsigned long long)pass << (16 * s);
+            for (int e = 0; e < S::E; e++) pass |= (cur[u][e] > tau) ? (1u << (u * S::E + e)) : 0u;  // out of range and masked read -inf
+        passed |= (unsigned long long)pass << (S::U * S::E * s);
     }
-    static_assert(kFlatSteps * 16 <= 64, "one bit per element of a thread");
+    static_assert(STEPS * 16 <= 64, "one bit per element of a thread");
     while (passed != 0ull) {
         const int b = __ffsll((long long)passed) - 1;
         passed &= passed - 1ull;
-        const int idx = i0 + (b >> 2) * 1024 + (b & 3);  // bit 16 s + 4 u + e: sub-step 4 s + u, element e
+        const int idx = i0 + b / S::E * S::kStride + b % S::E;  // bit E (U s + u) + e
         const unsigned long long key = make_key(load_one<BF16>(rowp, idx), idx);
         const int slot = atomicAdd(&stage_cnt, 1);
         if (slot < kFlatStage) {
@@ -139,10 +124,16 @@ __global__ void __launch_bounds__(kFlatThreads, STG_CHUNKS_MB) k_flat_stream_chu
 
 cudaError_t launch_flat_stream_chunks(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
 {
-    const dim3 grid((unsigned)((a.vocab + kFlatPiece - 1) / kFlatPiece), (unsigned)a.n_items);
+    const int pieces = (a.vocab + kFlatPiece - 1) / kFlatPiece;
+    const bool few = (long long)pieces * a.n_items < 2 * 148;
+    const dim3 grid((unsigned)(few ? (a.vocab + 4095) / 4096 : pieces), (unsigned)a.n_items);
     const bool cap = a.softcap != 0.f;
-    if (a.dtype == 1) { if (cap) k_flat_stream_chunks<true, true><<<grid, kFlatThreads, 0, stream>>>(a, fr); else k_flat_stream_chunks<true, false><<<grid, kFlatThreads, 0, stream>>>(a, fr); }
-    else { if (cap) k_flat_stream_chunks<false, true><<<grid, kFlatThreads, 0, stream>>>(a, fr); else k_flat_stream_chunks<false, false><<<grid, kFlatThreads, 0, stream>>>(a, fr); }
+    void (*fn)(const SampleArgs, FlatRow *);
+    if (a.dtype == 1) fn = few ? (cap ? k_flat_stream_chunks<true, true, 1> : k_flat_stream_chunks<true, false, 1>)
+                               : (cap ? k_flat_stream_chunks<true, true, 4> : k_flat_stream_chunks<true, false, 4>);
+    else fn = few ? (cap ? k_flat_stream_chunks<false, true, 1> : k_flat_stream_chunks<false, false, 1>)
+                  : (cap ? k_flat_stream_chunks<false, true, 4> : k_flat_stream_chunks<false, false, 4>);
+    fn<<<grid, kFlatThreads, 0, stream>>>(a, fr);
     return cudaGetLastError();
 }
 

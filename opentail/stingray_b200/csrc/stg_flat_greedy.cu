@@ -10,63 +10,48 @@
 #include <stdint.h>
 
 #include "stg_flat.cuh"
+#include "stg_flat_load.cuh"
 #include "stg_launch.h"
 #include "stg_select.cuh"
 #include "stg_types.h"
 
 namespace stg {
 
-template <bool BF16>
-__device__ __forceinline__ void greedy_load4(const LogitRow rowp, const uint32_t *mrow, int i, int end, float v[4])
-{
-    if (i + 3 < end) {
-        load_vec4<BF16, true>(rowp, i, v);
-    } else {
-#pragma unroll
-        for (int e = 0; e < 4; e++) v[e] = (i + e < end) ? load_one<BF16>(rowp, i + e) : -CUDART_INF_F;
-    }
-    if (mrow != nullptr && i < end) {
-        const uint32_t bits = __ldg(mrow + (i >> 5)) >> (i & 31);
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-            if (!((bits >> e) & 1u)) v[e] = -CUDART_INF_F;
-    }
-}
-
-// grid (pieces of kFlatPiece elements, rows of a.items); 256 threads; in step s thread t reads elements
-// 4096 s + 1024 u + 4 t .. + 3 (u = 0..3) of the piece as four independent 16-byte loads.
+// grid (pieces of STEPS * 4096 elements, rows of a.items); 256 threads; in round s thread t has
+// U independent 16-byte loads in flight; STEPS, rounds and elements as in stg_flat_chunks.cu.
 // Measured on the 256 x 151,936 batch, microseconds per step: this form 29.5 (launch bounds 256 x 5; the
 // same source under 256 x 6 or 256 x 8 gives 34.0 and 31.4, all at 31-40 registers - the difference is
 // the instruction schedule); the next four loads prefetched into a second register set (60 registers,
 // four CTAs per SM) 31.6; a grid resident all at once with equal runs of 4096-element units per CTA
 // 31.5; deeper prefetch at fewer CTAs per SM (3 x 3 units, 2 x 4 units in registers) 39.7 and 39.9.
-template <bool BF16, bool CAP>
+template <bool BF16, bool CAP, int STEPS>
 __global__ void __launch_bounds__(kFlatThreads, 5) k_greedy_step(const __grid_constant__ SampleArgs a, FlatRow *fr)
 {
     __shared__ unsigned long long red[kFlatThreads / 32];
     const int row = __ldg(&a.items[blockIdx.y].row), tid = threadIdx.x, lane = tid & 31;
     const RowPlan *rpp = a.plans + row;
-    const int begin = blockIdx.x * kFlatPiece;
-    const int end = min(a.vocab, begin + kFlatPiece);
+    const int begin = blockIdx.x * (STEPS * 4096);
+    const int end = min(a.vocab, begin + STEPS * 4096);
     const int esz = BF16 ? 2 : 4;
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, CAP ? a.softcap : 0.f};
     const uint32_t *mrow = (__ldg(&rpp->use_mask) && a.mask) ? a.mask + (int64_t)row * a.mask_stride : nullptr;
-    const int i0 = begin + tid * 4;
+    typedef FlatShare<BF16, STEPS> S;
+    const int i0 = begin + tid * S::E;
 
     // No register double-buffering: a thread has the four 16-byte loads of one step in flight and the
     // other warps of the SM (40 registers: six CTAs) cover their latency.
     float best = -CUDART_INF_F;
     int best_i = -1;
 #pragma unroll 1
-    for (int s = 0; s < kFlatPiece / 4096; s++) {
-        float cur[4][4];
+    for (int s = 0; s < S::R; s++) {
+        float cur[S::U][S::E];
 #pragma unroll
-        for (int u = 0; u < 4; u++) greedy_load4<BF16>(rowp, mrow, i0 + (s * 4 + u) * 1024, end, cur[u]);
+        for (int u = 0; u < S::U; u++) flat_load<BF16>(rowp, mrow, i0 + (s * S::U + u) * S::kStride, end, cur[u]);
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+        for (int u = 0; u < S::U; u++)
 #pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (cur[u][e] > best) { best = cur[u][e]; best_i = i0 + (s * 4 + u) * 1024 + e; }
+            for (int e = 0; e < S::E; e++)
+                if (cur[u][e] > best) { best = cur[u][e]; best_i = i0 + (s * S::U + u) * S::kStride + e; }
     }
     // a thread visits ascending indices, so it holds its lowest index of the value; the key order
     // (value, then lower index) settles ties between threads, pieces and CTAs
@@ -110,10 +95,16 @@ __global__ void __launch_bounds__(kFlatThreads, 5) k_greedy_step(const __grid_co
 
 cudaError_t launch_greedy_step(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
 {
-    const dim3 grid((unsigned)((a.vocab + kFlatPiece - 1) / kFlatPiece), (unsigned)a.n_items);
+    const int pieces = (a.vocab + kFlatPiece - 1) / kFlatPiece;
+    const bool few = (long long)pieces * a.n_items < 2 * 148;
+    const dim3 grid((unsigned)(few ? (a.vocab + 4095) / 4096 : pieces), (unsigned)a.n_items);
     const bool cap = a.softcap != 0.f;
-    if (a.dtype == 1) { if (cap) k_greedy_step<true, true><<<grid, kFlatThreads, 0, stream>>>(a, fr); else k_greedy_step<true, false><<<grid, kFlatThreads, 0, stream>>>(a, fr); }
-    else { if (cap) k_greedy_step<false, true><<<grid, kFlatThreads, 0, stream>>>(a, fr); else k_greedy_step<false, false><<<grid, kFlatThreads, 0, stream>>>(a, fr); }
+    void (*fn)(const SampleArgs, FlatRow *);
+    if (a.dtype == 1) fn = few ? (cap ? k_greedy_step<true, true, 1> : k_greedy_step<true, false, 1>)
+                               : (cap ? k_greedy_step<true, true, 4> : k_greedy_step<true, false, 4>);
+    else fn = few ? (cap ? k_greedy_step<false, true, 1> : k_greedy_step<false, false, 1>)
+                  : (cap ? k_greedy_step<false, true, 4> : k_greedy_step<false, false, 4>);
+    fn<<<grid, kFlatThreads, 0, stream>>>(a, fr);
     return cudaGetLastError();
 }
 
