@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(kThreads) k_flat_prep(const __grid_constant__ 
 {
     __shared__ uint32_t red[32];
     __shared__ uint32_t list[kPrepList + 2];
+    pdl_release();
     const int row = blockIdx.x;
     const RowPlan rp = a.plans[row];
     if (rp.n_chunks == 0) return;  // not a row of the flat step
@@ -34,6 +35,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_flat_finish(const __grid_consta
     extern __shared__ __align__(16) unsigned char arena[];
     __shared__ SelCtl ctl;
     __shared__ FlatShared fs;
+    pdl_wait();
     if (!SHARED) {
         flat_finish_row<BF16>(a, fr, a.items[blockIdx.x].row, blockIdx.x, a.cap, arena, ctl, fs);
         return;
@@ -42,6 +44,22 @@ __global__ void __launch_bounds__(kThreads, 1) k_flat_finish(const __grid_consta
         flat_finish_row<BF16>(a, fr, a.items[i].row, i, a.cap, arena, ctl, fs);
         __syncthreads();
     }
+}
+
+cudaError_t launch_behind(void (*fn)(const SampleArgs, FlatRow *), dim3 grid, int block, size_t smem, const SampleArgs &a, FlatRow *fr,
+                          cudaStream_t stream)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, a, fr);
 }
 
 cudaError_t launch_flat_prep(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
@@ -59,8 +77,7 @@ cudaError_t launch_flat_finish(const SampleArgs &a, FlatRow *fr, int grid, size_
                                                            : (shared ? k_flat_finish<false, true> : k_flat_finish<false, false>);
     cudaError_t e = ensure_dynamic_smem((const void *)fn, smem);
     if (e != cudaSuccess) return e;
-    fn<<<grid, kThreads, smem, stream>>>(a, fr);
-    return cudaGetLastError();
+    return launch_behind(fn, grid, kThreads, smem, a, fr, stream);
 }
 
 }  // namespace stg

@@ -27,12 +27,18 @@ __global__ void __launch_bounds__(kFlatThreads, STG_CHUNKS_MB) k_flat_stream_chu
 {
     const int row = __ldg(&a.items[blockIdx.y].row), tid = threadIdx.x, lane = tid & 31;
     const RowPlan *rpp = a.plans + row;
-    if (__ldg(&rpp->n_chunks) == 0) return;  // not a row of this pass
     const int begin = blockIdx.x * (STEPS * 4096);
     const int end = min(a.vocab, begin + STEPS * 4096);
-    if (begin >= end) return;
     const int esz = BF16 ? 2 : 4;
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, CAP ? a.softcap : 0.f};
+    const bool mine = __ldg(&rpp->n_chunks) != 0 && begin < end;
+    // While the rows' bounds are still being found: the pieces of the CTAs that are resident by then, into L2.
+    if (mine && blockIdx.y * gridDim.x + blockIdx.x < 148u * STG_CHUNKS_MB)
+        for (int i = begin + tid * (128 / esz); i < end; i += kFlatThreads * (128 / esz))
+            asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)rowp.p + (int64_t)i * esz));
+    pdl_release();
+    pdl_wait();
+    if (!mine) return;  // not a row of this pass
     const uint32_t *mrow = (__ldg(&rpp->use_mask) && a.mask) ? a.mask + (int64_t)row * a.mask_stride : nullptr;
     typedef FlatShare<BF16, STEPS> S;
     const int i0 = begin + tid * S::E;
@@ -133,8 +139,7 @@ cudaError_t launch_flat_stream_chunks(const SampleArgs &a, FlatRow *fr, cudaStre
                                : (cap ? k_flat_stream_chunks<true, true, 4> : k_flat_stream_chunks<true, false, 4>);
     else fn = few ? (cap ? k_flat_stream_chunks<false, true, 1> : k_flat_stream_chunks<false, false, 1>)
                   : (cap ? k_flat_stream_chunks<false, true, 4> : k_flat_stream_chunks<false, false, 4>);
-    fn<<<grid, kFlatThreads, 0, stream>>>(a, fr);
-    return cudaGetLastError();
+    return launch_behind(fn, grid, kFlatThreads, 0, a, fr, stream);
 }
 
 }  // namespace stg
