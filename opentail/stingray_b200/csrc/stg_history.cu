@@ -38,11 +38,21 @@ __global__ void __launch_bounds__(256) k_history_append(int32_t *ids, int32_t *l
         }
         return;
     }
-    for (int base = 0; base < cap - 1; base += 32) {
-        const int j = base + lane;
-        const int32_t v = (j + 1 < cap) ? row[j + 1] : 0;
+    // A full history moves down by one, 256 tokens at a time: eight loads of a lane in flight and two barriers (one
+    // load a time, a history of 256 took eight dependent rounds of them: 7.0 us for 96 rows).
+    for (int base = 0; base < cap - 1; base += 256) {
+        int32_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int j = base + k * 32 + lane;
+            v[k] = j + 1 < cap ? row[j + 1] : 0;
+        }
         __syncwarp();
-        if (j + 1 < cap) row[j] = v;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const int j = base + k * 32 + lane;
+            if (j + 1 < cap) row[j] = v[k];
+        }
         __syncwarp();
     }
     if (lane == 0) row[cap - 1] = tok;
