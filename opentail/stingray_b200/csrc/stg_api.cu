@@ -367,6 +367,17 @@ bool rows_aligned(const void *p, int64_t row_stride, int dtype)
 
 namespace stg {
 
+int order_behind_last(StgHandle h, cudaStream_t stream)
+{
+    if (h->last_stream_valid && stream != h->last_stream) {
+        CK(cudaEventRecord(h->ev_order, h->last_stream));
+        CK(cudaStreamWaitEvent(stream, h->ev_order, 0));
+    }
+    h->last_stream = stream;
+    h->last_stream_valid = true;
+    return STG_OK;
+}
+
 int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *stream_)
 {
     const int mode = x.mode;
@@ -380,12 +391,10 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     // The workspace, the plan and the work counters belong to the handle, so consecutive calls must
     // not overlap on the device.  On one stream they cannot; when the stream changes, this call is
     // put behind everything enqueued so far on the previous one.
-    if (h->last_stream_valid && stream != h->last_stream) {
-        CK(cudaEventRecord(h->ev_order, h->last_stream));
-        CK(cudaStreamWaitEvent(stream, h->ev_order, 0));
+    if (!x.beside) {
+        rc = order_behind_last(h, stream);
+        if (rc) return rc;
     }
-    h->last_stream = stream;
-    h->last_stream_valid = true;
     const uint32_t mf = b->mem_flags;
     const int rows = b->rows, V = b->vocab;
     if ((mode == 0 || mode == 3) && !pairs_out && !b->tokens && !x.shard_mode) return fail(h, STG_ERR_INVALID_ARGUMENT, "tokens is required");
@@ -505,9 +514,9 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     a.lookback_drill = h->lookback_drill;
     a.phase_ticks = (unsigned long long *)h->ticks.p;
     h->ticks_items = (int)pl.items.size();
-    a.escratch = (float *)h->escratch.p;
-    a.keyscratch = (unsigned long long *)h->keyscratch.p;
-    a.listscratch = (unsigned long long *)h->listscratch.p;
+    a.escratch = (float *)(x.beside ? h->dr_escratch : h->escratch).p;
+    a.keyscratch = (unsigned long long *)(x.beside ? h->dr_keyscratch : h->keyscratch).p;
+    a.listscratch = (unsigned long long *)(x.beside ? h->dr_listscratch : h->listscratch).p;
     a.dists = x.dists_out;
     // vocabulary-sharded mode: one block per rank, [rows, stride] keys followed by [rows] counts,
     // with the stride of this step (its largest selection count), so that one all-gather of
@@ -556,7 +565,8 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     int launches = 0;
     int row_grid = 0;
     FlatRow *fr = (FlatRow *)h->flat_rows.p;
-    const RowWs rw{(float *)h->fw_e.p, (int32_t *)h->fw_ids.p, h->escratch_stride, (int32_t *)h->fw_redo.p};
+    const RowWs rw{(float *)(x.beside ? h->dr_e : h->fw_e).p, x.beside ? nullptr : (int32_t *)h->fw_ids.p, h->escratch_stride,
+                   (int32_t *)(x.beside ? h->dr_redo : h->fw_redo).p};
     const bool flat_chunks = pl.flat && n_chunk_items > 0, flat_full = pl.flat_full && n_rows_items > 0;
     auto launch_rows_kernel = [&](bool redo_only, cudaStream_t on) {
         SampleArgs r = a;
@@ -754,7 +764,8 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
 // every device buffer a handle owns
 std::vector<DevBuf *> all_buffers(StgHandle h)
 {
-    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->fw_ids, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
+    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->fw_ids, &h->dr_redo, &h->dr_e,
+            &h->dr_escratch, &h->dr_keyscratch, &h->dr_listscratch, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
             &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
             &h->st_mask, &h->st_logits, &h->o_tokens, &h->o_probs, &h->o_flags, &h->o_topk_ids, &h->o_topk_vals, &h->o_topk_probs,
             &h->o_pairs, &h->ticks, &h->ring_ids, &h->ring_len_dev, &h->mc_words, &h->mc_slots, &h->sp_draft, &h->sp_uniforms,
@@ -823,6 +834,13 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
     A(h->escratch, (size_t)h->sm_count * h->escratch_stride * 4);
     A(h->keyscratch, (size_t)h->sm_count * h->key_stride * 8);
     A(h->listscratch, (size_t)h->sm_count * (h->key_stride + 512) * 8);  // + 2 sub-tiles: padded reads
+    if (cfg->max_spec_draft > 0) {
+        A(h->dr_redo, (size_t)h->full_cap * 4);
+        A(h->dr_e, (size_t)h->full_cap * (size_t)h->escratch_stride * 4);
+        A(h->dr_escratch, h->escratch.bytes);
+        A(h->dr_keyscratch, h->keyscratch.bytes);
+        A(h->dr_listscratch, h->listscratch.bytes);
+    }
     A(h->st_hist, R * std::max<size_t>(cfg->max_history, 1) * 4);
     A(h->ring_ids, R * std::max<size_t>(cfg->max_history, 1) * 4);
     A(h->ring_len_dev, R * 4);

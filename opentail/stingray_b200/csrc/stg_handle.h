@@ -88,6 +88,8 @@ struct StgSampler_ {
     stg::DevBuf flat_rows;               // FlatRow per row (stg_flat.cuh)
     // full-vocabulary rows: RowWs arrays (stg_row.cuh) for up to full_cap rows
     stg::DevBuf fw_redo, fw_e, fw_ids;
+    // the same (and the row kernel's scratch) for the draft rows of a speculative step, which run beside the target rows
+    stg::DevBuf dr_redo, dr_e, dr_escratch, dr_keyscratch, dr_listscratch;
     int full_cap = 0;
     stg::DevBuf cand, cand_count, tickets, work_counter, escratch, keyscratch, listscratch, dists;
     stg::DevBuf st_hist, st_bias_ids, st_bias_vals, st_uniforms, st_mask, st_logits;
@@ -142,8 +144,11 @@ struct BatchExtra {
     int vocab_offset = 0;
     int global_vocab = 0;         // 0: same as the batch's vocab
     int plan_slot = 0;            // StgSampler_::plans
+    bool beside = false;          // mode 2: runs beside another pass on the handle's side stream, in the draft rows' scratch
     bool want_argmax = false;     // mode 2: the arg-max of the raw rows goes with the descriptors
 };
+// puts what follows on `stream` behind everything the handle has enqueued on another stream
+int order_behind_last(StgHandle h, cudaStream_t stream);
 int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *stream);
 int stage_in(StgHandle h, const void *src, size_t bytes, bool on_host, DevBuf &stage, cudaStream_t stream,
              const void **out);
