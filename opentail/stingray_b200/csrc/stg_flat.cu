@@ -46,22 +46,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_flat_finish(const __grid_consta
     }
 }
 
-cudaError_t launch_behind(void (*fn)(const SampleArgs, FlatRow *), dim3 grid, int block, size_t smem, const SampleArgs &a, FlatRow *fr,
-                          cudaStream_t stream)
-{
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, a, fr);
-}
-
 cudaError_t launch_flat_prep(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
 {
     const bool cap = a.softcap != 0.f;
@@ -77,7 +61,7 @@ cudaError_t launch_flat_finish(const SampleArgs &a, FlatRow *fr, int grid, size_
                                                            : (shared ? k_flat_finish<false, true> : k_flat_finish<false, false>);
     cudaError_t e = ensure_dynamic_smem((const void *)fn, smem);
     if (e != cudaSuccess) return e;
-    return launch_behind(fn, grid, kThreads, smem, a, fr, stream);
+    return launch_behind(fn, dim3((unsigned)grid), kThreads, smem, stream, a, fr);
 }
 
 }  // namespace stg

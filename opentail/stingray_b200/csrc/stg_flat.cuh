@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "stg_pdl.cuh"
 #include "stg_types.h"
 
 namespace stg {
@@ -49,16 +50,8 @@ struct FlatRow {
 };
 static_assert(sizeof(FlatRow) == 32, "FlatRow layout");
 
-// The kernels of the step are launched behind one another before the one ahead has ended: each lets its successor
-// start (pdl_release, once all of its own CTAs are resident) and the successor waits for it in its first
-// instructions (pdl_wait: all of the kernel ahead has ended and its writes are seen).  Every CTA waits, also one
-// without work, so that a kernel's end implies that of all before it in the step.  One fp32 row with top-k 18.4 ->
-// 16.7 us a step, 512 rows of 256,000 140.1 -> 135.5 us.
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-cudaError_t launch_behind(void (*fn)(const SampleArgs, FlatRow *), dim3 grid, int block, size_t smem, const SampleArgs &a, FlatRow *fr,
-                          cudaStream_t stream);
-
+// The kernels of the step are launched behind one another (stg_pdl.cuh).  One fp32 row with top-k 18.4 -> 16.7 us a
+// step, 512 rows of 256,000 140.1 -> 135.5 us.
 cudaError_t launch_flat_prep(const SampleArgs &a, FlatRow *fr, cudaStream_t stream);
 // the HBM pass over rows of the top-k path and plain arg-max rows only (stg_flat_chunks.cu)
 cudaError_t launch_flat_stream_chunks(const SampleArgs &a, FlatRow *fr, cudaStream_t stream);

@@ -139,7 +139,7 @@ cudaError_t launch_flat_stream_chunks(const SampleArgs &a, FlatRow *fr, cudaStre
                                : (cap ? k_flat_stream_chunks<true, true, 4> : k_flat_stream_chunks<true, false, 4>);
     else fn = few ? (cap ? k_flat_stream_chunks<false, true, 1> : k_flat_stream_chunks<false, false, 1>)
                   : (cap ? k_flat_stream_chunks<false, true, 4> : k_flat_stream_chunks<false, false, 4>);
-    return launch_behind(fn, grid, kFlatThreads, 0, a, fr, stream);
+    return launch_behind(fn, grid, kFlatThreads, 0, stream, a, fr);
 }
 
 }  // namespace stg

@@ -12,6 +12,7 @@
 #include <math_constants.h>
 #include <stdint.h>
 
+#include "stg_pdl.cuh"
 #include "stg_launch.h"
 #include "stg_rowdist.cuh"
 #include "stg_select.cuh"
@@ -236,6 +237,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_sample_rows(const __grid_consta
     __shared__ SelCtl ctl;
     __shared__ int sh_item;
     int next = blockIdx.x;
+    if (a.redo_flags != nullptr) pdl_wait();
     for (;;) {
         int item;
         if (a.static_items) {

@@ -32,6 +32,7 @@
 #include "stg_launch.h"
 #include "stg_row.cuh"
 #include "stg_rowdist.cuh"
+#include "stg_pdl.cuh"
 #include "stg_spec_prov.cuh"
 #include "stg_walk.cuh"
 
@@ -1725,6 +1726,7 @@ __global__ void __launch_bounds__(kRT, 2) k_spec_row(const __grid_constant__ Spe
     // the target of a residual is u times its sum: where it should lie is known well enough
     summarise(sh, wa, dst, get, t0, t1, base, sh.tot[0][rank], all, 1.0, residual ? (double)u0 * all : (double)u0);
     cl.sync();
+    pdl_release();
     if (rank != 0 || warp != 0) return;
     float target = u0;
     if (residual) {

@@ -12,6 +12,7 @@
 
 #include "stg_launch.h"
 #include "stg_rowdist.cuh"
+#include "stg_pdl.cuh"
 #include "stg_spec_prov.cuh"
 
 namespace stg {
@@ -32,6 +33,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_spec_finish(const __grid_consta
     Emul2Work *wk2 = (Emul2Work *)spec_dyn;
     const int tid = threadIdx.x;
     const int s = blockIdx.x;
+    pdl_wait();
     if (a.only != nullptr && a.only[s] == 0) return;  // the flat form has finished this sequence
     const int L = a.n_draft, V = a.vocab;
     const int esz = BF16 ? 2 : 4;
@@ -149,6 +151,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_spec_finish(const __grid_consta
 
 cudaError_t launch_spec_finish(const SpecArgs &a, cudaStream_t stream)
 {
+    if (a.only != nullptr)  // behind k_spec_row
+        return launch_behind(a.dtype == 1 ? k_spec_finish<true> : k_spec_finish<false>, dim3((unsigned)a.n_seq), kThreads, sizeof(Emul2Work),
+                             stream, a);
     if (a.dtype == 1) k_spec_finish<true><<<a.n_seq, kThreads, sizeof(Emul2Work), stream>>>(a);
     else k_spec_finish<false><<<a.n_seq, kThreads, sizeof(Emul2Work), stream>>>(a);
     return cudaGetLastError();
