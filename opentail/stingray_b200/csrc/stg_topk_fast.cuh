@@ -9,8 +9,9 @@
 //
 // The row's order is (penalised value descending, raw order among equals).  Keys hold the penalised value, a
 // bit that says a penalty lowered it - its raw logit was higher than those of its equals that none did, so it
-// comes first - and the token.  Two lowered logits that come out equal from different raw values would need
-// more; such a pair among the best k is noticed and the caller takes the general path.
+// comes first - and the token.  Lowered logits that come out equal from different raw values (common with bf16:
+// 11 / 1.1^2 = 10 / 1.1) are put into raw order at the end; left to the general path they made a step of 96
+// rows of 151,936 with histories of their own sampled tokens take 102 us instead of 47.
 #pragma once
 #include <math_constants.h>
 
@@ -194,6 +195,49 @@ __device__ __forceinline__ u64 fast_penalise(u64 key, const int *hkey, const uns
     return ((u64)now << 32) | (key & 0x7FFFFFFFull) | (now != was ? 0x80000000ull : 0ull);
 }
 
+// The sorted keys of one warp, with every run of equal lowered values put into the order of the raw logits.  Keys behind
+// the last one were dropped, so a run that reaches it may lack members; that, or a run beyond 32, is answered
+// with true: the general path.  `buf`: the 32 * KPL keys, in shared memory.
+template <int KPL, class Raw>
+__device__ __noinline__ bool order_by_raw(const Raw raw, u64 *buf, int k)
+{
+    constexpr int K2 = 32 * KPL;
+    const int lane = threadIdx.x & 31;
+    bool fail = false;
+    u64 r[KPL];
+    int to[KPL];
+#pragma unroll
+    for (int q = 0; q < KPL; q++) {
+        const int i = q * 32 + lane;
+        const u64 key = buf[i];
+        r[q] = key;
+        int at = i;
+        if ((key >> 31) & 1ull) {
+            int lo = i, hi = i;
+            while (lo > 0 && i - lo < 32 && (buf[lo - 1] >> 31) == (key >> 31)) lo--;
+            while (hi + 1 < K2 && hi - i < 32 && (buf[hi + 1] >> 31) == (key >> 31)) hi++;
+            if (lo < k && (hi == K2 - 1 || hi - lo >= 32)) {
+                fail = true;
+            } else if (lo < k && lo < hi) {
+                const uint32_t mine = ord32(__fadd_rn(raw(fast_idx(key)), 0.f));
+                at = lo;
+                for (int j = lo; j <= hi; j++) {
+                    if (j == i) continue;
+                    const uint32_t other = ord32(__fadd_rn(raw(fast_idx(buf[j])), 0.f));
+                    at += other > mine || (other == mine && j < i) ? 1 : 0;
+                }
+            }
+        }
+        to[q] = at;
+    }
+    __syncwarp();
+    if (__any_sync(0xFFFFFFFFu, fail)) return true;
+#pragma unroll
+    for (int q = 0; q < KPL; q++) buf[to[q]] = r[q];
+    __syncwarp();
+    return false;
+}
+
 // One CTA, all threads; `list`: cnt keys in device memory, `arena`: shared memory, (kThreads / 64) * 32 * KPL * 8
 // bytes for the merges and, behind them, 8 bytes per slot of the history's hash.  False: nothing was written,
 // the general path has to do the row.  raw(id): the row's logit at token id.
@@ -278,17 +322,28 @@ __device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, i
     if (warp == 0) {
         const int k = rp.top_k;
         bool fail = false;
+        if (pen) {
+            bool tie = false;
 #pragma unroll
-        for (int q = 0; q < KPL; q++) {
-            const int i = q * 32 + lane;
-            if (pen) {
+            for (int q = 0; q < KPL; q++) {
                 // the key behind this one
                 u64 next = __shfl_down_sync(0xFFFFFFFFu, r[q], 1);
                 const u64 head = q + 1 < KPL ? __shfl_sync(0xFFFFFFFFu, r[q + 1 < KPL ? q + 1 : q], 0) : 0ull;
                 if (lane == 31) next = head;
-                if (i < k && next != 0ull && (r[q] >> 31) == (next >> 31) && ((r[q] >> 31) & 1ull))
-                    fail |= ord32(raw(fast_idx(r[q]))) != ord32(raw(fast_idx(next)));
+                tie |= q * 32 + lane < k && next != 0ull && (r[q] >> 31) == (next >> 31) && ((r[q] >> 31) & 1ull);
             }
+            if (__any_sync(0xFFFFFFFFu, tie)) {
+#pragma unroll
+                for (int q = 0; q < KPL; q++) merge[q * 32 + lane] = r[q];
+                __syncwarp();
+                fail = order_by_raw<KPL>(raw, merge, k);
+#pragma unroll
+                for (int q = 0; q < KPL; q++) r[q] = merge[q * 32 + lane];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < KPL; q++) {
+            const int i = q * 32 + lane;
             if (i < k) {
                 fs.vals[i] = r[q] ? key_val(r[q]) : -CUDART_INF_F;
                 fs.ids[i] = r[q] ? fast_idx(r[q]) : -1;
