@@ -33,7 +33,7 @@ def _workload(rows, vocab, bf16, seed, topk=False, sigma=2.5):
     if topk:
         p["top_k"] = rng.choice(np.array([1, 31, 63, 64, 127, 128, 255, 256]), rows)
     hist = W.zipf_ids(rng, rows, 96, vocab)
-    ids, off = W._csr(hist)
+    ids, off = W._csr(np.array(hist))
     return W.SampleWorkload("rows", W.to_bf16_bits(x) if bf16 else x, p, W.uniforms24(rng, rows), ids, off)
 
 
@@ -57,3 +57,25 @@ def test_top_k_rows(bs, rows, vocab, bf16):
     w = _workload(rows, vocab, bf16, 11 * vocab + rows, topk=True)
     stats = parity.compare(w, parity.run_gpu(bs, w, want_topk=256))
     assert stats["boundary_draws"] <= 1
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("top_k,run", [(1, 2), (4, 2), (31, 5), (40, 31), (40, 40), (100, 2)])
+def test_penalised_logits_that_come_out_equal(bs, top_k, run, bf16):
+    """Pairs like 11 / 1.1^2 and 10 / 1.1 among the best, and runs of equal values up to and beyond what is
+    ordered in place: the order among them is that of the raw logits."""
+    rows, vocab = 3, 33000
+    rng = np.random.default_rng(top_k)
+    x = rng.normal(0, 1.0, (rows, vocab)).astype(np.float32)
+    hist = []
+    for r in range(rows):
+        tok = rng.permutation(vocab)[: 2 * run + 12]
+        x[r, tok[:run]], x[r, tok[run:2 * run]] = 11.0, 10.0
+        x[r, tok[2 * run:]] = np.repeat(np.float32([22, 20, 5.5, 5, 8.8125, 8.0]), 2)
+        h = np.concatenate([np.repeat(tok[:run], 2), tok[run:2 * run], np.repeat(tok[2 * run::2], 2), tok[2 * run + 1::2]])
+        hist.append(rng.permutation(h))
+    p = W._params(rows, repetition_penalty=1.1)
+    p["temperature"], p["top_p"], p["top_k"], p["repeat_last_n"] = 1.0, 0.999, top_k, 256
+    ids, off = W._csr(np.array(hist))
+    w = W.SampleWorkload("ties", W.to_bf16_bits(x) if bf16 else x, p, W.uniforms24(rng, rows), ids, off)
+    parity.compare(w, parity.run_gpu(bs, w, want_topk=100))
