@@ -565,7 +565,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     int launches = 0;
     int row_grid = 0;
     FlatRow *fr = (FlatRow *)h->flat_rows.p;
-    const RowWs rw{(float *)(x.beside ? h->dr_e : h->fw_e).p, x.beside ? nullptr : (int32_t *)h->fw_ids.p, h->escratch_stride,
+    const RowWs rw{(float *)(x.beside ? h->fw_ids : h->fw_e).p, x.beside ? nullptr : (int32_t *)h->fw_ids.p, h->escratch_stride,
                    (int32_t *)(x.beside ? h->dr_redo : h->fw_redo).p};
     const bool flat_chunks = pl.flat && n_chunk_items > 0, flat_full = pl.flat_full && n_rows_items > 0;
     auto launch_rows_kernel = [&](bool redo_only, cudaStream_t on) {
@@ -575,7 +575,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         r.work_counter = (uint32_t *)h->work_counter.p + 1;
         r.work_base = h->work_base_rows;
         if (redo_only) { r.redo_flags = rw.redo; r.redo_stride = 1; r.static_items = 1; }
-        row_grid = std::min(n_rows_items, h->sm_count);
+        row_grid = std::min(n_rows_items, x.beside ? StgSampler_::kDraftRedoCtas : h->sm_count);
         cudaError_t er = launch_sample_rows(r, row_grid, on);
         if (er == cudaSuccess) { if (!redo_only) h->work_base_rows += (uint32_t)n_rows_items + (uint32_t)row_grid; launches++; }
         return er;
@@ -764,7 +764,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
 // every device buffer a handle owns
 std::vector<DevBuf *> all_buffers(StgHandle h)
 {
-    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->fw_ids, &h->dr_redo, &h->dr_e,
+    return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->fw_ids, &h->dr_redo,
             &h->dr_escratch, &h->dr_keyscratch, &h->dr_listscratch, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
             &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
             &h->st_mask, &h->st_logits, &h->o_tokens, &h->o_probs, &h->o_flags, &h->o_topk_ids, &h->o_topk_vals, &h->o_topk_probs,
@@ -836,10 +836,10 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
     A(h->listscratch, (size_t)h->sm_count * (h->key_stride + 512) * 8);  // + 2 sub-tiles: padded reads
     if (cfg->max_spec_draft > 0) {
         A(h->dr_redo, (size_t)h->full_cap * 4);
-        A(h->dr_e, (size_t)h->full_cap * (size_t)h->escratch_stride * 4);
-        A(h->dr_escratch, h->escratch.bytes);
-        A(h->dr_keyscratch, h->keyscratch.bytes);
-        A(h->dr_listscratch, h->listscratch.bytes);
+        const size_t n = StgSampler_::kDraftRedoCtas;
+        A(h->dr_escratch, n * h->escratch_stride * 4);
+        A(h->dr_keyscratch, n * h->key_stride * 8);
+        A(h->dr_listscratch, n * (h->key_stride + 512) * 8);
     }
     A(h->st_hist, R * std::max<size_t>(cfg->max_history, 1) * 4);
     A(h->ring_ids, R * std::max<size_t>(cfg->max_history, 1) * 4);

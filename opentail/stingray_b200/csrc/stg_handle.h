@@ -88,8 +88,10 @@ struct StgSampler_ {
     stg::DevBuf flat_rows;               // FlatRow per row (stg_flat.cuh)
     // full-vocabulary rows: RowWs arrays (stg_row.cuh) for up to full_cap rows
     stg::DevBuf fw_redo, fw_e, fw_ids;
-    // the same (and the row kernel's scratch) for the draft rows of a speculative step, which run beside the target rows
-    stg::DevBuf dr_redo, dr_e, dr_escratch, dr_keyscratch, dr_listscratch;
+    // what the draft rows of a speculative step need of their own beside the target rows: redo flags and scratch for
+    // kDraftRedoCtas CTAs of the row kernel; their exp values lie in fw_ids, which only masked sampling rows use
+    static constexpr int kDraftRedoCtas = 16;
+    stg::DevBuf dr_redo, dr_escratch, dr_keyscratch, dr_listscratch;
     int full_cap = 0;
     stg::DevBuf cand, cand_count, tickets, work_counter, escratch, keyscratch, listscratch, dists;
     stg::DevBuf st_hist, st_bias_ids, st_bias_vals, st_uniforms, st_mask, st_logits;
