@@ -799,10 +799,7 @@ __device__ __forceinline__ int cut_bins(RowSh &sh, unsigned char *dyn, float top
         }
         if (lane == 0) {
             sh.stop = redo ? 1 : (more >= 0 ? 2 : 0);
-            if (more >= 0) {
-                sh.new_bits[more >> 5] |= 1u << (more & 31);
-                sh.tie_bits[more >> 5] |= 1u << (more & 31);
-            }
+            if (more >= 0) sh.new_bits[more >> 5] |= 1u << (more & 31);  // not tie_bits: another CTA may still be reading those
             sh.tstar = tstar;
             sh.hit_keep = keep < all ? keep : 0;
             if (!redo && hit >= 0 && (s - top_p <= kNearTol || top_p - before <= kNearTol)) sh.flags |= kFlagNearCut;
@@ -1422,8 +1419,15 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         cl.sync();
         tick(tk, 7);
         for (int round = 0;; round++) {
-            // bins with an exact rounding tie, or that the sum asked for: their order counts too
-            if (tid < kBins / 32) sh.new_bits[tid] = round == 0 ? sh0->tie_bits[tid] : sh0->new_bits[tid];
+            // bins with an exact rounding tie, or that the sum asked for: their order counts too.  Whether there are any
+            // decides about the barrier below, so every CTA has to see the same bits: rank 0's tie_bits stand still
+            // from the barrier above until all have passed the one that ends the first round, and its
+            // new_bits from there to the barrier in the block (a further round always has a bit).
+            if (tid < kBins / 32) {
+                const unsigned bits = round == 0 ? sh0->tie_bits[tid] : sh0->new_bits[tid];
+                sh.new_bits[tid] = bits;
+                if (rank == 0 && round > 0) sh.tie_bits[tid] |= bits;
+            }
             if (__syncthreads_or(tid < kBins / 32 && sh.new_bits[tid] != 0u)) {
                 if (rank != 0) {
                     if (tid == 0) sh.list_n = 0;
