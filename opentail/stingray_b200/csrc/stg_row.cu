@@ -818,6 +818,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     extern __shared__ __align__(128) unsigned char dyn[];
     __shared__ RowSh sh;
     cg::cluster_group cl = cg::this_cluster();
+    cl.barrier_arrive();  // waited for before the first push: another CTA's shared memory is there once that CTA runs
     const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int fi = blockIdx.x / C;
@@ -868,7 +869,8 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     int32_t *ids = nullptr;
     int first_id = 0;  // of this CTA's allowed tokens, in the closed-up row
     int *tile_at = (int *)sh.tile_sum;
-    if (CLOSE && src.mrow != nullptr && !greedy && a.mode == 0) {
+    const bool counted = CLOSE && src.mrow != nullptr && !greedy && a.mode == 0;  // the same for every thread of the cluster
+    if (counted) {
         for (int t = t0 + warp; t < t1; t += kRW) {
             const int base = t * kSub + lane * 32;
             uint32_t w = 0u;
@@ -880,6 +882,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
             if (lane == 0) tile_at[t - t0] = c;
         }
         __syncthreads();
+        cl.barrier_wait();
         if (warp == 0) {
             int run = 0;
             for (int b = 0; b < t1 - t0; b += 32) {
@@ -904,6 +907,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     // P1: the maximum
     {
         float best = -CUDART_INF_F;
+        u64 key = 0ull, raw = 0ull;
         if (CLOSE && ids != nullptr) {
             for (int t = t0 + warp; t < t1; t += kRW) {
                 const int base = t * kSub + lane * 8;
@@ -924,11 +928,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                     }
             }
             best = block_max_f(best, sh.red_f);
-            if (tid < C) {
-                RowSh *o = cl.map_shared_rank(&sh, tid);
-                o->maxkey[rank] = best > -CUDART_INF_F ? make_key(best, 0) : 0ull;
-                o->rawkey[rank] = 0ull;
-            }
+            if (best > -CUDART_INF_F) key = make_key(best, 0);
             nsub = (n + kSub - 1) / kSub;
             per = (nsub + C - 1) / C;
             t0 = min(rank * per, nsub);
@@ -951,14 +951,9 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                 for (int j = 0; j < 8; j++)
                     if (x[j] > best) { best = x[j]; best_i = base + j; }
             }
-            const u64 k = block_max_k(best_i >= 0 ? make_key(best, best_i) : 0ull, sh.red_k);
+            key = block_max_k(best_i >= 0 ? make_key(best, best_i) : 0ull, sh.red_k);
             __syncthreads();
-            const u64 rk = block_max_k(rbest_i >= 0 ? make_key(rbest, rbest_i) : 0ull, sh.red_k);
-            if (tid < C) {
-                RowSh *o = cl.map_shared_rank(&sh, tid);
-                o->maxkey[rank] = k;
-                o->rawkey[rank] = rk;
-            }
+            raw = block_max_k(rbest_i >= 0 ? make_key(rbest, rbest_i) : 0ull, sh.red_k);
         } else {
             // unscaled: multiplying by 1 / T > 0 and rounding is monotonic, so the maximum is scaled at the end
             for (int t = t0 + warp; t < t1; t += 2 * kRW) {
@@ -981,11 +976,13 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
             }
             best = block_max_f(best, sh.red_f);
             if (src.scale) best = __fmul_rn(best, src.inv_t);
-            if (tid < C) {
-                RowSh *o = cl.map_shared_rank(&sh, tid);
-                o->maxkey[rank] = best > -CUDART_INF_F ? make_key(best, 0) : 0ull;
-                o->rawkey[rank] = 0ull;
-            }
+            if (best > -CUDART_INF_F) key = make_key(best, 0);
+        }
+        if (!counted) cl.barrier_wait();
+        if (tid < C) {
+            RowSh *o = cl.map_shared_rank(&sh, tid);
+            o->maxkey[rank] = key;
+            o->rawkey[rank] = raw;
         }
         cl.sync();
     }
@@ -1675,6 +1672,7 @@ __global__ void __launch_bounds__(kRT, 2) k_spec_row(const __grid_constant__ Spe
         if (lane == 0) { s_acc = acc; s_bad = bad_draft ? 1 : 0; }
     }
     if (greedy) return;
+    cl.barrier_arrive();  // waited for before the first push, as in k_row
     __syncthreads();
     const int acc = s_acc;
     const bool residual = !(acc == L || a.mode == 1);
@@ -1713,6 +1711,7 @@ __global__ void __launch_bounds__(kRT, 2) k_spec_row(const __grid_constant__ Spe
         }
     }
     __syncthreads();
+    cl.barrier_wait();
     if (warp == 0) {
         double v = 0.0;
         for (int t = lane; t < t1 - t0; t += 32) v += (double)sh.tile_sum[t];

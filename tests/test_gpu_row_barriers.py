@@ -1,5 +1,5 @@
-"""The cluster barriers of the full-vocabulary kernels (stg_row.cu): the rounds in which the nucleus sum asks for a
-histogram bin whose order it was not expected to need."""
+"""The cluster barriers of the full-vocabulary kernels (stg_row.cu), on rows that put the least work between them, and the
+rounds in which the nucleus sum asks for a histogram bin whose order it was not expected to need."""
 import numpy as np
 import pytest
 
@@ -70,3 +70,20 @@ def test_a_sum_that_asks_for_more_bins(bs, rows, vocab):
     for _ in range(3):
         stats = parity.compare(w, parity.run_gpu(bs, w))
         assert stats["boundary_draws"] <= 1
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows,vocab", [(1, 4096), (1, 262144), (12, 33001), (40, 151936), (150, 32000), (310, 4095)])
+def test_rows_of_a_few_allowed_tokens(bs, rows, vocab, bf16):
+    """Nothing to read and nothing to sum: every CTA reaches its first push to the others at once."""
+    rng = np.random.default_rng(vocab + rows)
+    x = rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)
+    mask = np.zeros((rows, (vocab + 31) // 32), np.uint32)
+    for r in range(rows):
+        for t in rng.integers(0, vocab, 1 + r % 3):
+            mask[r, t >> 5] |= np.uint32(1) << np.uint32(t & 31)
+    p = W._params(rows, temperature=0.8)
+    p["top_p"] = rng.choice(np.array([0.7, 0.95, 1.0], np.float32), rows)
+    w = W.SampleWorkload("few", W.to_bf16_bits(x) if bf16 else x, p, W.uniforms24(rng, rows), None, None, mask)
+    stats = parity.compare(w, parity.run_gpu(bs, w))
+    assert stats["boundary_draws"] <= 1
