@@ -575,9 +575,8 @@ __device__ __forceinline__ void plan_bins(RowSh &sh, unsigned char *dyn, float t
         for (int j = 0; j < 8; j++) {
             const unsigned pb = kBinBase + (unsigned)(b0 + 7 - j);  // upper 16 bits of the bin's values
             lc[j] = m[j] ? max(1, (int)((float)m[j] / (4111.5f + 32.f * (float)(pb & 127u)) + 0.5f)) : 0;
-            // the mantissas were cut: half a unit each for those whose lower bits are not known
-            lm[j] = ((double)m[j] + 0.5 * (double)max(lc[j] - (int)(h[j] >> 20), 0) + (double)(h[j] & 0xFFFFFu) * (1.0 / 2048.0)) *
-                    pow2_double((int)(pb >> 7) - 139) * scale_p;
+            // the mantissas were cut: half a unit each, and what those whose lower bits are known have above or below it
+            lm[j] = ((double)m[j] + 0.5 * (double)lc[j] + (double)(int)h[j] * (1.0 / 2048.0)) * pow2_double((int)(pb >> 7) - 139) * scale_p;
             tm += lm[j];
             tc += lc[j];
         }
@@ -1103,9 +1102,9 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     tick(tk, 4);
 
     // P3: the exact sum on rank 0's first warp; the histogram of the exp values everywhere else.  Masses are of
-    // the upper 13 mantissa bits, completed by the lower 11 (in the increments' array, with their count) of the
-    // few values that weigh something.  Values below tau are left out: all of them together cannot be more
-    // than half of what the nucleus may leave behind.
+    // the upper 13 mantissa bits, completed by the lower 11 (less their middle, in the increments' array) of the at
+    // most 16,383 values that weigh something: their signed sum stays within 2^24.  Values below tau are left
+    // out: all of them together cannot be more than half of what the nucleus may leave behind.
     const float minp_e = min_p > 0.f ? min_p * (1.0f - 1.0f / 1024.0f) : 0.f;
     const float tau = 0.5f * (1.0f - top_p) * (float)(all / (double)n);
     if (rank == 0 && warp == 0) {
@@ -1128,7 +1127,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                         const uint32_t eb = __float_as_uint(x[u][j]), m = (eb & 0x7FFFFFu) | 0x800000u;
                         const int b = row_bin(eb);
                         atomicAdd(&mass[b], m >> 11);
-                        if (x[u][j] > heavy_e) atomicAdd(&dd[b], (m & 2047u) | (1u << 20));
+                        if (x[u][j] > heavy_e) atomicAdd(&dd[b], (m & 2047u) - 1024u);
                     }
             }
         }

@@ -79,3 +79,43 @@ def test_penalised_logits_that_come_out_equal(bs, top_k, run, bf16):
     ids, off = W._csr(np.array(hist))
     w = W.SampleWorkload("ties", W.to_bf16_bits(x) if bf16 else x, p, W.uniforms24(rng, rows), ids, off)
     parity.compare(w, parity.run_gpu(bs, w, want_topk=100))
+
+
+def _row_of_many_equal_top_logits(rng, vocab):
+    """Over a thousand tokens of one exp value just above 1/4 whose lower mantissa bits are high - together more than 20 bits
+    hold - bring the sum of the probabilities to just above 1/2; behind them a few single tokens, then half of the mass in
+    bins of two or three hundred.  Those differ a little: of hundreds of equal addends half a unit of the sum off its grid, a
+    last bit of exp decides the rounding of all."""
+    v = 0.25 + 2000.0 * 2.0 ** -25
+    while True:
+        n, over = int(rng.integers(1055, 1110)), rng.uniform(7e-5, 9e-5)
+        total = 2.0 * (1.0 + n * v) / (1.0 + over)
+        if abs((v / total * 2.0 ** 25 + 0.5) % 1.0 - 0.5) < 0.03:  # the sequential sum stays close to the real one
+            break
+    bins = 0.0078125 * 2.0 ** (-(np.arange(260) // 128)) * (1.0 - (np.arange(260) % 128 + 0.5) / 256.0)
+    single, rest = bins[:8], bins[8:]
+    counts = np.full(rest.size, int((total - 1.0 - n * v) / rest.sum()))
+    left = total - 1.0 - n * v - single.sum() - (counts * rest).sum()
+    for i in range(rest.size):  # what is missing, a token at a time
+        more = int(left / rest[i]) if i + 40 > rest.size else min(int(left / rest[i]), 1)
+        counts[i] += more
+        left -= more * rest[i]
+    rest = np.repeat(rest, counts)
+    e = np.concatenate([[1.0], np.full(n, v), single, rest * (1.0 + rng.uniform(-1e-3, 1e-3, rest.size))])
+    x = np.full(vocab, -80.0, np.float32)
+    x[:e.size] = np.log(e)
+    return rng.permutation(x)
+
+
+@pytest.mark.parametrize("rows", [1, 20, 80])
+def test_a_thousand_equal_top_logits(bs, rows):
+    """The histogram's masses of such a row have to be good to 6e-5 for the binades of the nucleus sum to be known, else the
+    row is done twice."""
+    vocab = 131072
+    rng = np.random.default_rng(rows)
+    p = W._params(rows, top_p=0.9)
+    w = W.SampleWorkload("equal", np.stack([_row_of_many_equal_top_logits(rng, vocab) for _ in range(rows)]), p, W.uniforms24(rng, rows))
+    gpu = parity.run_gpu(bs, w)
+    stats = parity.compare(w, gpu)
+    assert stats["boundary_draws"] <= 1
+    assert not (gpu["flags"].view(np.uint32) >> 8 & 1).any()
