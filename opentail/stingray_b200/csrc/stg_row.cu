@@ -809,6 +809,95 @@ __device__ __forceinline__ int cut_bins(RowSh &sh, unsigned char *dyn, float top
     return sh.stop;
 }
 
+// s = fl(s + p) from 0, at most `count` times, until s >= target: the index of the addition that got there, -1 when none
+// does.  One thread.  Inside a binade the sum grows by the same number of units with every addition behind the first (where p
+// lies half way between two units, the first leaves the sum even, and from even sums the rounding always goes the same
+// way), so a binade takes three additions and a division.
+__device__ __forceinline__ int equal_sum(float p, int count, float target, float &s, float &before)
+{
+    s = 0.f;
+    before = 0.f;
+    for (int i = 0; i < count;) {
+        before = s;
+        s = __fadd_rn(s, p);
+        if (s >= target) return i;
+        i++;
+        const uint32_t at0 = __float_as_uint(before), at = __float_as_uint(s), next = __float_as_uint(__fadd_rn(s, p));
+        if (next == at) return -1;  // it stays there
+        if ((at0 ^ at) >> 23 || (at ^ next) >> 23) continue;
+        // floats >= 0 are ordered as their bits: as many more as stay below the target and the next binade
+        const uint32_t d = next - at, end = min(((at >> 23) + 1u) << 23, __float_as_uint(target));
+        const int k = min((int)((end - 1u - at) / d), count - i);
+        if (k > 0) {
+            s = __uint_as_float(at + (uint32_t)k * d);
+            before = __uint_as_float(at + (uint32_t)(k - 1) * d);
+            i += k;
+        }
+    }
+    return -1;
+}
+
+// A row without a finite logit.  Softmax gives each of its tokens 1 / V (Sampler.cs:452-458): the filters and the draw
+// are sums of equal addends, done by the first thread; where the distribution is asked for, every CTA of the cluster
+// writes the tokens [lo, hi) of it.  Out of line: it is over in two microseconds, and k_row has no registers to spare.
+__device__ __noinline__ void uniform_row(const SampleArgs &a, const RowPlan &rp, RowSh &sh, int row, int rank, int lo, int hi, u64 rk)
+{
+    const int tid = threadIdx.x, n = a.vocab;
+    if (tid == 0) {
+        RowDist d;
+        d.flags = kDistUniform;
+        d.uniform_p = __fdiv_rn(1.0f, (float)n);
+        d.max_x = -CUDART_INF_F;
+        d.inv_t = rp.temperature != 1.0f ? __fdiv_rn(1.0f, rp.temperature) : 1.0f;
+        d.inv1 = 1.f; d.kth = 0.f; d.inv2 = 1.f; d.minp_thr = 0.f; d.tstar = 0.f; d.inv3 = 1.f;
+        d.tie_idx_max = INT_MAX;
+        d.argmax = rk ? key_idx(rk) : 0;
+        d.sum_end = 0.f;
+        int kept = n;  // the first `kept` tokens
+        float s, before;
+        if (rp.min_p > 0.f) {
+            d.minp_thr = __fmul_rn(rp.min_p, d.uniform_p);
+            d.flags |= kDistMinP;
+            if (d.uniform_p < d.minp_thr) kept = 0;
+        }
+        if (rp.top_p < 1.0f && rp.top_p > 0.f && kept > 0) {
+            const int hit = equal_sum(d.uniform_p, n, rp.top_p, s, before);
+            d.flags |= kDistTopP;
+            if (hit >= 0) {
+                kept = hit + 1;
+                d.tstar = d.uniform_p;
+                if (s - rp.top_p <= kNearTol || rp.top_p - before <= kNearTol) sh.flags |= kFlagNearCut;
+                if (kept < n) { sh.flags |= 1u << 4; d.tie_idx_max = hit; }
+            }
+        }
+        const float s3 = (float)((double)kept * (double)d.uniform_p);
+        if (s3 > 0.f && s3 != 1.0f) { d.flags |= kDistScale3; d.inv3 = __fdiv_rn(1.0f, s3); }
+        sh.dist = d;
+        if (rank == 0) {
+            if (a.mode == 2) a.dists[row] = d;
+            if (a.mode == 1 && a.row_flags) a.row_flags[row] = kPathFull | sh.flags;
+            if (a.mode == 0 || a.mode == 3) {
+                const float u01 = a.uniforms ? __ldg(a.uniforms + row) : 0.5f;
+                const int hit = u01 > 0.f ? equal_sum(eval_p3(d.uniform_p, 0, d), kept, u01, s, before) : 0;
+                const int tok = hit >= 0 ? hit : n - 1;
+                uint32_t fl = kPathFull | sh.flags | (1u << 6);
+                if (hit < 0) fl |= 1u << 5;
+                else if (u01 > 0.f && (u01 - before <= kNearTol || s - u01 <= kNearTol)) fl |= kFlagNearBoundary;
+                a.tokens[row] = tok;
+                if (a.token_probs) a.token_probs[row] = eval_p3(d.uniform_p, tok, d);
+                if (a.row_flags) a.row_flags[row] = fl;
+                count_row_flags(a.counters, fl);
+            }
+        }
+    }
+    if ((a.mode == 1 || a.mode == 3) && a.dist_out) {
+        __syncthreads();
+        const RowDist d = sh.dist;
+        float *o = a.dist_out + (int64_t)row * n;
+        for (int i = lo + tid; i < hi; i += kRT) o[i] = eval_p3(d.uniform_p, i, d);
+    }
+}
+
 // ---- the kernel ----------------------------------------------------------------------------------------
 // CLOSE: for batches with masks (the code that closes rows up costs the other batches 3 %)
 template <bool BF16, bool CLOSE>
@@ -1018,9 +1107,13 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         }
         return;
     }
-    // nothing finite: Softmax's 1/V case (Sampler.cs:452-458), left to the row kernel
-    if (mk == 0ull || a.lookback_drill == 1) {
+    if (a.lookback_drill == 1) {
         if (rank == 0 && tid == 0) ws.redo[fi] = 1;
+        return;
+    }
+    if (mk == 0ull) {  // nothing finite; [t0, t1) may be tiles of the closed-up row, but that is of no distribution
+        if (rank == 0 && tid == 0) ws.redo[fi] = 0;
+        uniform_row(a, rp, sh, row, rank, t0 * kSub, min(n, t1 * kSub), rk);
         return;
     }
     const float mx = key_val(mk);
