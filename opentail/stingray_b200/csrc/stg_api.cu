@@ -514,9 +514,9 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     a.lookback_drill = h->lookback_drill;
     a.phase_ticks = (unsigned long long *)h->ticks.p;
     h->ticks_items = (int)pl.items.size();
-    a.escratch = (float *)(x.beside ? h->dr_escratch : h->escratch).p;
-    a.keyscratch = (unsigned long long *)(x.beside ? h->dr_keyscratch : h->keyscratch).p;
-    a.listscratch = (unsigned long long *)(x.beside ? h->dr_listscratch : h->listscratch).p;
+    a.escratch = (float *)h->escratch.p + x.scratch_first * h->escratch_stride;
+    a.keyscratch = (unsigned long long *)h->keyscratch.p + x.scratch_first * h->key_stride;
+    a.listscratch = (unsigned long long *)h->listscratch.p + x.scratch_first * (h->key_stride + 2 * kSub);
     a.dists = x.dists_out;
     // vocabulary-sharded mode: one block per rank, [rows, stride] keys followed by [rows] counts,
     // with the stride of this step (its largest selection count), so that one all-gather of
@@ -575,7 +575,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         r.work_counter = (uint32_t *)h->work_counter.p + 1;
         r.work_base = h->work_base_rows;
         if (redo_only) { r.redo_flags = rw.redo; r.redo_stride = 1; r.static_items = 1; }
-        row_grid = std::min(n_rows_items, x.beside ? StgSampler_::kDraftRedoCtas : h->sm_count);
+        row_grid = std::min(n_rows_items, x.scratch_rows > 0 ? x.scratch_rows : h->sm_count);
         cudaError_t er = launch_sample_rows(r, row_grid, on);
         if (er == cudaSuccess) { if (!redo_only) h->work_base_rows += (uint32_t)n_rows_items + (uint32_t)row_grid; launches++; }
         return er;
@@ -765,8 +765,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
 std::vector<DevBuf *> all_buffers(StgHandle h)
 {
     return {&h->plans[0].dev, &h->plans[1].dev, &h->flat_rows, &h->fw_redo, &h->fw_e, &h->fw_ids, &h->dr_redo,
-            &h->dr_escratch, &h->dr_keyscratch, &h->dr_listscratch, &h->cand, &h->cand_count, &h->tickets, &h->work_counter,
-            &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
+            &h->cand, &h->cand_count, &h->tickets, &h->work_counter, &h->escratch, &h->keyscratch, &h->listscratch, &h->dists, &h->st_hist, &h->st_bias_ids, &h->st_bias_vals, &h->st_uniforms,
             &h->st_mask, &h->st_logits, &h->o_tokens, &h->o_probs, &h->o_flags, &h->o_topk_ids, &h->o_topk_vals, &h->o_topk_probs,
             &h->o_pairs, &h->ticks, &h->ring_ids, &h->ring_len_dev, &h->mc_words, &h->mc_slots, &h->sp_draft, &h->sp_uniforms,
             &h->sp_accepted, &h->sp_correction, &h->sp_aprobs, &h->sp_flags, &h->sp_rowstats, &h->xchg_local, &h->xchg_gather};
@@ -833,14 +832,8 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
     A(h->work_counter, 256);
     A(h->escratch, (size_t)h->sm_count * h->escratch_stride * 4);
     A(h->keyscratch, (size_t)h->sm_count * h->key_stride * 8);
-    A(h->listscratch, (size_t)h->sm_count * (h->key_stride + 512) * 8);  // + 2 sub-tiles: padded reads
-    if (cfg->max_spec_draft > 0) {
-        A(h->dr_redo, (size_t)h->full_cap * 4);
-        const size_t n = StgSampler_::kDraftRedoCtas;
-        A(h->dr_escratch, n * h->escratch_stride * 4);
-        A(h->dr_keyscratch, n * h->key_stride * 8);
-        A(h->dr_listscratch, n * (h->key_stride + 512) * 8);
-    }
+    A(h->listscratch, (size_t)h->sm_count * (h->key_stride + 2 * kSub) * 8);  // + 2 sub-tiles: padded reads
+    if (cfg->max_spec_draft > 0) A(h->dr_redo, (size_t)h->full_cap * 4);
     A(h->st_hist, R * std::max<size_t>(cfg->max_history, 1) * 4);
     A(h->ring_ids, R * std::max<size_t>(cfg->max_history, 1) * 4);
     A(h->ring_len_dev, R * 4);

@@ -88,10 +88,11 @@ struct StgSampler_ {
     stg::DevBuf flat_rows;               // FlatRow per row (stg_flat.cuh)
     // full-vocabulary rows: RowWs arrays (stg_row.cuh) for up to full_cap rows
     stg::DevBuf fw_redo, fw_e, fw_ids;
-    // what the draft rows of a speculative step need of their own beside the target rows: redo flags and scratch for
-    // kDraftRedoCtas CTAs of the row kernel; their exp values lie in fw_ids, which only masked sampling rows use
-    static constexpr int kDraftRedoCtas = 16;
-    stg::DevBuf dr_redo, dr_escratch, dr_keyscratch, dr_listscratch;
+    // what the draft rows of a speculative step need of their own beside the target rows: redo flags.  Their exp values lie
+    // in fw_ids, which only masked sampling rows use, and their CTAs of the row kernel take the last draft_redo_ctas()
+    // of the sm_count scratch rows below, which the target rows' leave to them
+    stg::DevBuf dr_redo;
+    int draft_redo_ctas() const { return std::max(1, std::min(16, sm_count / 2)); }
     int full_cap = 0;
     stg::DevBuf cand, cand_count, tickets, work_counter, escratch, keyscratch, listscratch, dists;
     stg::DevBuf st_hist, st_bias_ids, st_bias_vals, st_uniforms, st_mask, st_logits;
@@ -147,6 +148,8 @@ struct BatchExtra {
     int global_vocab = 0;         // 0: same as the batch's vocab
     int plan_slot = 0;            // StgSampler_::plans
     bool beside = false;          // mode 2: runs beside another pass on the handle's side stream, in the draft rows' scratch
+    int scratch_first = 0;        // the scratch rows that this pass's CTAs of the row kernel may take: from this one on,
+    int scratch_rows = 0;         // so many; 0: all
     bool want_argmax = false;     // mode 2: the arg-max of the raw rows goes with the descriptors
 };
 // puts what follows on `stream` behind everything the handle has enqueued on another stream

@@ -151,6 +151,11 @@ int stg_spec_verify(StgHandle h, const StgSpecBatch *b, void *stream_)
         x.dists_out = which == 0 ? tdist : ddist;
         x.plan_slot = which;
         x.beside = beside && which == 1;
+        if (beside) {  // both passes may have rows to redo: the draft rows' CTAs take the last scratch rows
+            const int d = h->draft_redo_ctas();
+            x.scratch_first = which == 1 ? h->sm_count - d : 0;
+            x.scratch_rows = which == 1 ? d : h->sm_count - d;
+        }
         x.want_argmax = b->mode == 1;  // the looser accept rule compares against it
         return run_batch(h, &sb, x, on);
     };

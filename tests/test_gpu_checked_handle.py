@@ -117,3 +117,42 @@ def test_a_look_back_that_runs_out_costs_a_second_pass_not_the_result(drilled_pa
         assert bs.stats()["reread_rows"] >= int(full.sum())
     finally:
         bs.close()
+
+
+def test_target_and_draft_rows_redone_side_by_side():
+    """Both descriptor passes of a speculative step have every row redone at once, in the same scratch rows: more target
+    rows than their share of it, more draft rows than theirs."""
+    from opentail.stingray_b200 import workloads as W
+    from tests.test_gpu_spec_shard import _check_spec
+
+    rng = np.random.default_rng(12)
+    n, L, vocab = 44, 3, 20011
+    draft = rng.normal(0, 2.5, (n, L, vocab)).astype(np.float32)
+    target = np.concatenate([draft + rng.normal(0, 0.5, draft.shape), rng.normal(0, 2.5, (n, 1, vocab))], 1).astype(np.float32)
+    p = W._params(n, temperature=0.9)
+    p["top_p"][::2] = 0.95
+    w = W.SpecWorkload("redo", target, draft, draft.argmax(-1).astype(np.int32), p, rng.random((n, L + 2)))
+    os.environ["STG_LOOKBACK_DRILL"] = "1"
+    try:
+        for _ in range(2):
+            _check_spec(w)
+    finally:
+        del os.environ["STG_LOOKBACK_DRILL"]
+
+
+def test_a_handle_for_drafts_costs_little_more():
+    """What a handle with room for draft tokens takes more than one without: descriptors and small arrays, no rows of V."""
+    import torch
+    from opentail.stingray_b200 import BatchSampler
+
+    def taken(**kw):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        bs = BatchSampler(max_rows=8, max_vocab=262144, max_history=8, max_top_k=8, **kw)
+        try:
+            return before - torch.cuda.mem_get_info()[0]
+        finally:
+            bs.close()
+
+    taken()  # the library's own context and modules
+    assert taken(max_spec_draft=7) - taken() <= 16 << 20
