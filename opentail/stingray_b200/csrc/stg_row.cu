@@ -1198,7 +1198,9 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     // the upper 13 mantissa bits, completed by the lower 11 (less their middle, in the increments' array) of the at
     // most 16,383 values that weigh something: their signed sum stays within 2^24.  Values below tau are left
     // out: all of them together cannot be more than half of what the nucleus may leave behind.
-    const float minp_e = min_p > 0.f ? min_p * (1.0f - 1.0f / 1024.0f) : 0.f;
+    // Values below minp_e cannot reach min-p's threshold, whatever the sum is: fl(e * inv) >= fl(min_p * inv) takes an
+    // e >= min_p * (1 - 2^-23).  A mass that holds more than the survivors' makes the bound too high.
+    const float minp_e = min_p > 0.f ? min_p * (1.0f - 1.0f / 1048576.0f) : 0.f;
     const float tau = 0.5f * (1.0f - top_p) * (float)(all / (double)n);
     if (rank == 0 && warp == 0) {
         const WalkOut o = row_walk(wa, get_e, n, nsub, 0.f, false);

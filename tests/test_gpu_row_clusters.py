@@ -119,3 +119,22 @@ def test_a_thousand_equal_top_logits(bs, rows):
     stats = parity.compare(w, gpu)
     assert stats["boundary_draws"] <= 1
     assert not (gpu["flags"].view(np.uint32) >> 8 & 1).any()
+
+
+@pytest.mark.parametrize("below", [1e-4, 9e-4])
+@pytest.mark.parametrize("rows,vocab", [(1, 300), (7, 40000)])
+def test_min_p_leaves_less_than_top_p(bs, rows, vocab, below):
+    """A token a little below min-p's threshold, whose mass is what the survivors lack to top_p: the sum never gets there and
+    every survivor stays.  Nothing has to be done twice for that."""
+    rng = np.random.default_rng(vocab)
+    p = W._params(rows)
+    x = np.full((rows, vocab), -40.0, np.float32)
+    for r in range(rows):
+        min_p = np.float32(rng.uniform(0.01, 0.1))
+        e = np.concatenate([[1.0], rng.uniform(1.5 * min_p, 0.9, 12), [min_p * (1.0 - below)], rng.uniform(0, 0.3 * min_p, 100)])
+        x[r, rng.permutation(vocab)[: e.size]] = np.log(e)
+        p["min_p"][r], p["top_p"][r] = min_p, (e[:13].sum() + 0.5 * e[13]) / e.sum()
+    w = W.SampleWorkload("min_p", x, p, W.uniforms24(rng, rows))
+    gpu = parity.run_gpu(bs, w)
+    parity.compare(w, gpu)
+    assert not (gpu["flags"].view(np.uint32) >> 8 & 1).any()
