@@ -512,6 +512,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     a.counters = (unsigned long long *)h->work_counter.p + 16;  // bytes 128..191 of the same small buffer
     a.softcap = b->logit_softcap;
     a.lookback_drill = h->lookback_drill;
+    a.sm_count = h->sm_count;
     a.phase_ticks = (unsigned long long *)h->ticks.p;
     h->ticks_items = (int)pl.items.size();
     a.escratch = (float *)h->escratch.p + x.scratch_first * h->escratch_stride;

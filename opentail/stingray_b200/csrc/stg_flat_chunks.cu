@@ -33,7 +33,7 @@ __global__ void __launch_bounds__(kFlatThreads, STG_CHUNKS_MB) k_flat_stream_chu
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, CAP ? a.softcap : 0.f};
     const bool mine = __ldg(&rpp->n_chunks) != 0 && begin < end;
     // While the rows' bounds are still being found: the pieces of the CTAs that are resident by then, into L2.
-    if (mine && blockIdx.y * gridDim.x + blockIdx.x < 148u * STG_CHUNKS_MB)
+    if (mine && blockIdx.y * gridDim.x + blockIdx.x < (unsigned)a.sm_count * STG_CHUNKS_MB)
         for (int i = begin + tid * (128 / esz); i < end; i += kFlatThreads * (128 / esz))
             asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)rowp.p + (int64_t)i * esz));
     pdl_release();
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kFlatThreads, STG_CHUNKS_MB) k_flat_stream_chu
 cudaError_t launch_flat_stream_chunks(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
 {
     const int pieces = (a.vocab + kFlatPiece - 1) / kFlatPiece;
-    const bool few = (long long)pieces * a.n_items < 2 * 148;
+    const bool few = (long long)pieces * a.n_items < 2 * a.sm_count;
     const dim3 grid((unsigned)(few ? (a.vocab + 4095) / 4096 : pieces), (unsigned)a.n_items);
     const bool cap = a.softcap != 0.f;
     void (*fn)(const SampleArgs, FlatRow *);

@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kFlatThreads, 5) k_greedy_step(const __grid_co
 cudaError_t launch_greedy_step(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
 {
     const int pieces = (a.vocab + kFlatPiece - 1) / kFlatPiece;
-    const bool few = (long long)pieces * a.n_items < 2 * 148;
+    const bool few = (long long)pieces * a.n_items < 2 * a.sm_count;
     const dim3 grid((unsigned)(few ? (a.vocab + 4095) / 4096 : pieces), (unsigned)a.n_items);
     const bool cap = a.softcap != 0.f;
     void (*fn)(const SampleArgs, FlatRow *);

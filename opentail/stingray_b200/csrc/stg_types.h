@@ -123,6 +123,7 @@ struct SampleArgs {
     int32_t n_ranks;
     unsigned long long *counters;    // kCtr* event counters, never null
     float softcap;                   // != 0: every logit is read as tanh(x / softcap) * softcap
+    int32_t sm_count;                // of the device
     int32_t finish_cap;              // candidates per buffer of the half-size finish (stg_flat_finish_half.cu)
     int32_t static_items;            // row kernel: CTA b takes items b, b + grid, ... (no work counter: the launch can be replayed)
     int32_t lookback_drill;          // STG_LOOKBACK_DRILL at stg_create: k_row gives every row up before its sum (1) or at its draw (2)
