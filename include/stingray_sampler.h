@@ -24,10 +24,10 @@
  * event, no host wait), which must therefore still exist.  Inputs and outputs follow the usual
  * rule: they must be ready on, and are ready after, the stream of the call that uses them.
  *
- * Repeated steps: a decode loop calls stg_sample_batch with the same buffers and the same per-row
+ * Repeated steps: a decode loop calls stg_sample_rows with the same buffers and the same per-row
  * parameters step after step, only the contents of the buffers change.  The second time the library
  * sees such a call on a stream that can be captured (any stream but the legacy default stream, which
- * CUDA cannot capture) it records the step's launches - a dozen kernels on three streams - as a CUDA
+ * CUDA cannot capture) it records the step's launches - up to five kernels on two streams - as a CUDA
  * graph, and from then on submits the step as one graph launch.  Nothing changes for the caller;
  * StgStats.graph_replays counts those steps, and STG_NO_GRAPH=1 in the environment at stg_create turns
  * the mechanism off.  Steps with host-memory inputs are never captured.

@@ -147,10 +147,7 @@ int make_plan(StgHandle h, const StgSampleBatch *b, int mode, bool shard, int gl
             return fail(h, STG_ERR_UNSUPPORTED, "vocabulary-sharded mode supports top-k and plain greedy rows only");
         const bool chunked = mode == 0 && (rp.path == kPathGreedy || rp.path == kPathTopK);
         if (chunked) { n_chunk_rows++; max_sel = std::max(max_sel, rp.sel); }
-        else pl.any_row_item = true;
         if (rp.path == kPathTopK) pl.n_topk++; else if (rp.path == kPathFull) pl.n_full++; else pl.n_greedy++;
-        if (rp.path == kPathFull && !(p.top_p < 1.0f && p.top_p > 0.f)) pl.n_full_without_top_p++;
-        if (rp.path == kPathFull && p.top_p < 1.0f && p.top_p > 0.f) pl.n_full_with_top_p++;
     }
     pl.n_chunk_rows = n_chunk_rows;
     // The flat step needs long, aligned rows and a candidate list (N + kFlatSlack entries) that about 3 N
@@ -511,7 +508,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     a.work_counter = (uint32_t *)h->work_counter.p;
     a.counters = (unsigned long long *)h->work_counter.p + 16;  // bytes 128..191 of the same small buffer
     a.softcap = b->logit_softcap;
-    a.lookback_drill = h->lookback_drill;
+    a.row_drill = h->row_drill;
     a.sm_count = h->sm_count;
     a.phase_ticks = (unsigned long long *)h->ticks.p;
     h->ticks_items = (int)pl.items.size();
@@ -575,7 +572,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
         r.item_base = 0;
         r.work_counter = (uint32_t *)h->work_counter.p + 1;
         r.work_base = h->work_base_rows;
-        if (redo_only) { r.redo_flags = rw.redo; r.redo_stride = 1; r.static_items = 1; }
+        if (redo_only) { r.redo_flags = rw.redo; r.static_items = 1; }
         row_grid = std::min(n_rows_items, x.scratch_rows > 0 ? x.scratch_rows : h->sm_count);
         cudaError_t er = launch_sample_rows(r, row_grid, on);
         if (er == cudaSuccess) { if (!redo_only) h->work_base_rows += (uint32_t)n_rows_items + (uint32_t)row_grid; launches++; }
@@ -585,7 +582,7 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
     c.items = a.items + n_rows_items;
     c.n_items = n_chunk_items;
     // The launches of the step.  When this plan and these arguments (every pointer included) have been
-    // launched before, the whole sequence - three streams, their events - is captured once into a CUDA
+    // launched before, the whole sequence - both streams, their events - is captured once into a CUDA
     // graph and replayed from then on: one submission instead of a dozen, and no host time between the
     // kernels of the chain.  Only steps made of replayable launches qualify: the flat form (the
     // persistent kernels of the first design draw work from counters whose base the host advances),
@@ -630,12 +627,12 @@ int run_batch(StgHandle h, const StgSampleBatch *b, const BatchExtra &x, void *s
             constexpr int kHalfCap = 6912, kQuarterCap = 3456;  // 2 x 110,592 B, 4 x 55,296 B (+ static) fit an SM
             if (!no_small && n_chunk_items <= 2 * sms && pl.max_sel + 2048 + 512 <= kHalfCap) {
                 c.finish_cap = kHalfCap;
-                e = launch_flat_finish_half(c, fr, n_chunk_items, cs);
+                e = launch_flat_finish_half(c, fr, cs);
             } else if (!no_small && n_chunk_items <= 4 * sms && pl.max_sel + 1024 + 512 <= kQuarterCap) {
                 c.finish_cap = kQuarterCap;
-                e = launch_flat_finish_quarter(c, fr, n_chunk_items, cs);
+                e = launch_flat_finish_quarter(c, fr, cs);
             } else {
-                e = launch_flat_finish(c, fr, n_chunk_items, pl.smem, cs);
+                e = launch_flat_finish(c, fr, pl.smem, cs);
             }
             if (e == cudaSuccess) launches++;
             if (!fork) h->kt.mark("flat_finish", cs);
@@ -803,7 +800,8 @@ int stg_create(const StgConfig *cfg, StgHandle *out)
     h = new StgSampler_();
     h->cfg = *cfg;
     h->checked = getenv("STG_CHECKED") != nullptr && getenv("STG_CHECKED")[0] == '1';
-    if (const char *drill = getenv("STG_LOOKBACK_DRILL")) h->lookback_drill = drill[0] == '1' ? 1 : drill[0] == '2' ? 2 : 0;
+    for (const char *name : {"STG_LOOKBACK_DRILL", "STG_ROW_DRILL"})  // the first: its name before rows were done by clusters
+        if (const char *drill = getenv(name)) h->row_drill = drill[0] == '1' ? 1 : drill[0] == '2' ? 2 : 0;
     h->graphs_off = getenv("STG_NO_GRAPH") != nullptr;
     h->sm_count = prop.multiProcessorCount;
     h->smem_optin = prop.sharedMemPerBlockOptin > 4096 ? prop.sharedMemPerBlockOptin - 4096 : 0;

@@ -27,23 +27,15 @@ __global__ void __launch_bounds__(kThreads) k_flat_prep(const __grid_constant__ 
 }
 
 // ---- k_flat_finish ------------------------------------------------------------------------------------
-// The rows of a.items: one per CTA, or (SHARED) shared between the CTAs of a smaller grid, which
-// leaves SMs to the kernels of the full-vocabulary rows it runs beside.
-template <bool BF16, bool SHARED>
+// The rows of a.items, one per CTA.
+template <bool BF16>
 __global__ void __launch_bounds__(kThreads, 1) k_flat_finish(const __grid_constant__ SampleArgs a, FlatRow *fr)
 {
     extern __shared__ __align__(16) unsigned char arena[];
     __shared__ SelCtl ctl;
     __shared__ FlatShared fs;
     pdl_wait();
-    if (!SHARED) {
-        flat_finish_row<BF16>(a, fr, a.items[blockIdx.x].row, blockIdx.x, a.cap, arena, ctl, fs);
-        return;
-    }
-    for (int i = blockIdx.x; i < a.n_items; i += gridDim.x) {
-        flat_finish_row<BF16>(a, fr, a.items[i].row, i, a.cap, arena, ctl, fs);
-        __syncthreads();
-    }
+    flat_finish_row<BF16>(a, fr, a.items[blockIdx.x].row, blockIdx.x, a.cap, arena, ctl, fs);
 }
 
 cudaError_t launch_flat_prep(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
@@ -54,14 +46,12 @@ cudaError_t launch_flat_prep(const SampleArgs &a, FlatRow *fr, cudaStream_t stre
     return cudaGetLastError();
 }
 
-cudaError_t launch_flat_finish(const SampleArgs &a, FlatRow *fr, int grid, size_t smem, cudaStream_t stream)
+cudaError_t launch_flat_finish(const SampleArgs &a, FlatRow *fr, size_t smem, cudaStream_t stream)
 {
-    const bool shared = grid < a.n_items;
-    void (*fn)(const SampleArgs, FlatRow *) = a.dtype == 1 ? (shared ? k_flat_finish<true, true> : k_flat_finish<true, false>)
-                                                           : (shared ? k_flat_finish<false, true> : k_flat_finish<false, false>);
+    void (*fn)(const SampleArgs, FlatRow *) = a.dtype == 1 ? k_flat_finish<true> : k_flat_finish<false>;
     cudaError_t e = ensure_dynamic_smem((const void *)fn, smem);
     if (e != cudaSuccess) return e;
-    return launch_behind(fn, dim3((unsigned)grid), kThreads, smem, stream, a, fr);
+    return launch_behind(fn, dim3((unsigned)a.n_items), kThreads, smem, stream, a, fr);
 }
 
 }  // namespace stg

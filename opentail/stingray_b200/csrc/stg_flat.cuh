@@ -58,9 +58,9 @@ cudaError_t launch_flat_stream_chunks(const SampleArgs &a, FlatRow *fr, cudaStre
 // a step of plain arg-max rows only, in one launch (stg_flat_greedy.cu); needs every row's key and ticket at zero
 cudaError_t launch_greedy_step(const SampleArgs &a, FlatRow *fr, cudaStream_t stream);
 // the small-CTA finishes (512 threads, two CTAs per SM; 256 threads, four per SM; a.finish_cap entries per buffer)
-cudaError_t launch_flat_finish_half(const SampleArgs &a, FlatRow *fr, int grid, cudaStream_t stream);
-cudaError_t launch_flat_finish_quarter(const SampleArgs &a, FlatRow *fr, int grid, cudaStream_t stream);
-// grid: CTAs that share the rows of a.items between them (at most a.n_items)
-cudaError_t launch_flat_finish(const SampleArgs &a, FlatRow *fr, int grid, size_t smem, cudaStream_t stream);
+cudaError_t launch_flat_finish_half(const SampleArgs &a, FlatRow *fr, cudaStream_t stream);
+cudaError_t launch_flat_finish_quarter(const SampleArgs &a, FlatRow *fr, cudaStream_t stream);
+// one CTA of 1024 threads per row of a.items
+cudaError_t launch_flat_finish(const SampleArgs &a, FlatRow *fr, size_t smem, cudaStream_t stream);
 
 }  // namespace stg

@@ -29,7 +29,6 @@ struct Plan {
     std::vector<float> pow_tab;
     int chunk_len = 0;
     int cap = kSubTile + 1;
-    bool any_row_item = false;
     int n_row_items = 0;
     size_t smem = 0;
     uint64_t n_greedy = 0, n_topk = 0, n_full = 0;
@@ -38,8 +37,6 @@ struct Plan {
     bool flat = false;        // the chunked rows run as the flat step (stg_flat.cuh)
     bool flat_full = false;   // ... and so do the full-vocabulary rows
     int n_chunk_rows = 0;
-    int n_full_without_top_p = 0;  // sampled full-vocabulary rows with top-p off
-    int n_full_with_top_p = 0;     // ... and on
 };
 
 // The plan of the last step of a kind, as long as the batch description stays the same
@@ -77,7 +74,7 @@ struct StgSampler_ {
     uint64_t graph_tick = 0;
     uint64_t plan_version = 0;             // bumped with every new plan
     bool graphs_off = false;               // STG_NO_GRAPH=1, or a capture failed on this handle
-    int lookback_drill = 0;              // STG_LOOKBACK_DRILL=1 or 2 at creation: see SampleArgs::lookback_drill
+    int row_drill = 0;                     // STG_ROW_DRILL=1 or 2 at creation: see SampleArgs::row_drill
 
     // workspace (allocated once at creation)
     stg::PlanSlot plans[2];              // [1]: the draft rows of a speculative step, whose plan is another one than the target rows'

@@ -1107,7 +1107,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         }
         return;
     }
-    if (a.lookback_drill == 1) {
+    if (a.row_drill == 1) {
         if (rank == 0 && tid == 0) ws.redo[fi] = 1;
         return;
     }
@@ -1282,7 +1282,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     };
     // hit: the element of the row the draw met, -1: none.  One thread.
     auto write_row = [&](int hit, uint32_t fl) {
-        if (a.lookback_drill == 2) { ws.redo[fi] = 1; return; }
+        if (a.row_drill == 2) { ws.redo[fi] = 1; return; }
         int tok = hit >= 0 ? (CLOSE && ids ? ids[hit] : hit) : a.vocab - 1, at = hit >= 0 ? hit : n - 1;
         if (hit < 0) fl |= 1u << 5;
         if (!(u01 > 0.f)) { tok = 0; at = 0; fl &= ~(1u << 5); }  // the first token meets such a target whatever its probability

@@ -532,20 +532,6 @@ __device__ __forceinline__ u64 block_max_key_r(u64 k, u64 *scratch)
     return k;
 }
 
-__device__ __forceinline__ float block_max_float(float v, float *scratch)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
-    __syncthreads();
-    v = scratch[threadIdx.x & 31];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    __syncthreads();
-    return v;
-}
-
 // (max value, lowest index of it) of the source as a key; 0 when nothing is > -infinity
 template <class Src>
 static __device__ u64 pass_max(const Src &src, int n, u64 *red)
@@ -1392,7 +1378,7 @@ static __device__ void run_row(const SampleArgs &a, int row, int item, SelCtl *s
     __syncthreads();
     const RowPlan &rp = sh_rp;
     // second chance of the flat step: only the rows it flagged are run
-    if (a.redo_flags != nullptr && (rp.flat_full < 0 || a.redo_flags[(size_t)rp.flat_full * a.redo_stride] == 0)) return;
+    if (a.redo_flags != nullptr && (rp.flat_full < 0 || a.redo_flags[rp.flat_full] == 0)) return;
     const int n = a.vocab;
     const int esz = BF16 ? 2 : 4;
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, a.softcap};

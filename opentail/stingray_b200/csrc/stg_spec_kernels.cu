@@ -1,7 +1,8 @@
 // Second phase of speculative verification and the MTP accept rule.
 //
-// Phase one (k_sample in descriptor mode) leaves a RowDist per target and draft row, from which
-// p[i] and q[i] are evaluated pointwise out of the logits.  k_spec_finish then runs, per sequence,
+// Phase one (k_row in descriptor mode) leaves a RowDist per target and draft row, from which
+// p[i] and q[i] are evaluated pointwise out of the logits.  k_spec_finish then runs, for every sequence
+// that k_spec_row (stg_row.cu) did not finish,
 // the accept chain of SpeculativeDecoder.StepSampled
 // (src/OpenTail.Stingray.Engine/SpeculativeDecoder.cs:532-559) and the one draw it ends with:
 // ResampleResidual (Sampler.cs:587-618), a draw from p, or the bonus draw.  The sequential fp32

@@ -15,7 +15,6 @@ constexpr int kPowTab = 32;             // host-computed powf(rep, occ) entries 
 constexpr int kEmulItems = 8;           // consecutive elements per thread in the sequential-sum scan
 constexpr int kEmulTile = kThreads * kEmulItems;
 constexpr int kSortCap = 32768;         // top-p candidate keys sorted in shared memory
-constexpr int kHistBins = 4096;         // probability histogram bins (exponent + 4 mantissa bits)
 constexpr int kMaxOverride = 2048;      // history + bias entries per row on the full-vocabulary path
 
 constexpr uint32_t kFlagFlatRedo = 1u << 8;       // row flag: an optimistic bound failed, the row was processed twice
@@ -126,9 +125,9 @@ struct SampleArgs {
     int32_t sm_count;                // of the device
     int32_t finish_cap;              // candidates per buffer of the half-size finish (stg_flat_finish_half.cu)
     int32_t static_items;            // row kernel: CTA b takes items b, b + grid, ... (no work counter: the launch can be replayed)
-    int32_t lookback_drill;          // STG_LOOKBACK_DRILL at stg_create: k_row gives every row up before its sum (1) or at its draw (2)
+    int32_t row_drill;               // STG_ROW_DRILL at stg_create: k_row gives every row up before its sum (1) or at its draw (2)
     const int32_t *redo_flags;       // row kernel as the flat step's second chance: only rows whose flag
-    int32_t redo_stride;             // redo_flags[flat_full * redo_stride] is set are run; null: every row item
+                                     // redo_flags[flat_full] is set are run; null: every row item
 };
 
 #ifdef __CUDACC__

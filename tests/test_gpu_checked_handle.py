@@ -91,22 +91,21 @@ def test_unchecked_handles_carry_no_guards():
 
 
 @pytest.mark.parametrize("drilled_pass", ["1", "2"])
-def test_a_look_back_that_runs_out_costs_a_second_pass_not_the_result(drilled_pass):
-    """The one wait between CTAs in the library - the look-back over the pieces of a row, in the exp
-    pass (1) and in the pass over the final probabilities (2) - is bounded.  The drill makes it run out
-    without any fault: piece 0 of every row withholds its flag in the drilled pass and the wait gives
-    up after 64 polls, so every later piece times out, flags its row, and the row kernel redoes the row.  Tokens and probabilities must still be the oracle's, every
-    full-vocabulary row must report the second pass, and the handle must keep working."""
+def test_a_row_that_is_given_up_costs_a_second_pass_not_the_result(drilled_pass):
+    """k_row works with bounds that the exact sums behind them check; a row whose check fails is left to the row kernel.
+    The drill makes k_row give every row up, before its sum (1) or at its draw (2).  Tokens and probabilities
+    must still be the oracle's, every full-vocabulary row must report the second pass, and the handle must keep
+    working."""
     from opentail.stingray_b200 import BatchSampler
     from opentail.stingray_b200 import workloads as W
     from tests import parity
 
     w = W.config2(rows=24, seed=11)
-    os.environ["STG_LOOKBACK_DRILL"] = drilled_pass
+    os.environ["STG_ROW_DRILL"] = drilled_pass
     try:
         bs = BatchSampler(max_rows=w.rows, max_vocab=w.vocab, max_history=512, max_top_k=128)
     finally:
-        del os.environ["STG_LOOKBACK_DRILL"]
+        del os.environ["STG_ROW_DRILL"]
     try:
         for _ in range(2):
             gpu = parity.run_gpu(bs, w, want_topk=int(w.params["top_k"].max()))
@@ -132,12 +131,12 @@ def test_target_and_draft_rows_redone_side_by_side():
     p = W._params(n, temperature=0.9)
     p["top_p"][::2] = 0.95
     w = W.SpecWorkload("redo", target, draft, draft.argmax(-1).astype(np.int32), p, rng.random((n, L + 2)))
-    os.environ["STG_LOOKBACK_DRILL"] = "1"
+    os.environ["STG_ROW_DRILL"] = "1"
     try:
         for _ in range(2):
             _check_spec(w)
     finally:
-        del os.environ["STG_LOOKBACK_DRILL"]
+        del os.environ["STG_ROW_DRILL"]
 
 
 def test_a_handle_for_drafts_costs_little_more():

@@ -3,7 +3,7 @@ every time, whatever the handle ran before.  The sweep's batches are repeated in
 handle, on the legacy default stream (direct launches) and on a stream of the test's own (where the
 library replays repeated steps as CUDA graphs); the first run of each batch is checked against the
 oracle, every later run against the first.  Results that depend on what a CTA processed before, or
-on how three streams happened to interleave, show up here and nowhere else."""
+on how the streams happened to interleave, show up here and nowhere else."""
 import numpy as np
 import pytest
 
