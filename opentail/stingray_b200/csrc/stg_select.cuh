@@ -465,7 +465,9 @@ static __device__ void sel_stream_pass(Sel &s, const LogitRow rowp, const uint32
         int idx[4];
         load_items<VEC, BF16, true>(rowp, mrow, begin, 0, first_end, v, idx);
         sel_append_exact(s, v, idx, first_end);
-        if (c->cnt > s.n) {
+        const int cnt = c->cnt;
+        __syncthreads();  // nobody appends before all have read the count: whether it is raised has to be the same for all
+        if (cnt > s.n) {
             // optimistic bound: the first sub-tile taken as a sample of the range, tau is set where
             // about 2.5 N elements of the whole range should pass (the caller checks the outcome)
             const int n_saved = s.n;
@@ -474,13 +476,14 @@ static __device__ void sel_stream_pass(Sel &s, const LogitRow rowp, const uint32
                 const int target = (int)max(32ll, min((long long)s.n, m));
                 // the floor of 32 may exceed N: a sample with fewer keys than that (a sparse mask) keeps N,
                 // which it is known to exceed - the selection needs more keys than it is asked for
-                if (target < c->cnt) s.n = target;
+                if (target < cnt) s.n = target;
             }
             sel_raise(s);
             s.n = n_saved;
         }
     }
     int cnt0 = c->cnt;
+    __syncthreads();  // as above
     int base = first_end;
     if (base < end) {
         float va[4][4], vb[4][4];
