@@ -1369,16 +1369,20 @@ template <bool BF16>
 static __device__ void run_row(const SampleArgs &a, int row, int item, SelCtl *sctl, unsigned char *arena)
 {
     u64 *tk = a.phase_ticks ? a.phase_ticks + (int64_t)item * 32 : nullptr;
-    tick(tk, 0);
     __shared__ RowCtl rc;
     __shared__ RowPlan sh_rp;  // kept in shared memory: the row's parameters are read rarely
+    __shared__ int sh_skip;
     const int tid = threadIdx.x;
     __syncthreads();
-    if (tid == 0) sh_rp = a.plans[row];
+    if (tid == 0) {
+        sh_rp = a.plans[row];
+        // second chance of the flat step: only the rows it flagged are run.  One thread reads the flag for all.
+        sh_skip = a.redo_flags != nullptr && (sh_rp.flat_full < 0 || a.redo_flags[sh_rp.flat_full] == 0) ? 1 : 0;
+    }
     __syncthreads();
     const RowPlan &rp = sh_rp;
-    // second chance of the flat step: only the rows it flagged are run
-    if (a.redo_flags != nullptr && (rp.flat_full < 0 || a.redo_flags[rp.flat_full] == 0)) return;
+    if (sh_skip) return;
+    tick(tk, 0);
     const int n = a.vocab;
     const int esz = BF16 ? 2 : 4;
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, a.softcap};

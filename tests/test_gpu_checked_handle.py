@@ -155,3 +155,27 @@ def test_a_handle_for_drafts_costs_little_more():
 
     taken()  # the library's own context and modules
     assert taken(max_spec_draft=7) - taken() <= 16 << 20
+
+
+def test_phase_stamps_of_rows_that_were_not_redone():
+    """The stamps of a row's phases are k_row's: the redo pass behind it leaves those of the rows it skips alone."""
+    from opentail.stingray_b200 import BatchSampler
+    from opentail.stingray_b200 import workloads as W
+    from tests import parity
+
+    w = W.config2(rows=8, seed=2)
+    w.params["top_k"], w.params["top_p"], w.params["temperature"] = 0, 1.0, 1.0  # the phases of a full row, one after the other
+    os.environ["STG_PHASE_TICKS"] = "1"
+    try:
+        bs = BatchSampler(max_rows=w.rows, max_vocab=w.vocab, max_history=512, max_top_k=8)
+    finally:
+        del os.environ["STG_PHASE_TICKS"]
+    try:
+        gpu = parity.run_gpu(bs, w)
+        assert not (gpu["flags"].view(np.uint32) >> 8 & 1).any()
+        stamps, n = np.zeros((w.rows, 32), np.uint64), C.c_int32(0)
+        assert bs._lib.stg_debug_phase_ticks(bs._h, stamps.ctypes.data, w.rows, C.byref(n)) == 0 and n.value == w.rows
+        order = stamps[:, [0, 1, 2, 3, 4, 5, 10, 11, 12]].astype(np.int64)
+        assert (np.diff(order, axis=1) >= 0).all() and (order[:, -1] - order[:, 0] < 10_000_000).all()
+    finally:
+        bs.close()
