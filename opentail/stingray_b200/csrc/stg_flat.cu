@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_flat_finish(const __grid_consta
     __shared__ FlatShared fs;
     pdl_wait();
     flat_finish_row<BF16>(a, fr, a.items[blockIdx.x].row, blockIdx.x, a.cap, arena, ctl, fs);
+    __syncthreads();  // all warps leave together, as in the smaller forms (stg_flat_finish_small.inc)
 }
 
 cudaError_t launch_flat_prep(const SampleArgs &a, FlatRow *fr, cudaStream_t stream)
