@@ -15,6 +15,19 @@ pytestmark = pytest.mark.gpu
 CASES = [0, 1, 2, 3, 4, 9, 11, 69, 78, 141, 149, 171, 195]
 
 
+def _run(bs, w, dev, outs, it):
+    import torch
+
+    kw = dict(uniforms=dev["uniforms"], want_probs=True, want_flags=True, want_topk=512)
+    if w.history_ids is not None:
+        kw.update(history_ids=dev["history_ids"], history_offsets=w.history_offsets)
+    if w.mask is not None:
+        kw["mask"] = dev["mask"]
+    outs[it] = bs.sample_rows(dev["logits"], w.params, out=outs.get(it), **kw)
+    torch.cuda.synchronize()
+    return {k: v.cpu().numpy() for k, v in outs[it].items()}
+
+
 @pytest.mark.parametrize("own_stream", [False, True])
 def test_repeated_batches_in_random_order(own_stream):
     import torch
@@ -26,18 +39,22 @@ def test_repeated_batches_in_random_order(own_stream):
         with torch.cuda.stream(st):
             ws = {it: _workload(it) for it in CASES}
             devs = {it: parity.to_device(ws[it]) for it in CASES}
-            first = {}
+            first, outs = {}, {}
             rng = np.random.default_rng(7)
             for rep in range(25):
                 for it in (rng.permutation(CASES) if rep else CASES):
                     it = int(it)
-                    gpu = parity.run_gpu(bs, ws[it], devs[it], want_topk=512)
-                    if it not in first:
-                        parity.compare(ws[it], gpu)
-                        first[it] = gpu
-                        continue
-                    for key in ("tokens", "flags", "probs"):
-                        np.testing.assert_array_equal(gpu[key].view(np.uint32), first[it][key].view(np.uint32),
-                                                      err_msg=f"case {it}, repeat {rep}: {key} differ from the first run")
+                    # a step is replayed when it follows itself: a batch of another kind has another plan
+                    for _ in range(3 if own_stream else 1):
+                        gpu = _run(bs, ws[it], devs[it], outs, it)
+                        if it not in first:
+                            parity.compare(ws[it], gpu)
+                            first[it] = gpu
+                            continue
+                        for key in ("tokens", "flags", "probs"):
+                            np.testing.assert_array_equal(gpu[key].view(np.uint32), first[it][key].view(np.uint32),
+                                                          err_msg=f"case {it}, repeat {rep}: {key} differ from the first run")
+        # (a replay also needs the same output buffers, which a batch keeps here)
+        assert (bs.stats()["graph_replays"] > 100) == own_stream
     finally:
         bs.close()
