@@ -165,25 +165,31 @@ __device__ __forceinline__ bool fast_eligible(const RowPlan &rp, int cnt, size_t
            (!rp.has_penalty || (rp.rep >= 1.0f && rp.pres >= 0.f && rp.freq >= 0.f));
 }
 
-// occurrences in the history | inside the window << 16
+// Occurrences of `id` in the history | inside the window << 16.  Whole warps call it, and the warp leaves the loop
+// together, when the last of its lanes is done: with a loop that each lane left by itself the lane that had found its
+// token stayed apart from the others through the shuffles of the sort behind it, and its warp's candidates were lost
+// (rows of 262,144 bf16 logits behind 700-token histories: once in 400 to 9,000 steps, a `__syncwarp` notwithstanding).
 __device__ __forceinline__ unsigned fast_occurrences(const int *hkey, const unsigned *hcnt, int hmask, int id)
 {
     int h = (int)(((unsigned)id * 2654435761u) >> 7) & hmask;
+    int at = -1;
+    bool open = true;
 #pragma unroll 1
-    for (;;) {
+    while (__any_sync(0xFFFFFFFFu, open)) {
         const int kx = hkey[h];
-        if (kx == id) return hcnt[h];
-        if (kx == -1) return 0u;
+        at = open && kx == id ? h : at;
+        open = open && kx != id && kx != -1;
         h = (h + 1) & hmask;
     }
+    return at >= 0 ? hcnt[at] : 0u;
 }
-// the key of a candidate with the penalties applied (Sampler.cs:263-287)
+// the keys of a warp's candidates (0: none) with the penalties applied (Sampler.cs:263-287)
 __device__ __forceinline__ u64 fast_penalise(u64 key, const int *hkey, const unsigned *hcnt, int hmask, const RowPlan &rp, const float *pow_tab)
 {
-    if (key == 0ull) return key;
     key &= 0xFFFFFFFF7FFFFFFFull;
-    const unsigned c = fast_occurrences(hkey, hcnt, hmask, fast_idx(key));
-    if (c == 0u) return key;
+    unsigned c = fast_occurrences(hkey, hcnt, hmask, fast_idx(key));
+    if (key == 0ull) c = 0u;  // reads as token 2^31 - 1
+    if (!__any_sync(0xFFFFFFFFu, c != 0u)) return key;
     float x = key_val(key);
     const int occ_all = (int)(c & 0xFFFFu), occ_w = (int)(c >> 16);
     if (rp.rep != 1.0f && occ_w > 0) {
@@ -191,8 +197,9 @@ __device__ __forceinline__ u64 fast_penalise(u64 key, const int *hkey, const uns
         x = x > 0.f ? __fdiv_rn(x, pw) : __fmul_rn(x, pw);
     }
     x = __fsub_rn(x, __fadd_rn(rp.pres, __fmul_rn(rp.freq, (float)occ_all)));
+    __syncwarp();
     const uint32_t was = (uint32_t)(key >> 32), now = ord32(x);
-    return ((u64)now << 32) | (key & 0x7FFFFFFFull) | (now != was ? 0x80000000ull : 0ull);
+    return c != 0u ? ((u64)now << 32) | (key & 0x7FFFFFFFull) | (now != was ? 0x80000000ull : 0ull) : key;
 }
 
 // The sorted keys of one warp, with every run of equal lowered values put into the order of the raw logits.  Keys behind

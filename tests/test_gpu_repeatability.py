@@ -58,3 +58,32 @@ def test_repeated_batches_in_random_order(own_stream):
         assert (bs.stats()["graph_replays"] > 100) == own_stream
     finally:
         bs.close()
+
+
+def test_penalised_top_k_rows_keep_every_candidate():
+    """Rows whose candidates are looked up in a long history and sorted in registers right behind that: three rows of the
+    sweep's batch 1, repeated.  Lanes that left the lookup one by one used to lose a warp's candidates once in
+    a few hundred to a few thousand steps."""
+    import torch
+    from opentail.stingray_b200 import BatchSampler, workloads as W
+
+    w, rows = _workload(1), [10, 22, 32]
+    h = int(w.history_offsets[1])
+    w = W.SampleWorkload("s", np.ascontiguousarray(w.logits[rows]), w.params[rows].copy(), w.uniforms[rows].copy(),
+                         np.concatenate([w.history_ids[r * h:(r + 1) * h] for r in rows]), np.arange(4, dtype=np.int32) * h, None)
+    bs = BatchSampler(max_rows=4, max_vocab=262144, max_history=1024, max_top_k=64)
+    try:
+        dev = parity.to_device(w)
+        kw = dict(uniforms=dev["uniforms"], history_ids=dev["history_ids"], history_offsets=w.history_offsets,
+                  want_probs=True, want_flags=True, want_topk=40)
+        out = bs.sample_rows(dev["logits"], w.params, **kw)
+        torch.cuda.synchronize()
+        parity.compare(w, {k: v.cpu().numpy() for k, v in out.items()})
+        first = {k: v.clone() for k, v in out.items()}
+        differ = torch.zeros(1, dtype=torch.int64, device="cuda")
+        for _ in range(10_000):
+            out = bs.sample_rows(dev["logits"], w.params, out=out, **kw)
+            differ += (out["topk_ids"] != first["topk_ids"]).any() | (out["probs"] != first["probs"]).any()
+        assert int(differ) == 0
+    finally:
+        bs.close()
