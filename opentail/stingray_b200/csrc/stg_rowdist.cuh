@@ -335,19 +335,20 @@ struct ProvExp {
         int low = 0;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            float e = (base + j < n) ? expf(__fsub_rn(x[j], mx)) : 0.f;
-            x[j] = e;
-            if (hist && e > 0.f) {
-                const uint32_t eb = __float_as_uint(e);
-                const unsigned bin = bin_of(eb);
-                if (bin == 0u) low++;
-                else atomicAdd(&hist[bin], (1ull << 40) | (unsigned long long)(((eb & 0x7FFFFFu) | 0x800000u) >> 12));
-            }
+            x[j] = (base + j < n) ? expf(__fsub_rn(x[j], mx)) : 0.f;
+            low += x[j] > 0.f && bin_of(__float_as_uint(x[j])) == 0u ? 1 : 0;
         }
         if (hist) {
+            // ahead of the lanes' own branches: behind them the lanes were seen apart
             low = __reduce_add_sync(0xFFFFFFFFu, low);
             if (low && (threadIdx.x & 31) == 0)
                 atomicAdd(&hist[0], ((unsigned long long)low << 40) | ((unsigned long long)low * 0xFFFull));
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const uint32_t eb = __float_as_uint(x[j]);
+                const unsigned bin = bin_of(eb);
+                if (x[j] > 0.f && bin != 0u) atomicAdd(&hist[bin], (1ull << 40) | (unsigned long long)(((eb & 0x7FFFFFu) | 0x800000u) >> 12));
+            }
         }
         if (base < n) store8(scratch, base, n, x);
     }
