@@ -8,10 +8,10 @@
 // summaries, histograms, candidates) is pushed into its shared memory:
 //
 //   P0  history / bias overrides of the CTA's own tokens -> hash table
-//   P1  maximum                                              (the only pass that goes to HBM)
-//   P2  e = exp(x - max) -> scratch (L2), tile sums; then the guesses, compositions and runs of
-//       stg_walk.cuh
-//   P3  rank 0's first warp walks to the exact sum; all other warps histogram the exp values
+//   P1  maximum, and per tile an estimate of its sum of exp values that needs none (the only pass that goes to HBM)
+//   P2  e = exp(x - max) -> scratch (L2); on the way the guesses, compositions and runs of stg_walk.cuh and the
+//       histogram of the exp values
+//   P3  rank 0's first warp walks to the exact sum; the other CTAs' histograms go to rank 0
 //   P4  rank 0 bounds the nucleus.  Narrow (the usual case for a peaked row: up to kNarrow candidates):
 //       the candidates go to rank 0, are sorted, cut, sorted by token and drawn from there.
 //   P5  wide: per histogram bin the integer increment of all its elements (no order needed inside a
@@ -20,10 +20,14 @@
 //   P6  the sorted-order sum bin by bin -> top-p threshold
 //   P7  Normalize's sum; compositions of the final probabilities; the walk to the uniform
 //
-// Bound: the latency of the phases one after the other; a lone row of 32,000 spends 2 to 5 us in each (table 2.2,
-// maximum 2.5, exp 3.0, summaries 4.8, walk 5.2, plan 4.8; narrow another 8, wide 31).  The row is read from HBM once and
-// from L2 in every later pass as long as the rows in flight fit there (64 rows of 151,936: 40 MB read for 39); 288 rows,
-// one CTA each and 1.2 MB with their exp values, do not: 695 MB read and 175 written for 175, 196 us, 4.4 TB/s.
+// Bound: the latency of the phases one after the other; a lone row of 32,000 spends 1 to 6 us in each (table 2.4,
+// maximum 3.5, guesses 0.9, exp values 5.5, walk 4.8, plan 4.8; narrow another 8, wide 31).  As passes of their own - exp
+// values, compositions, histogram, each reading them again - the first four took as long for a lone row, but 64 rows of
+// 151,936 took 172 us instead of 159, and 288 + 256 descriptors of a verification step 455 instead of 375.  Where many rows run,
+// warps wait for instructions as much as for data: hence one tile to a turn of a loop (for_tiles), rare cases out of line, and
+// additions by predicate instead of branch (add_if: the increments of 64 rows 25 -> 19 us).  The row is read from HBM
+// once and from L2 in every later pass as long as the rows in flight fit there (64 rows of 151,936 do: 40 MB read for 39);
+// 288 rows, one CTA each and 1.2 MB with their exp values, do not, and their passes run at 4.7 TB/s.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <limits.h>
@@ -52,23 +56,25 @@ constexpr int kFlagged = 512;        // bins whose order counts at most
 constexpr unsigned char kBinOrder = 255;  // bin_e: the bin's order counts; 0: below the nucleus
 static_assert(kBins == 8 * kRT, "the bin scans give 8 bins to a thread");
 
-// dynamic shared memory: the override table of P0..P2, later the histogram and the candidate lists
-constexpr int kOffTabKey = 0;                                   // int[4096]
-constexpr int kOffTabCnt = kMaxOvSlots * 4;                     // u32[4096]: occurrences (12 bits), in the window (12), bias (1)
-constexpr int kOffTabVal = kOffTabCnt + kMaxOvSlots * 4;        // float[4096]
-constexpr int kOffTabMap = kOffTabVal + kMaxOvSlots * 4;        // 65536 folded bits
-constexpr int kTabEnd = kOffTabMap + 8192;
+// dynamic shared memory: the override table of P0..P2, the histogram and the candidate lists.  The table of `slots` entries
+// is int key[], u32 cnt[] (occurrences 12 bits, in the window 12, bias 1), float val[] and 65536 folded bits; one of up to
+// kSmallTable slots (512 history and bias entries) lies where the lists will be, so that the histogram can be filled
+// while it is in use, a larger one lies over the histogram too.
+constexpr int kSmallTable = 1024;
+constexpr int kTabEnd = kMaxOvSlots * 12 + 8192;
 constexpr int kOffBinMass = 0;                                  // u32[kBins]
 constexpr int kOffBinD = kBins * 4;                             // u32[kBins]
 constexpr int kOffBinE = 2 * kBins * 4;                         // u8[kBins]
 constexpr int kOffList = 2 * kBins * 4 + kBins;                 // u32[kRowList] | u64[kNarrow]
 constexpr int kListEnd = kOffList + kRowList * 4;
+static_assert(kSmallTable * 12 + 8192 <= kRowList * 4, "a small table fits the list");
 constexpr int kOffWalk = (kListEnd > kTabEnd ? kListEnd : kTabEnd);
 constexpr int kRowSmem = kOffWalk + (int)sizeof(WalkArea);
 static_assert(kNarrow * 8 <= kRowList * 4, "the narrow list borrows the wide one");
 
 struct RowSh {
     u64 maxkey[kRowMaxCluster], rawkey[kRowMaxCluster];
+    float cmax[kRowMaxCluster];
     double tot[2][kRowMaxCluster];
     double part[kRowMaxCluster];
     int cnt[kRowMaxCluster];
@@ -93,6 +99,14 @@ struct RowSh {
     unsigned short flagged[kFlagged];
     uint32_t flags;
 };
+
+// out of line, like everything that few rows or few tiles need (stg_walk.cuh)
+__device__ __noinline__ Lane8 soft_cap_8(Lane8 x, float cap)
+{
+#pragma unroll
+    for (int j = 0; j < 8; j++) x.v[j] = soft_cap(x.v[j], cap);
+    return x;
+}
 
 // ---- the row's adjusted, temperature-scaled logits ---------------------------------------------------
 template <bool BF16>
@@ -153,9 +167,10 @@ struct RowSrc {
             return;
         }
         if (rowp.cap != 0.f) {
+            const Lane8 y = soft_cap_8(lane8(x), rowp.cap);
 #pragma unroll
             for (int j = 0; j < 8; j++)
-                if (base + j < n) x[j] = soft_cap(x[j], rowp.cap);
+                if (base + j < n) x[j] = y.v[j];
         }
         if (bits != 0xFFu) {
 #pragma unroll
@@ -165,7 +180,7 @@ struct RowSrc {
     }
     __device__ __forceinline__ int find(int id) const
     {
-        const int *key = (const int *)(tab + kOffTabKey);
+        const int *key = (const int *)tab;
         int h = (int)(((unsigned)id * 2654435761u) >> 7) & tab_mask;
         for (;;) {
             const int k = key[h];
@@ -177,14 +192,16 @@ struct RowSrc {
     __device__ __forceinline__ void override_(float x[8], int base) const
     {
         if (tab != nullptr) {
-            const unsigned m = (tab + kOffTabMap)[(base & 0xFFFF) >> 3];
-            if (m) {
+            unsigned m = (tab + 12 * (tab_mask + 1))[(base & 0xFFFF) >> 3];
+#pragma unroll 1
+            while (m) {
+                const int j = __ffs(m) - 1;
+                m &= m - 1u;
+                const int slot = base + j < n ? find(base + j) : -1;
+                if (slot >= 0) {
+                    const float v = ((const float *)(tab + 8 * (tab_mask + 1)))[slot];
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    if (((m >> j) & 1u) && base + j < n) {
-                        const int slot = find(base + j);
-                        if (slot >= 0) x[j] = ((const float *)(tab + kOffTabVal))[slot];
-                    }
+                    for (int k = 0; k < 8; k++) x[k] = k == j ? v : x[k];
                 }
             }
         }
@@ -192,6 +209,10 @@ struct RowSrc {
     __device__ __forceinline__ void adjust(float x[8], int base) const
     {
         override_(x, base);
+        rescale(x);
+    }
+    __device__ __forceinline__ void rescale(float x[8]) const
+    {
         if (scale) {
 #pragma unroll
             for (int j = 0; j < 8; j++) x[j] = __fmul_rn(x[j], inv_t);
@@ -216,6 +237,50 @@ __device__ __forceinline__ double widen(float p)
 {
     const uint32_t b = __float_as_uint(p);
     return __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
+}
+
+// adds v to a word of this CTA's shared memory where `on`.  By a predicate: a branch around every one of eight additions
+// parts the warp eight times, and costs more than the addition.
+__device__ __forceinline__ void add_if(bool on, unsigned *at, unsigned v)
+{
+    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p red.shared.add.u32 [%1], %2;\n}"
+                 ::"r"((unsigned)on), "r"((unsigned)__cvta_generic_to_shared(at)), "r"(v) : "memory");
+}
+__device__ __forceinline__ float exp2_approx(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float warp_max_f(float x)
+{
+    float y;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float warp_sum_f(float v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    return v;
+}
+// One warp: {maximum, sum of 2^((x - maximum) k2)} of a tile's elements (8 per lane), to *est, and the lane's maximum.  What the
+// tile will weigh against the row's maximum, before that is known: a guess, good to some 1e-6.
+__device__ __forceinline__ float estimate_tile(const float x[8], float k2, float2 *est)
+{
+    float m = x[0];
+#pragma unroll
+    for (int j = 1; j < 8; j++) m = fmaxf(m, x[j]);
+    const float top = warp_max_f(m), ref = top > -CUDART_INF_F ? top : 0.f;
+    float2 s2 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {  // two elements to an instruction
+        const float2 v = __fmul2_rn(__fadd2_rn(make_float2(x[j], x[j + 1]), make_float2(-ref, -ref)), make_float2(k2, k2));
+        s2 = __fadd2_rn(s2, make_float2(exp2_approx(v.x), exp2_approx(v.y)));
+    }
+    const float s = warp_sum_f(s2.x + s2.y);
+    if ((threadIdx.x & 31) == 0) *est = make_float2(top, s);
+    return m;
 }
 
 __device__ __forceinline__ double warp_sum_d(double v)
@@ -347,14 +412,14 @@ __device__ __forceinline__ void row_sort_desc(u64 *a, int p2)
 // P0: the overrides among the tokens [lo, hi): ApplyHistoryPenalties after the logit bias
 // (Sampler.cs:50-56, :367-419).  Every CTA reads the whole history and keeps its own tokens.
 template <bool BF16>
-__device__ __forceinline__ void build_table(const SampleArgs &a, const RowPlan &rp, const RowSrc<BF16> &src, unsigned char *dyn, int slots,
+__device__ __forceinline__ void build_table(const SampleArgs &a, const RowPlan &rp, const RowSrc<BF16> &src, unsigned char *tab, int slots,
                                             int nh, int nb, int lo, int hi)
 {
     const int tid = threadIdx.x, mask = slots - 1;
-    int *key = (int *)(dyn + kOffTabKey);
-    unsigned *cnt = (unsigned *)(dyn + kOffTabCnt);
-    float *val = (float *)(dyn + kOffTabVal);
-    unsigned *map = (unsigned *)(dyn + kOffTabMap);
+    int *key = (int *)tab;
+    unsigned *cnt = (unsigned *)(key + slots);
+    float *val = (float *)(cnt + slots);
+    unsigned *map = (unsigned *)(val + slots);
     for (int t = tid; t < slots; t += kRT) { key[t] = -1; cnt[t] = 0u; val[t] = 0.f; }
     for (int t = tid; t < 2048; t += kRT) map[t] = 0u;
     __syncthreads();
@@ -395,67 +460,129 @@ __device__ __forceinline__ void build_table(const SampleArgs &a, const RowPlan &
     __syncthreads();
 }
 
-// guesses, compositions and runs of the CTA's tiles [t0, t1) over the elements get(t, x), whose sums are in
-// tile_sum (times `scale` they are what the walk will see), into rank 0's walk area.  `base`: the sum of
-// the tiles before t0, `mine` of these, `all` of the row, all unscaled.
-template <class Get>
-__device__ __forceinline__ void summarise(RowSh &sh, WalkArea *wa, WalkArea *dst, const Get &get, int t0, int t1, double base, double mine,
-                                          double all, double scale, double target)
+// body(t, x) for a warp's tiles t = first, first + stride, ... below end, whose elements load(t, x) fetches: one tile at a time,
+// the next one's elements on the way.  Two tiles to a turn hide as much latency, but their loop is twice as long, and
+// the warps wait for its instructions: 64 rows of 151,936 166 -> 161 us with this (and the rare cases out of line) in P2 alone.
+template <class Load, class Body>
+__device__ __forceinline__ void for_tiles(int first, int end, int stride, const Load &load, const Body &body)
+{
+    float nx[8];
+    if (first < end) load(first, nx);
+#pragma unroll 1
+    for (int t = first; t < end; t += stride) {
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = nx[j];
+        if (t + stride < end) load(t + stride, nx);
+        body(t, x);
+    }
+}
+
+// The fp64 prefix sums of the CTA's tiles: thread i holds those around its tiles 2 i and 2 i + 1.
+struct TilePrefix { double in, mid, out, all; };
+// every thread; two block barriers, the first of them ahead of any access to `red`
+__device__ __forceinline__ TilePrefix tile_prefix(const float *tile_sum, int nt, double *red)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g_end = exp_of_double(all * scale);
-    if (warp == 0) {
-        double run = base;
-        for (int b = t0; b < t1; b += 32) {
-            const int t = b + lane;
-            const double v = t < t1 ? (double)sh.tile_sum[t - t0] : 0.0;
-            const double inc = warp_scan_d(v);
-            if (t < t1) {
-                const double lo = (run + (inc - v)) * scale, hi = (t + 1 == t1 ? base + mine : run + inc) * scale;
-                const int g = exp_of_double(lo);
-                int k = walk_kind(t, g, exp_of_double(hi), g_end);
-                if (lo < target && target <= hi && t > 0) k = kTileSlot + kWalkCross;
-                sh.guess[t - t0] = (unsigned char)g;
-                sh.kind[t - t0] = (unsigned char)k;
-            }
-            run += __shfl_sync(0xFFFFFFFFu, inc, 31);
-        }
-    }
     __syncthreads();
-    for (int tb = t0 + warp; tb < t1; tb += 2 * kRW) {
-        float x[2][8];
-        get(tb, x[0]);
-        if (tb + kRW < t1) get(tb + kRW, x[1]);
+    const double v = 2 * tid < nt ? (double)tile_sum[2 * tid] : 0.0, w = 2 * tid + 1 < nt ? (double)tile_sum[2 * tid + 1] : 0.0;
+    TilePrefix p;
+    const double inc = warp_scan_d(v + w);
+    if (lane == 31) red[warp] = inc;
+    __syncthreads();
+    double before = 0.0, all = 0.0;
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int t = tb + u * kRW;
-            if (t >= t1) break;
-            const int k = sh.kind[t - t0], g = sh.guess[t - t0];
-            const double ts = (double)sh.tile_sum[t - t0] * scale;
-            int a0 = 0, a1 = 0;
-            if (k == kTileRun) {
-                if (ts != 0.0) {
-                    if (g >= 48 && g < 250 && ts < __hiloint2double((g - 2 + 896) << 20, 0)) tile_composite(x[u], g, a0, a1);
-                    else subtile_composite<false>(x[u], g, a0, a1);
-                }
-            } else if (k != kTileReplay || t == 0) {
-                WalkCross *c = &dst->xs[k >= kTileSlot ? (k - kTileSlot) % (kWalkCross + 1) : k - 1];
-                if (t != 0) {
-                    if (k < kTileSlot) walk_cross(c, x[u], g);
-                    if (lane == 0) c->tile = t;
-                }
-                float4 *q = (float4 *)((t == 0 ? dst->head : c->x) + lane * 8);
-                q[0] = make_float4(x[u][0], x[u][1], x[u][2], x[u][3]);
-                q[1] = make_float4(x[u][4], x[u][5], x[u][6], x[u][7]);
-            }
-            if (lane == 0) {
-                wa->comp[t] = make_int2(a0, a1);
-                if (dst != wa) dst->comp[t] = make_int2(a0, a1);
-            }
+    for (int k = 0; k < kRW; k++) {
+        const double r = red[k];
+        before += k < warp ? r : 0.0;
+        all += r;
+    }
+    p.in = before + (inc - (v + w));
+    p.mid = p.in + v;
+    p.out = before + inc;
+    p.all = all;
+    return p;
+}
+
+// guessed binades and kinds of the CTA's tiles [t0, t1): the sum in front of tile t is base + factor times the
+// prefix; `end`: the guess for the whole sum, `target` where the walk is to end.  Ends in a block barrier.
+__device__ __forceinline__ void guess_tiles(RowSh &sh, const TilePrefix &p, int t0, int t1, double base, double factor, double all, double target)
+{
+    const int tid = threadIdx.x, g_end = exp_of_double(all);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int i = 2 * tid + u, t = t0 + i;
+        if (t < t1) {
+            const double lo = base + (u ? p.mid : p.in) * factor, hi = base + (t + 1 == t1 ? p.all : u ? p.out : p.mid) * factor;
+            const int g = exp_of_double(lo);
+            int k = walk_kind(t, g, exp_of_double(hi), g_end);
+            if (lo < target && target <= hi && t > 0) k = kTileSlot + kWalkCross;
+            sh.guess[i] = (unsigned char)g;
+            sh.kind[i] = (unsigned char)k;
         }
     }
     __syncthreads();
-    if (warp == 0) walk_runs(dst, wa->comp + t0, sh.guess, sh.kind, t0, t1);
+}
+
+// One warp: the composition of tile t (8 elements per lane in x, their sum about `ts`) under its guess, or what its kind
+// asks for, into rank 0's walk area.
+__device__ __forceinline__ void compose_tile(const RowSh &sh, WalkArea *wa, WalkArea *dst, const float x[8], int t, int t0, float ts)
+{
+    const int lane = threadIdx.x & 31;
+    const int k = sh.kind[t - t0], g = sh.guess[t - t0];
+    int a0 = 0, a1 = 0;
+    if (k == kTileRun) {
+        if (g >= 48 && g < 250 && ts < __uint_as_float((uint32_t)(g - 2) << 23)) {
+            tile_composite(x, g, a0, a1);
+        } else {
+            float any = x[0];
+#pragma unroll
+            for (int j = 1; j < 8; j++) any = fmaxf(any, x[j]);
+            if (__any_sync(0xFFFFFFFFu, any > 0.f)) {
+                const int2 r = composite_any(lane8(x), g);
+                a0 = r.x;
+                a1 = r.y;
+            }
+        }
+    } else if (k != kTileReplay || t == 0) {
+        WalkCross *c = &dst->xs[k >= kTileSlot ? (k - kTileSlot) % (kWalkCross + 1) : k - 1];
+        if (t != 0) {
+            if (k < kTileSlot) walk_cross(c, lane8(x), g);
+            if (lane == 0) c->tile = t;
+        }
+        float4 *q = (float4 *)((t == 0 ? dst->head : c->x) + lane * 8);
+        q[0] = make_float4(x[0], x[1], x[2], x[3]);
+        q[1] = make_float4(x[4], x[5], x[6], x[7]);
+    }
+    if (lane == 0) {
+        wa->comp[t] = make_int2(a0, a1);
+        if (dst != wa) dst->comp[t] = make_int2(a0, a1);
+    }
+}
+
+// The runs of the CTA's composed tiles, a group of them per warp (behind a block barrier).  A run ends with its group, so
+// that the groups need nothing of each other: one warp over all 594 tiles of a row of 151,936 took as long as the rest.
+constexpr int kRunGroup = 64;
+__device__ __forceinline__ void runs_of_tiles(const RowSh &sh, const WalkArea *wa, WalkArea *dst, int t0, int t1)
+{
+    for (int g = t0 + (int)(threadIdx.x >> 5) * kRunGroup; g < t1; g += kRW * kRunGroup)
+        walk_runs(dst, wa->comp + g, sh.guess + (g - t0), sh.kind + (g - t0), g, min(t1, g + kRunGroup));
+}
+
+// guesses, compositions and runs of the CTA's tiles [t0, t1) over the elements load(t, x) and then map(t, x), whose sums are in
+// tile_sum (times `scale` they are what the walk will see) and whose prefix is `p`, into rank 0's walk area.
+// `base`: the sum of the tiles before t0, `all` of the row, both unscaled.
+template <class Load, class Map>
+__device__ __forceinline__ void summarise(RowSh &sh, WalkArea *wa, WalkArea *dst, const Load &load, const Map &map, int t0, int t1,
+                                          const TilePrefix &p, double base, double all, double scale, double target)
+{
+    guess_tiles(sh, p, t0, t1, base * scale, scale, all * scale, target);
+    for_tiles(t0 + (int)(threadIdx.x >> 5), t1, kRW, load, [&](int t, float (&x)[8]) {
+        map(t, x);
+        compose_tile(sh, wa, dst, x, t, t0, sh.tile_sum[t - t0] * (float)scale);
+    });
+    __syncthreads();
+    runs_of_tiles(sh, wa, dst, t0, t1);
 }
 
 // a warp's sort of a short list (descending) by counting ranks; lists of one value - the rule for rows that
@@ -940,17 +1067,27 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     }
     src.tab = nullptr;
     src.tab_mask = 0;
+    bool small_table = true;
     if (tid == 0) { sh.flags = 0u; sh.n_cand = 0; sh.list_n = 0; sh.stop = 0; sh.hit_keep = 0; sh.tie_idx = INT_MAX; }
     {
         const int nh = rp.has_penalty ? rp.hist_len : 0, nb = greedy ? 0 : rp.bias_len;
         if (nh + nb > 0) {
             int slots = 64;
             while (slots < 2 * (nh + nb)) slots <<= 1;
-            build_table<BF16>(a, rp, src, dyn, slots, nh, nb, t0 * kSub, min(n, t1 * kSub));
-            src.tab = dyn;
+            small_table = slots <= kSmallTable;
+            unsigned char *tab = dyn + (small_table ? kOffList : 0);
+            build_table<BF16>(a, rp, src, tab, slots, nh, nb, t0 * kSub, min(n, t1 * kSub));
+            src.tab = tab;
             src.tab_mask = slots - 1;
         }
     }
+    unsigned *mass = (unsigned *)(dyn + kOffBinMass);
+    unsigned *dd = (unsigned *)(dyn + kOffBinD);
+    unsigned char *bin_e = dyn + kOffBinE;
+    auto clear_bins = [&]() {
+        for (int b = tid; b < kBins / 2; b += kRT) ((uint4 *)mass)[b] = make_uint4(0u, 0u, 0u, 0u);  // mass and dd
+    };
+    if (want_topp && small_table) clear_bins();
     tick(tk, 1);
 
     // A row behind a mask that allows at most half of the vocabulary is closed up as it is read: its allowed tokens, in
@@ -961,15 +1098,18 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     int *tile_at = (int *)sh.tile_sum;
     const bool counted = CLOSE && src.mrow != nullptr && !greedy && a.mode == 0;  // the same for every thread of the cluster
     if (counted) {
-        for (int t = t0 + warp; t < t1; t += kRW) {
-            const int base = t * kSub + lane * 32;
+        // a word per lane, four tiles to a load
+        for (int g = t0 + 4 * warp; g < t1; g += 4 * kRW) {
+            const int t = g + lane / 8, base = g * kSub + lane * 32;
             uint32_t w = 0u;
-            if (lane < kSub / 32 && base < n) {
+            if (t < t1 && base < n) {
                 w = __ldg(src.mrow + (base >> 5));
                 if (base + 32 > n) w &= (1u << (n - base)) - 1u;
             }
-            const int c = __reduce_add_sync(0xFFFFFFFFu, __popc(w));
-            if (lane == 0) tile_at[t - t0] = c;
+            int c = __popc(w);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+            if ((lane & 7) == 0 && t < t1) tile_at[t - t0] = c;
         }
         __syncthreads();
         cl.barrier_wait();
@@ -994,28 +1134,41 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         }
     }
 
-    // P1: the maximum
+    // P1: the maximum, and for the tiles' sums of exp values estimates that need no maximum
+    const float k2 = src.inv_t * 1.44269504f;
+    float2 *est = (float2 *)wa->comp;
+    TilePrefix tp{0.0, 0.0, 0.0, 0.0};
     {
-        float best = -CUDART_INF_F;
+        float best = -CUDART_INF_F, cmax = -CUDART_INF_F;  // cmax: unscaled, what the CTA's estimates are relative to
         u64 key = 0ull, raw = 0ull;
         if (CLOSE && ids != nullptr) {
-            for (int t = t0 + warp; t < t1; t += kRW) {
+            float nx[8];
+            unsigned nbits = 0u;
+            if (t0 + warp < t1) src.fetch((t0 + warp) * kSub + lane * 8, nx, nbits);
+#pragma unroll 1
+            for (int t = t0 + warp; t < t1; t += kRW) {  // the next tile's logits on the way, as in for_tiles
                 const int base = t * kSub + lane * 8;
                 float x[8];
-                unsigned bits;
-                src.fetch(base, x, bits);
-                src.mask(x, bits, base);
+#pragma unroll
+                for (int j = 0; j < 8; j++) x[j] = nx[j];
+                const unsigned bits = nbits;
+                if (t + kRW < t1) src.fetch(base + kRW * kSub, nx, nbits);
+                if (!__any_sync(0xFFFFFFFFu, bits != 0u)) continue;
+                src.mask(x, bits, base);  // what is not allowed is -infinity
                 src.adjust(x, base);
                 const int c = __popc(bits);
-                int at = first_id + tile_at[t - t0] + warp_scan_i(c) - c;
+                const int at = first_id + tile_at[t - t0] + warp_scan_i(c) - c;
+                float *ep = e + at;
+                int32_t *ip = ids + at;
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if ((bits >> j) & 1u) {
-                        best = fmaxf(best, x[j]);
-                        e[at] = x[j];
-                        ids[at] = base + j;
-                        at++;
-                    }
+                for (int j = 0; j < 8; j++) {
+                    const unsigned on = (bits >> j) & 1u;
+                    best = fmaxf(best, on ? x[j] : -CUDART_INF_F);
+                    asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p st.global.f32 [%1], %2;\n @p st.global.s32 [%3], %4;\n}"
+                                 ::"r"(on), "l"(ep), "f"(x[j]), "l"(ip), "r"(base + j) : "memory");  // by a predicate, as in add_if
+                    ep += on;
+                    ip += on;
+                }
             }
             best = block_max_f(best, sh.red_f);
             if (best > -CUDART_INF_F) key = make_key(best, 0);
@@ -1036,7 +1189,9 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     if (x[j] > rbest) { rbest = x[j]; rbest_i = base + j; }
-                src.adjust(x, base);
+                src.override_(x, base);
+                if (!greedy) cmax = fmaxf(cmax, estimate_tile(x, k2, est + t));
+                src.rescale(x);
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     if (x[j] > best) { best = x[j]; best_i = base + j; }
@@ -1044,6 +1199,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
             key = block_max_k(best_i >= 0 ? make_key(best, best_i) : 0ull, sh.red_k);
             __syncthreads();
             raw = block_max_k(rbest_i >= 0 ? make_key(rbest, rbest_i) : 0ull, sh.red_k);
+            cmax = block_max_f(cmax, sh.red_f);
         } else {
             // unscaled: multiplying by 1 / T > 0 and rounding is monotonic, so the maximum is scaled at the end
             for (int t = t0 + warp; t < t1; t += 2 * kRW) {
@@ -1055,24 +1211,35 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                 if (two) src.fetch(b1, x[1], bits[1]);
                 src.mask(x[0], bits[0], b0);
                 src.override_(x[0], b0);
-#pragma unroll
-                for (int j = 0; j < 8; j++) best = fmaxf(best, x[0][j]);
+                cmax = fmaxf(cmax, estimate_tile(x[0], k2, est + t));
                 if (two) {
                     src.mask(x[1], bits[1], b1);
                     src.override_(x[1], b1);
-#pragma unroll
-                    for (int j = 0; j < 8; j++) best = fmaxf(best, x[1][j]);
+                    cmax = fmaxf(cmax, estimate_tile(x[1], k2, est + t + kRW));
                 }
             }
-            best = block_max_f(best, sh.red_f);
+            best = cmax = block_max_f(cmax, sh.red_f);
             if (src.scale) best = __fmul_rn(best, src.inv_t);
             if (best > -CUDART_INF_F) key = make_key(best, 0);
+        }
+        if (!greedy && !(CLOSE && ids != nullptr)) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int i = 2 * tid + u;
+                if (t0 + i < t1) {
+                    const float2 v = est[t0 + i];
+                    sh.tile_sum[i] = v.x > -CUDART_INF_F ? v.y * exp2_approx((v.x - cmax) * k2) : 0.f;
+                }
+            }
+            tp = tile_prefix(sh.tile_sum, t1 - t0, sh.red_d);
         }
         if (!counted) cl.barrier_wait();
         if (tid < C) {
             RowSh *o = cl.map_shared_rank(&sh, tid);
             o->maxkey[rank] = key;
             o->rawkey[rank] = raw;
+            o->cmax[rank] = cmax;
+            o->tot[0][rank] = tp.all;
         }
         cl.sync();
     }
@@ -1120,116 +1287,109 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     }
     const float mx = key_val(mk);
 
-    // P2: exp values and tile sums
+    double base = 0.0, all = 0.0;
+    float own = 1.f;  // what the CTA's estimates are to be multiplied by
     if (CLOSE && ids != nullptr) {
+        // the closed-up row's tiles, now that the maximum is known
         for (int t = t0 + warp; t < t1; t += kRW) {
             const int b = t * kSub + lane * 8;
             float x[8], acc = 0.f;
             load_e(e, b, x);
 #pragma unroll
-            for (int j = 0; j < 8; j++) {
-                x[j] = b + j < n ? expf(__fsub_rn(x[j], mx)) : 0.f;
-                acc += x[j];
-            }
-            store_e(e, b, x);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+            for (int j = 0; j < 8; j++) acc += b + j < n ? exp2_approx((x[j] - mx) * 1.44269504f) : 0.f;
+            acc = warp_sum_f(acc);
             if (lane == 0) sh.tile_sum[t - t0] = acc;
         }
-    } else {
-        for (int t = t0 + warp; t < t1; t += 2 * kRW) {
-            float x[2][8];
-            unsigned bits[2];
-            const int b0 = t * kSub + lane * 8;
-            src.fetch(b0, x[0], bits[0]);
-            const bool two = t + kRW < t1;
-            if (two) src.fetch(b0 + kRW * kSub, x[1], bits[1]);
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (u == 1 && !two) break;
-                const int base = b0 + u * kRW * kSub;
-                src.mask(x[u], bits[u], base);
-                src.adjust(x[u], base);
-                float acc = 0.f;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    x[u][j] = expf(__fsub_rn(x[u][j], mx));  // 0 beyond the row, whose logits read as -inf
-                    acc += x[u][j];
-                }
-                store_e(e, base, x[u]);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-                if (lane == 0) sh.tile_sum[t - t0 + u * kRW] = acc;
-            }
-        }
-    }
-    __syncthreads();
-    unsigned *mass = (unsigned *)(dyn + kOffBinMass);
-    unsigned *dd = (unsigned *)(dyn + kOffBinD);
-    unsigned char *bin_e = dyn + kOffBinE;
-    if (want_topp)
-        for (int b = tid; b < kBins / 2; b += kRT) ((uint4 *)mass)[b] = make_uint4(0u, 0u, 0u, 0u);  // mass and dd
-    auto push_total = [&](int k) {
-        if (warp == 0) {
-            double v = 0.0;
-            for (int t = lane; t < t1 - t0; t += 32) v += (double)sh.tile_sum[t];
-            v = warp_sum_d(v);
-            if (lane < C) cl.map_shared_rank(&sh, lane)->tot[k][rank] = v;
-        }
-    };
-    auto totals = [&](int k, double &base, double &mine, double &all) {
-        base = 0.0;
-        all = 0.0;
+        tp = tile_prefix(sh.tile_sum, t1 - t0, sh.red_d);
+        if (tid < C) cl.map_shared_rank(&sh, tid)->tot[1][rank] = tp.all;
+        cl.sync();
         for (int r = 0; r < C; r++) {
             if (r == rank) base = all;
-            all += sh.tot[k][r];
+            all += sh.tot[1][r];
         }
-        mine = sh.tot[k][rank];
-    };
-    push_total(0);
-    cl.sync();
+    } else {
+        float cmax = -CUDART_INF_F;
+        for (int r = 0; r < C; r++) cmax = fmaxf(cmax, sh.cmax[r]);
+        for (int r = 0; r < C; r++) {
+            const float f = exp2_approx((sh.cmax[r] - cmax) * k2);
+            if (r == rank) { base = all; own = f; }
+            all += sh.tot[0][r] * (double)f;
+        }
+    }
+    guess_tiles(sh, tp, t0, t1, base, (double)own, all, CUDART_INF);
     tick(tk, 3);
-    double base, mine, all;
-    totals(0, base, mine, all);
-    auto get_e = [&](int t, float x[8]) { load_e(e, t * kSub + lane * 8, x); };
-    summarise(sh, wa, dst, get_e, t0, t1, base, mine, all, 1.0, CUDART_INF);
-    cl.sync();
-    tick(tk, 4);
 
-    // P3: the exact sum on rank 0's first warp; the histogram of the exp values everywhere else.  Masses are of
-    // the upper 13 mantissa bits, completed by the lower 11 (less their middle, in the increments' array) of the at
-    // most 16,383 values that weigh something: their signed sum stays within 2^24.  Values below tau are left
+    // P2: exp values, the tiles' compositions, and the histogram of the exp values (where the override table leaves room;
+    // else in P3).  Masses are of the upper 13 mantissa bits, completed by the lower 11 (less their middle, in the increments'
+    // array) of the at most 16,383 values that weigh something: their signed sum stays within 2^24.  Values below tau are left
     // out: all of them together cannot be more than half of what the nucleus may leave behind.
     // Values below minp_e cannot reach min-p's threshold, whatever the sum is: fl(e * inv) >= fl(min_p * inv) takes an
     // e >= min_p * (1 - 2^-23).  A mass that holds more than the survivors' makes the bound too high.
     const float minp_e = min_p > 0.f ? min_p * (1.0f - 1.0f / 1048576.0f) : 0.f;
     const float tau = 0.5f * (1.0f - top_p) * (float)(all / (double)n);
-    if (rank == 0 && warp == 0) {
-        const WalkOut o = row_walk(wa, get_e, n, nsub, 0.f, false);
-        if (lane < C) cl.map_shared_rank(&sh, lane)->sum = o.s;
-    } else if (want_topp) {
-        const float floor_e = fmaxf(tau, minp_e), heavy_e = (float)(all * (1.0 / 16384.0));
-        const int w0 = rank == 0 ? warp - 1 : warp, wn = rank == 0 ? kRW - 1 : kRW;
-        for (int t = t0 + w0; t < t1; t += 2 * wn) {
-            float x[2][8];
-            get_e(t, x[0]);
-            const bool two = t + wn < t1;
-            if (two) get_e(t + wn, x[1]);
+    const float floor_e = fmaxf(tau, minp_e), heavy_e = (float)(all * (1.0 / 16384.0));
+    auto to_bins = [&](const float (&x)[8]) {
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (u == 1 && !two) break;
+        for (int j = 0; j < 8; j++) {
+            const uint32_t eb = __float_as_uint(x[j]), m = (eb & 0x7FFFFFu) | 0x800000u;
+            const int b = row_bin(eb);
+            add_if(x[j] > floor_e, mass + b, m >> 11);
+            add_if(x[j] > fmaxf(floor_e, heavy_e), dd + b, (m & 2047u) - 1024u);
+        }
+    };
+    if (CLOSE && ids != nullptr) {
+        for (int t = t0 + warp; t < t1; t += kRW) {
+            const int b = t * kSub + lane * 8;
+            float x[8];
+            load_e(e, b, x);
 #pragma unroll
-                for (int j = 0; j < 8; j++)
-                    if (x[u][j] > floor_e) {
-                        const uint32_t eb = __float_as_uint(x[u][j]), m = (eb & 0x7FFFFFu) | 0x800000u;
-                        const int b = row_bin(eb);
-                        atomicAdd(&mass[b], m >> 11);
-                        if (x[u][j] > heavy_e) atomicAdd(&dd[b], (m & 2047u) - 1024u);
-                    }
-            }
+            for (int j = 0; j < 8; j++) x[j] = b + j < n ? expf(__fsub_rn(x[j], mx)) : 0.f;
+            store_e(e, b, x);
+            compose_tile(sh, wa, dst, x, t, t0, sh.tile_sum[t - t0]);
+            if (want_topp && small_table) to_bins(x);
+        }
+    } else {
+        // one tile at a time, the next one's logits on the way
+        float nx[8];
+        unsigned nbits = 0u;
+        if (t0 + warp < t1) src.fetch((t0 + warp) * kSub + lane * 8, nx, nbits);
+#pragma unroll 1
+        for (int t = t0 + warp; t < t1; t += kRW) {
+            const int at = t * kSub + lane * 8;
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = nx[j];
+            const unsigned bits = nbits;
+            if (t + kRW < t1) src.fetch(at + kRW * kSub, nx, nbits);
+            src.mask(x, bits, at);
+            src.adjust(x, at);
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = expf(__fsub_rn(x[j], mx));  // 0 beyond the row, whose logits read as -inf
+            store_e(e, at, x);
+            compose_tile(sh, wa, dst, x, t, t0, sh.tile_sum[t - t0] * own);
+            if (want_topp && small_table) to_bins(x);
         }
     }
     __syncthreads();
+    runs_of_tiles(sh, wa, dst, t0, t1);
+    if (want_topp && !small_table) clear_bins();
+    cl.sync();
+    tick(tk, 4);
+
+    auto get_e = [&](int t, float x[8]) { load_e(e, t * kSub + lane * 8, x); };
+    // P3: the exact sum on rank 0's first warp; beside it the other CTAs' histograms go to rank 0
+    if (rank == 0 && warp == 0) {
+        const WalkOut o = row_walk(wa, get_e, n, nsub, 0.f, false);
+        if (lane < C) cl.map_shared_rank(&sh, lane)->sum = o.s;
+    } else if (want_topp && !small_table) {
+        const int w0 = rank == 0 ? warp - 1 : warp, wn = rank == 0 ? kRW - 1 : kRW;
+        for (int t = t0 + w0; t < t1; t += wn) {
+            float x[8];
+            get_e(t, x);
+            to_bins(x);
+        }
+    }
+    if (!small_table) __syncthreads();
     if (want_topp && rank != 0) {
         unsigned *m0 = cl.map_shared_rank(mass, 0), *h0 = cl.map_shared_rank(dd, 0);
         for (int b = tid; b < kBins; b += kRT) {
@@ -1315,23 +1475,14 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         if (sh.narrow) {
             u64 *keys = (u64 *)(dyn + kOffList);
             u64 *keys0 = rank == 0 ? keys : cl.map_shared_rank(keys, 0);
-            for (int t = t0 + warp; t < t1; t += 2 * kRW) {
-                float x[2][8];
-                get_e(t, x[0]);
-                const bool two = t + kRW < t1;
-                if (two) get_e(t + kRW, x[1]);
+            for_tiles(t0 + warp, t1, kRW, get_e, [&](int t, float (&x)[8]) {
+                unsigned take = 0u;
 #pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    if (u == 1 && !two) break;
-                    unsigned take = 0u;
-#pragma unroll
-                    for (int j = 0; j < 8; j++)
-                        if (x[u][j] >= lo_e && prob(x[u][j]) > 0.f) take |= 1u << j;
-                    append(keys, kNarrow, rank == 0 ? &sh.n_cand : &sh.list_n, take, [&](int j) {
-                        return ((u64)__float_as_uint(prob(x[u][j])) << 32) | (u64)(0xFFFFFFFFu - (uint32_t)((t + u * kRW) * kSub + lane * 8 + j));
-                    });
-                }
-            }
+                for (int j = 0; j < 8; j++) take |= x[j] >= lo_e && prob(x[j]) > 0.f ? 1u << j : 0u;
+                append(keys, kNarrow, rank == 0 ? &sh.n_cand : &sh.list_n, take, [&](int j) {
+                    return ((u64)__float_as_uint(prob(x[j])) << 32) | (u64)(0xFFFFFFFFu - (uint32_t)(t * kSub + lane * 8 + j));
+                });
+            });
             __syncthreads();
             if (rank != 0 && sh.list_n > 0) {
                 if (tid == 0) sh.n_cand = atomicAdd(&sh0->n_cand, sh.list_n);
@@ -1468,41 +1619,37 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                     if (at + i < kRowList) list0[at + i] = list[i];
             }
         };
-        for (int t = t0 + warp; t < t1; t += 2 * kRW) {
-            float x[2][8];
-            get_e(t, x[0]);
-            const bool two = t + kRW < t1;
-            if (two) get_e(t + kRW, x[1]);
+        for_tiles(t0 + warp, t1, kRW, get_e, [&](int, float (&x)[8]) {
+            unsigned take = 0u, odd = 0u;
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (u == 1 && !two) break;
-                unsigned take = 0u;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    if (!(x[u][j] >= lo_e)) continue;
-                    const float p = prob(x[u][j]);
-                    if (!(p > 0.f)) continue;
-                    const int b = row_bin(__float_as_uint(x[u][j]));
-                    const int be = bin_e[b];
-                    if (be == kBinOrder) {
-                        take |= 1u << j;
-                    } else {
-                        // the increment in units of the running sum, as in tile_composite
-                        int d0, d1;
-                        if (be >= 48 && p < __uint_as_float((uint32_t)(be - 1) << 23)) {
-                            const float c = __uint_as_float(((uint32_t)be << 23) | 0x400000u), y = __fadd_rn(p, c);
-                            d0 = __float_as_int(y) - __float_as_int(c);
-                            d1 = fabsf(__fsub_rn(p, __fsub_rn(y, c))) == __uint_as_float((uint32_t)(be - 24) << 23) ? -1 : d0;
-                        } else {
-                            unit_incr(p, be, d0, d1);
-                        }
-                        if (d0 != d1) atomicOr(&sh0->tie_bits[b >> 5], 1u << (b & 31));
-                        if (d0) atomicAdd(&dd[b], (unsigned)d0);
-                    }
-                }
-                append(list, kRowList, &sh.list_n, take, [&](int j) { return __float_as_uint(x[u][j]); });
+            for (int j = 0; j < 8; j++) {
+                const float p = prob(x[j]);
+                const int b = row_bin(__float_as_uint(x[j])), be = bin_e[b];
+                const bool in = x[j] >= lo_e && p > 0.f, order = be == kBinOrder;
+                // the increment in units of the running sum, as in tile_composite
+                const float c = __uint_as_float(((uint32_t)be << 23) | 0x400000u), y = __fadd_rn(p, c);
+                const bool plain = be >= 48 && p < __uint_as_float((uint32_t)(be - 1) << 23) &&
+                                   fabsf(__fsub_rn(p, __fsub_rn(y, c))) != __uint_as_float((uint32_t)(be - 24) << 23);
+                take |= in && order ? 1u << j : 0u;
+                odd |= in && !order && !plain ? 1u << j : 0u;
+                add_if(in && !order && plain, dd + b, (unsigned)(__float_as_int(y) - __float_as_int(c)));
             }
-        }
+            // a rounding tie, or nearly as large as the sum
+#pragma unroll 1
+            while (odd) {
+                const int q = __ffs(odd) - 1;
+                odd &= odd - 1u;
+                float v = x[0];
+#pragma unroll
+                for (int j = 1; j < 8; j++) v = j == q ? x[j] : v;
+                const int b = row_bin(__float_as_uint(v));
+                int d0, d1;
+                unit_incr(prob(v), bin_e[b], d0, d1);
+                if (d0 != d1) atomicOr(&sh0->tie_bits[b >> 5], 1u << (b & 31));
+                if (d0) atomicAdd(&dd[b], (unsigned)d0);
+            }
+            append(list, kRowList, &sh.list_n, take, [&](int j) { return __float_as_uint(x[j]); });
+        });
         hand_over();
         if (rank != 0)
             for (int b = tid; b < kBins; b += kRT) {
@@ -1526,24 +1673,16 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                     if (tid == 0) sh.list_n = 0;
                     __syncthreads();
                 }
-                for (int t = t0 + warp; t < t1; t += 2 * kRW) {
-                    float x[2][8];
-                    get_e(t, x[0]);
-                    const bool two = t + kRW < t1;
-                    if (two) get_e(t + kRW, x[1]);
+                for_tiles(t0 + warp, t1, kRW, get_e, [&](int, float (&x)[8]) {
+                    unsigned take = 0u;
 #pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        if (u == 1 && !two) break;
-                        unsigned take = 0u;
-#pragma unroll
-                        for (int j = 0; j < 8; j++)
-                            if (x[u][j] >= lo_e) {
-                                const int b = row_bin(__float_as_uint(x[u][j]));
-                                if (((sh.new_bits[b >> 5] >> (b & 31)) & 1u) && prob(x[u][j]) > 0.f) take |= 1u << j;
-                            }
-                        append(list, kRowList, &sh.list_n, take, [&](int j) { return __float_as_uint(x[u][j]); });
-                    }
-                }
+                    for (int j = 0; j < 8; j++)
+                        if (x[j] >= lo_e) {
+                            const int b = row_bin(__float_as_uint(x[j]));
+                            if (((sh.new_bits[b >> 5] >> (b & 31)) & 1u) && prob(x[j]) > 0.f) take |= 1u << j;
+                        }
+                    append(list, kRowList, &sh.list_n, take, [&](int j) { return __float_as_uint(x[j]); });
+                });
                 hand_over();
                 cl.sync();
             }
@@ -1630,6 +1769,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     const bool tied = d.tie_idx_max != INT_MAX;
     {
         double part[2] = {0.0, 0.0};
+        // two tiles to a turn: little is done with them, and it is their loads that count
         for (int t = t0 + warp; t < t1; t += 2 * kRW) {
             float x[2][8];
             get_e(t, x[0]);
@@ -1646,14 +1786,17 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                     part[j & 1] += widen(p);
                     acc += p;
                 }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+                acc = warp_sum_f(acc);
                 if (lane == 0) sh.tile_sum[t - t0 + u * kRW] = acc;
             }
         }
         const double all_part = block_sum_d(part[0] + part[1], sh.red_d);
-        if (tid < C) cl.map_shared_rank(&sh, tid)->part[rank] = all_part;
-        push_total(1);
+        tp = tile_prefix(sh.tile_sum, t1 - t0, sh.red_d);
+        if (tid < C) {
+            RowSh *o = cl.map_shared_rank(&sh, tid);
+            o->part[rank] = all_part;
+            o->tot[1][rank] = tp.all;
+        }
     }
     cl.sync();
     tick(tk, 10);
@@ -1670,9 +1813,12 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         if (rank == 0 && tid == 0) { if (a.row_flags) a.row_flags[row] = kPathFull | sh.flags; ws.redo[fi] = 0; }
         return;
     }
-    totals(1, base, mine, all);
-    auto get_p = [&](int t, float x[8]) {
-        load_e(e, t * kSub + lane * 8, x);
+    base = all = 0.0;
+    for (int r = 0; r < C; r++) {
+        if (r == rank) base = all;
+        all += sh.tot[1][r];
+    }
+    auto final_p = [&](int t, float (&x)[8]) {
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             float p = fin(x[j]);
@@ -1680,7 +1826,8 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
             x[j] = __fmul_rn(p, d.inv3);
         }
     };
-    summarise(sh, wa, dst, get_p, t0, t1, base, mine, all, (double)d.inv3, (double)u01);
+    auto get_p = [&](int t, float (&x)[8]) { get_e(t, x); final_p(t, x); };
+    summarise(sh, wa, dst, get_e, final_p, t0, t1, tp, base, all, (double)d.inv3, (double)u01);
     cl.sync();
     tick(tk, 11);
     if (rank != 0 || warp != 0) return;
@@ -1806,14 +1953,9 @@ __global__ void __launch_bounds__(kRT, 2) k_spec_row(const __grid_constant__ Spe
             }
         }
     }
-    __syncthreads();
     cl.barrier_wait();
-    if (warp == 0) {
-        double v = 0.0;
-        for (int t = lane; t < t1 - t0; t += 32) v += (double)sh.tile_sum[t];
-        v = warp_sum_d(v);
-        if (lane < C) cl.map_shared_rank(&sh, lane)->tot[0][rank] = v;
-    }
+    const TilePrefix tp = tile_prefix(sh.tile_sum, t1 - t0, sh.red_d);
+    if (tid < C) cl.map_shared_rank(&sh, tid)->tot[0][rank] = tp.all;
     cl.sync();
     double base = 0.0, all = 0.0;
     for (int r = 0; r < C; r++) {
@@ -1823,7 +1965,7 @@ __global__ void __launch_bounds__(kRT, 2) k_spec_row(const __grid_constant__ Spe
     const float u0 = __double2float_rn(u[L]);
     auto get = [&](int t, float x[8]) { load_e(e, t * kSub + lane * 8, x); };
     // the target of a residual is u times its sum: where it should lie is known well enough
-    summarise(sh, wa, dst, get, t0, t1, base, sh.tot[0][rank], all, 1.0, residual ? (double)u0 * all : (double)u0);
+    summarise(sh, wa, dst, get, [](int, float (&)[8]) {}, t0, t1, tp, base, all, 1.0, residual ? (double)u0 * all : (double)u0);
     cl.sync();
     pdl_release();
     if (rank != 0 || warp != 0) return;

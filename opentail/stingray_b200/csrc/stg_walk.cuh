@@ -45,6 +45,23 @@ struct WalkArea {
     float head[kSub];             // elements of tile 0
 };
 
+// What few tiles need lies out of line: inlined into the loops that all tiles go through it made those wait for their
+// own instructions.
+struct Lane8 { float v[8]; };  // by value: a called function gets a lane's elements in registers
+__device__ __forceinline__ Lane8 lane8(const float x[8])
+{
+    Lane8 l;
+#pragma unroll
+    for (int j = 0; j < 8; j++) l.v[j] = x[j];
+    return l;
+}
+static __device__ __noinline__ int2 composite_any(const Lane8 x, int g)
+{
+    int r0, r1;
+    subtile_composite<false>(x.v, g, r0, r1);
+    return make_int2(r0, r1);
+}
+
 struct WalkOut {
     float s;        // the sum at the hit, or the final sum
     float before;   // the sum just before the element that met the target
@@ -250,8 +267,9 @@ __device__ __forceinline__ void walk_runs(WalkArea *dst, const int2 *cmp, const 
 }
 
 // One warp: prepares the crossing of a tile from binade g (this lane's 8 elements in x)
-__device__ __forceinline__ void walk_cross(WalkCross *dst, const float x[8], int g)
+static __device__ __noinline__ void walk_cross(WalkCross *dst, const Lane8 e, int g)
 {
+    const float (&x)[8] = e.v;
     const int lane = threadIdx.x & 31;
     int l0, l1, h0, h1;
     lane_composite(x, g, l0, l1);
@@ -288,17 +306,20 @@ __device__ __forceinline__ void tile_composite(const float x[8], int g, int &r0,
     unsigned a = 0u;  // modulo 2^32
     float m = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        const float y = __fadd_rn(x[j], c);
-        a += __float_as_uint(y);
-        m = fmaxf(m, fabsf(__fsub_rn(x[j], __fsub_rn(y, c))));
+    for (int j = 0; j < 8; j += 2) {  // two elements to an instruction
+        const float2 v = make_float2(x[j], x[j + 1]), y = __fadd2_rn(v, make_float2(c, c)), z = __fadd2_rn(y, make_float2(-c, -c));
+        const float2 w = __ffma2_rn(z, make_float2(-1.f, -1.f), v);
+        a += __float_as_uint(y.x) + __float_as_uint(y.y);
+        m = fmaxf(m, fmaxf(fabsf(w.x), fabsf(w.y)));
     }
     a -= 8u * __float_as_uint(c);
     if (__ballot_sync(0xFFFFFFFFu, m == __uint_as_float((uint32_t)(g - 24) << 23)) == 0u) {
         r0 = r1 = (int)__reduce_add_sync(0xFFFFFFFFu, a);
         return;
     }
-    subtile_composite<false>(x, g, r0, r1);
+    const int2 r = composite_any(lane8(x), g);
+    r0 = r.x;
+    r1 = r.y;
 }
 
 }  // namespace stg
