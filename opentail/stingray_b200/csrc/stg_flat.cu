@@ -34,7 +34,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_flat_finish(const __grid_consta
     extern __shared__ __align__(16) unsigned char arena[];
     __shared__ SelCtl ctl;
     __shared__ FlatShared fs;
-    pdl_wait();
     flat_finish_row<BF16>(a, fr, a.items[blockIdx.x].row, blockIdx.x, a.cap, arena, ctl, fs);
     __syncthreads();  // all warps leave together, as in the smaller forms (stg_flat_finish_small.inc)
 }

@@ -99,6 +99,7 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
     const int esz = BF16 ? 2 : 4;
     const LogitRow rowp{(const char *)a.logits + (int64_t)row * a.row_stride * esz, a.softcap};
     if (rp.path == kPathGreedy) {
+        pdl_wait();
         if (a.shard_mode == 1) {
             // vocabulary-sharded mode: this rank's best (value, global token) goes to the exchange buffer
             // (the streaming kernel numbers tokens by column; the global id is column + vocab_offset, and
@@ -136,6 +137,16 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
         return;
     }
     unsigned long long *tk = a.phase_ticks ? a.phase_ticks + (int64_t)(a.item_base + item) * 32 : nullptr;
+    const int32_t *hist = a.hist_ids ? a.hist_ids + rp.hist_off : nullptr;
+    const float *ptab = (a.pow_tab && rp.pow_off >= 0) ? a.pow_tab + rp.pow_off : nullptr;
+    const float u = a.uniforms ? __ldg(a.uniforms + row) : 0.5f;
+    const int64_t o = (int64_t)row * a.topk_stride;
+    const bool fast = a.shard_mode == 0 && fast_eligible(rp, (size_t)cap * 16);
+    if (fast) finish_fast_begin(rp, hist, arena);
+    // Up to here while the streaming pass is on: the plan, the history and the uniforms were there before the step began, as prep
+    // is not launched behind anything in this way.  A lone row's step 16.3 -> 14.3 us, 96 rows with 256-token histories
+    // 47.2 -> 45.5.
+    pdl_wait();
     tick(tk, 0);
     if (threadIdx.x == 0) {
         const FlatRow f = fr[row];
@@ -143,13 +154,9 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
     }
     __syncthreads();
     const int cnt = fs.ok;
-    const int32_t *hist = a.hist_ids ? a.hist_ids + rp.hist_off : nullptr;
-    const float *ptab = (a.pow_tab && rp.pow_off >= 0) ? a.pow_tab + rp.pow_off : nullptr;
-    const float u = a.uniforms ? __ldg(a.uniforms + row) : 0.5f;
-    const int64_t o = (int64_t)row * a.topk_stride;
     // a list that holds the N best (and, with no penalty that raises a logit, may hold any number more)
-    if (a.shard_mode == 0 && fast_eligible(rp, cnt, (size_t)cap * 16) &&
-        finish_fast([&](int id) { return load_one<BF16>(rowp, id); }, a.cand + rp.cand_off, cnt, rp, hist, ptab, u, arena, &fs.fout,
+    if (fast && cnt > 0 &&
+        finish_fast([&](int id) { return load_one<BF16>(rowp, id); }, a.cand + rp.cand_off, cnt, rp, ptab, u, arena, &fs.fout,
                     a.topk_ids ? a.topk_ids + o : nullptr, a.topk_logits ? a.topk_logits + o : nullptr,
                     a.topk_probs ? a.topk_probs + o : nullptr)) {
         tick(tk, 4);

@@ -156,12 +156,12 @@ __device__ __forceinline__ void fast_draw(FastShared &fs, const RowPlan &rp, flo
 
 // Whether the list qualifies: no penalty can raise a logit, so that any superset of the N best raw logits holds
 // the k best penalised ones (see finish_topk_select), and the shared memory suffices.
-__device__ __forceinline__ bool fast_eligible(const RowPlan &rp, int cnt, size_t arena_bytes)
+__device__ __forceinline__ bool fast_eligible(const RowPlan &rp, size_t arena_bytes)
 {
     int hslots = 0;
     if (rp.has_penalty)
         for (hslots = 64; hslots < 2 * rp.hist_len;) hslots <<= 1;
-    return sizeof(FastShared) + (kThreads / 64) * 256 * 8 + (size_t)hslots * 8 <= arena_bytes && cnt > 0 && rp.top_k <= kFastK &&
+    return sizeof(FastShared) + (kThreads / 64) * 256 * 8 + (size_t)hslots * 8 <= arena_bytes && rp.top_k <= kFastK &&
            (!rp.has_penalty || (rp.rep >= 1.0f && rp.pres >= 0.f && rp.freq >= 0.f));
 }
 
@@ -245,29 +245,27 @@ __device__ __noinline__ bool order_by_raw(const Raw raw, u64 *buf, int k)
     return false;
 }
 
-// One CTA, all threads; `list`: cnt keys in device memory, `arena`: shared memory, (kThreads / 64) * 32 * KPL * 8
-// bytes for the merges and, behind them, 8 bytes per slot of the history's hash.  False: nothing was written,
-// the general path has to do the row.  raw(id): the row's logit at token id.
-template <int KPL, class Raw>
-__device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, int cnt, const RowPlan &rp, const int32_t *hist,
-                                              const float *pow_tab, float uniform, unsigned char *arena, FastShared &fs, FinishOut *out)
+// Where a row's hash of its history lies in the arena, and its slots
+__device__ __forceinline__ int *fast_hash_at(const RowPlan &rp, unsigned char *arena)
 {
-    constexpr int K2 = 32 * KPL, W = kThreads / 32;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    u64 *merge = (u64 *)arena;
-    int *hkey = (int *)(arena + (W / 2) * K2 * 8);
-    int hslots = 64;
-    while (hslots < 2 * rp.hist_len) hslots <<= 1;
-    unsigned *hcnt = (unsigned *)(hkey + hslots);
-    const bool pen = rp.has_penalty != 0;
-    u64 r[KPL], nx[KPL];
-#pragma unroll
-    for (int q = 0; q < KPL; q++) {
-        const int i = warp * K2 + q * 32 + lane;
-        r[q] = i < cnt ? __ldcg(list + i) : 0ull;  // in flight while the history is hashed
-    }
-    if (tid == 0) fs.fail = 0;
-    if (pen) {
+    return (int *)(arena + sizeof(FastShared) + (kThreads / 64) * 32 * (rp.top_k < 64 ? 2 : rp.top_k < 128 ? 4 : 8) * 8);
+}
+__device__ __forceinline__ int fast_hash_slots(const RowPlan &rp)
+{
+    int n = 64;
+    while (n < 2 * rp.hist_len) n <<= 1;
+    return n;
+}
+// One CTA, all threads: what the finish of a row needs besides its candidates, done while those are still being found.
+// Ends in a block barrier.
+__device__ __forceinline__ void finish_fast_begin(const RowPlan &rp, const int32_t *hist, unsigned char *arena)
+{
+    const int tid = threadIdx.x;
+    if (tid == 0) ((FastShared *)arena)->fail = 0;
+    if (rp.has_penalty) {
+        int *hkey = fast_hash_at(rp, arena);
+        const int hslots = fast_hash_slots(rp);
+        unsigned *hcnt = (unsigned *)(hkey + hslots);
 #pragma unroll 1
         for (int t = tid; t < hslots; t += kThreads) { hkey[t] = -1; hcnt[t] = 0u; }
         __syncthreads();
@@ -284,7 +282,29 @@ __device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, i
             }
             atomicAdd(&hcnt[h], 1u + (t >= rp.window_start ? 65536u : 0u));
         }
-        __syncthreads();
+    }
+    __syncthreads();
+}
+
+// One CTA, all threads, behind finish_fast_begin; `list`: cnt keys in device memory, `arena`: shared memory, (kThreads / 64) *
+// 32 * KPL * 8 bytes for the merges and, behind them, 8 bytes per slot of the history's hash.  False: nothing was written,
+// the general path has to do the row.  raw(id): the row's logit at token id.
+template <int KPL, class Raw>
+__device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, int cnt, const RowPlan &rp, const float *pow_tab,
+                                              float uniform, unsigned char *arena, FastShared &fs, FinishOut *out)
+{
+    constexpr int K2 = 32 * KPL, W = kThreads / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    u64 *merge = (u64 *)arena;
+    const int *hkey = (const int *)(arena + (W / 2) * K2 * 8);
+    const int hslots = fast_hash_slots(rp);
+    const unsigned *hcnt = (const unsigned *)(hkey + hslots);
+    const bool pen = rp.has_penalty != 0;
+    u64 r[KPL], nx[KPL];
+#pragma unroll
+    for (int q = 0; q < KPL; q++) {
+        const int i = warp * K2 + q * 32 + lane;
+        r[q] = i < cnt ? __ldcg(list + i) : 0ull;
     }
     const int lists = (cnt + K2 - 1) / K2;
     if (pen) {
@@ -366,7 +386,7 @@ __device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, i
 }
 
 template <class Raw>
-__device__ __forceinline__ bool finish_fast(const Raw &raw, const u64 *list, int cnt, const RowPlan &rp, const int32_t *hist,
+__device__ __forceinline__ bool finish_fast(const Raw &raw, const u64 *list, int cnt, const RowPlan &rp,
                                             const float *pow_tab, float uniform, unsigned char *arena, FinishOut *out, int32_t *o_ids,
                                             float *o_vals, float *o_probs)
 {
@@ -374,9 +394,9 @@ __device__ __forceinline__ bool finish_fast(const Raw &raw, const u64 *list, int
     arena += sizeof(FastShared);
     static_assert(sizeof(FastShared) % 16 == 0, "what follows is aligned");
     bool ok;
-    if (rp.top_k < 64) ok = finish_fast_k<2>(raw, list, cnt, rp, hist, pow_tab, uniform, arena, fs, out);
-    else if (rp.top_k < 128) ok = finish_fast_k<4>(raw, list, cnt, rp, hist, pow_tab, uniform, arena, fs, out);
-    else ok = finish_fast_k<8>(raw, list, cnt, rp, hist, pow_tab, uniform, arena, fs, out);
+    if (rp.top_k < 64) ok = finish_fast_k<2>(raw, list, cnt, rp, pow_tab, uniform, arena, fs, out);
+    else if (rp.top_k < 128) ok = finish_fast_k<4>(raw, list, cnt, rp, pow_tab, uniform, arena, fs, out);
+    else ok = finish_fast_k<8>(raw, list, cnt, rp, pow_tab, uniform, arena, fs, out);
     if (!ok) return false;
 #pragma unroll 1
     for (int t = threadIdx.x; t < rp.top_k; t += kThreads) {

@@ -8,7 +8,7 @@ from tests import parity
 pytestmark = pytest.mark.gpu
 
 
-def _run(logits, params, hist=None, seed=5):
+def _run(logits, params, hist=None, seed=5, max_top_k=8):
     from opentail.stingray_b200 import BatchSampler, workloads as W
 
     rows, vocab = logits.shape
@@ -18,9 +18,9 @@ def _run(logits, params, hist=None, seed=5):
         ids = np.concatenate(hist).astype(np.int32)
         off = np.concatenate([[0], np.cumsum([len(h) for h in hist])]).astype(np.int32)
     w = W.SampleWorkload("s", np.ascontiguousarray(logits), params, W.uniforms24(rng, rows), ids, off, None)
-    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=2048, max_top_k=8)
+    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=2048, max_top_k=max_top_k)
     try:
-        stats = parity.compare(w, parity.run_gpu(bs, w))
+        stats = parity.compare(w, parity.run_gpu(bs, w, want_topk=int(params["top_k"].max())))
         assert stats["mismatch"] == stats["boundary_draws"] <= 1
     finally:
         bs.close()
@@ -73,3 +73,24 @@ def test_tiles_of_very_different_weight(vocab):
     p["top_p"] = 1.0
     p["min_p"] = 0.0
     _run(x, p)
+
+
+@pytest.mark.parametrize("top_k", [63, 64, 127, 128, 255, 256])
+@pytest.mark.parametrize("rows", [8, 300])
+def test_top_k_at_the_sizes_of_the_register_sort(top_k, rows):
+    """Where the sort takes twice as many keys and the history's hash, filled ahead of the candidates, lies elsewhere: logits in
+    steps of 1/4, penalised in small steps, half of the tokens near the cut in the history."""
+    from opentail.stingray_b200 import workloads as W
+
+    vocab = 32_000
+    rng = np.random.default_rng(top_k)
+    x = (np.round(rng.normal(0, 2.0, (rows, vocab)) * 4) / 4).astype(np.float32)
+    hist = []
+    for r in range(rows):
+        order = np.argsort(-x[r], kind="stable")[: 2 * top_k]
+        hist.append(order[rng.random(order.size) < (0.2, 0.5, 0.9)[r % 3]])
+    p = W._params(rows)
+    p["temperature"], p["top_p"], p["top_k"], p["repeat_last_n"] = 0.9, 0.98, top_k, 0
+    p["repetition_penalty"] = np.resize([1.0, 1.1, 1.25], rows)
+    p["presence_penalty"] = np.resize([0.25, 0.0, 0.5, 0.125], rows)
+    _run(x, p, hist, max_top_k=512)
