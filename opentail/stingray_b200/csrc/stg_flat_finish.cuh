@@ -156,7 +156,7 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
     const int cnt = fs.ok;
     // a list that holds the N best (and, with no penalty that raises a logit, may hold any number more)
     if (fast && cnt > 0 &&
-        finish_fast([&](int id) { return load_one<BF16>(rowp, id); }, a.cand + rp.cand_off, cnt, rp, ptab, u, arena, &fs.fout,
+        finish_fast(a.cand + rp.cand_off, cnt, rp, ptab, u, arena, (size_t)cap * 16, &fs.fout,
                     a.topk_ids ? a.topk_ids + o : nullptr, a.topk_logits ? a.topk_logits + o : nullptr,
                     a.topk_probs ? a.topk_probs + o : nullptr)) {
         tick(tk, 4);

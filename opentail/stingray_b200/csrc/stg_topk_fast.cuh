@@ -1,17 +1,12 @@
-// The finish of a top-k row from its candidate list, without sorting or radix-selecting the list.
+// The finish of a top-k row from its candidate list, without sorting the list.
 //
-// Every warp sorts its share of the list in registers (bitonic, keys exchanged by shuffles) and keeps its best
-// K2 = 32 * KPL keys; a tree of merges over the warps leaves the row's best K2 in the first warp, which
-// also runs the softmax, the filters and the draw of Sampler.cs:296-349.  The radix selection it stands in
-// for crosses two block barriers per digit and ranks ties against the whole list: on 96 rows of bf16 logits
-// (which tie in droves) with 256-token histories the finish took 70 us and takes 27, a lone row's step of
-// 151,936 logits went from 25 to 19 us.  Bound: latency of a few dozen dependent shuffles.
+// The row's order is (penalised value, raw logit, lower token first): a candidate is the pair (penalised value, raw logit)
+// in one 64-bit word, and its token.  The k best are fenced off by a histogram over the range of the penalised values, refined
+// inside the bin that holds the k-th until no more than kFastM candidates lie above its lower edge; those are put in
+// order by counting, each by a thread, which also computes its exp; then one warp runs the filters and the draw of
+// Sampler.cs:296-349.  Equal values share a bin, so ties at the k-th are all there to be ordered.
 //
-// The row's order is (penalised value descending, raw order among equals).  Keys hold the penalised value, a
-// bit that says a penalty lowered it - its raw logit was higher than those of its equals that none did, so it
-// comes first - and the token.  Lowered logits that come out equal from different raw values (common with bf16:
-// 11 / 1.1^2 = 10 / 1.1) are put into raw order at the end; left to the general path they made a step of 96
-// rows of 151,936 with histories of their own sampled tokens take 102 us instead of 47.
+// Bound: latency of a dozen dependent steps, six block barriers.
 #pragma once
 #include <math_constants.h>
 
@@ -19,60 +14,24 @@
 
 namespace stg {
 
-constexpr int kFastK = 255;       // largest top_k: one more key than k has to be seen
+constexpr int kFastK = 256;       // largest top_k
+constexpr int kFastM = 512;       // candidates put in order at most
+constexpr int kFastRoom = 1024;   // candidates there is room for at least
 
 struct FastShared {
     float vals[256], probs[256], pre[256];
     int ids[256];
-    int fail, pad[3];
+    u64 best[kFastM];
+    int tok[kFastM];
+    unsigned hist[256];
+    unsigned lo[32], hi[32];   // smallest and largest penalised value of each warp
+    unsigned base;             // lower edge of the window, then of the k best's bin
+    int shift;                 // bins of 2^shift values
+    int want;                  // how many of the k best lie in the window
+    int above;                 // candidates above the window
+    int state;                 // 0: another round, 1: fenced off, 2: too many equal values
+    int n, pad[2];
 };
-
-__device__ __forceinline__ int fast_idx(u64 k) { return (int)(0x7FFFFFFFu - ((uint32_t)k & 0x7FFFFFFFu)); }
-
-// steps j0 .. 1 of stage k of a bitonic sort (descending) of 32 * KPL keys; key i is r[i / 32] of lane i % 32.
-// Unrolled: in loops the same steps made a lone row's step 21.5 us instead of 18.8.
-template <int KPL>
-__device__ __forceinline__ void warp_steps(u64 (&r)[KPL], int k, int j0)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int j = 16 * KPL; j > 0; j >>= 1) {
-        if (j > j0) continue;
-        if (j >= 32) {
-            const int dj = j / 32;
-#pragma unroll
-            for (int q = 0; q < KPL; q++) {
-                if ((q & dj) == 0) {
-                    const bool desc = ((q * 32 + lane) & k) == 0;
-                    const u64 x = r[q], y = r[q | dj];
-                    if ((x < y) == desc) { r[q] = y; r[q | dj] = x; }
-                }
-            }
-        } else {
-            const bool lower = (lane & j) == 0;
-#pragma unroll
-            for (int q = 0; q < KPL; q++) {
-                const bool desc = ((q * 32 + lane) & k) == 0;
-                const u64 o = __shfl_xor_sync(0xFFFFFFFFu, r[q], j);
-                r[q] = (lower == desc) ? (r[q] > o ? r[q] : o) : (r[q] < o ? r[q] : o);
-            }
-        }
-    }
-}
-template <int KPL>
-__device__ __forceinline__ void warp_sort(u64 (&r)[KPL])
-{
-#pragma unroll
-    for (int k = 2; k <= 32 * KPL; k <<= 1) warp_steps<KPL>(r, k == 32 * KPL ? 1 << 30 : k, k >> 1);
-}
-// r = the best keys of r and of another descending list given reversed: rev[q] holds key 32 * KPL - 1 - (32 q + lane)
-template <int KPL>
-__device__ __forceinline__ void warp_best(u64 (&r)[KPL], const u64 (&rev)[KPL])
-{
-#pragma unroll
-    for (int q = 0; q < KPL; q++) r[q] = r[q] > rev[q] ? r[q] : rev[q];
-    warp_steps<KPL>(r, 1 << 30, 16 * KPL);
-}
 
 // o[i] = fl(o[i - 1] + x[i]) from 0 for i < m (a multiple of 8); one warp, returns the last
 __device__ __forceinline__ float warp_prefix_serial(const float *x, float *o, int m)
@@ -96,22 +55,11 @@ __device__ __forceinline__ float warp_prefix_serial(const float *x, float *o, in
 }
 
 // What is left of the row for one warp: softmax over the k ordered candidates, min-p, top-p, the draw
-// (Sampler.cs:296-349; every fp32 operation as in finish_topk_draw).  vals / ids [k] are in `fs`.
+// (Sampler.cs:296-349; every fp32 operation as in finish_topk_draw).  vals, their exps in probs, and ids [k] are in `fs`, zeros
+// in probs behind them up to a multiple of eight.
 __device__ __forceinline__ void fast_draw(FastShared &fs, const RowPlan &rp, float uniform, FinishOut *out)
 {
     const int lane = threadIdx.x & 31, k = rp.top_k, k8 = (k + 7) & ~7;
-    const float inv_t = rp.temperature == 1.0f ? 1.0f : __fdiv_rn(1.0f, rp.temperature);
-    const float mx = __fmul_rn(fs.vals[0], inv_t);
-#pragma unroll 1
-    for (int t = lane; t < k8; t += 32) {
-        float e = 0.f;
-        if (t < k) {
-            const float v = fs.vals[t];
-            if (!(isinf(v) && v < 0.f)) e = (float)exp((double)__fsub_rn(__fmul_rn(v, inv_t), mx));
-        }
-        fs.probs[t] = e;
-    }
-    __syncwarp();
     const float sum = warp_prefix_serial(fs.probs, fs.pre, k8);
     const float inv_sum = sum > 0.f ? __fdiv_rn(1.0f, sum) : 0.f;
 #pragma unroll 1
@@ -154,117 +102,29 @@ __device__ __forceinline__ void fast_draw(FastShared &fs, const RowPlan &rp, flo
     }
 }
 
-// Whether the list qualifies: no penalty can raise a logit, so that any superset of the N best raw logits holds
+// Whether the row qualifies: no penalty can raise a logit, so that any superset of the N best raw logits holds
 // the k best penalised ones (see finish_topk_select), and the shared memory suffices.
+__device__ __forceinline__ int fast_hash_slots(const RowPlan &rp)
+{
+    int n = 0;
+    if (rp.has_penalty)
+        for (n = 64; n < 2 * rp.hist_len;) n <<= 1;
+    return n;
+}
 __device__ __forceinline__ bool fast_eligible(const RowPlan &rp, size_t arena_bytes)
 {
-    int hslots = 0;
-    if (rp.has_penalty)
-        for (hslots = 64; hslots < 2 * rp.hist_len;) hslots <<= 1;
-    return sizeof(FastShared) + (kThreads / 64) * 256 * 8 + (size_t)hslots * 8 <= arena_bytes && rp.top_k <= kFastK &&
+    return sizeof(FastShared) + (size_t)fast_hash_slots(rp) * 8 + kFastRoom * 12 <= arena_bytes && rp.top_k <= kFastK &&
            (!rp.has_penalty || (rp.rep >= 1.0f && rp.pres >= 0.f && rp.freq >= 0.f));
 }
 
-// Occurrences of `id` in the history | inside the window << 16.  Whole warps call it, and the warp leaves the loop
-// together, when the last of its lanes is done: with a loop that each lane left by itself the lane that had found its
-// token stayed apart from the others through the shuffles of the sort behind it, and its warp's candidates were lost
-// (rows of 262,144 bf16 logits behind 700-token histories: once in 400 to 9,000 steps, a `__syncwarp` notwithstanding).
-__device__ __forceinline__ unsigned fast_occurrences(const int *hkey, const unsigned *hcnt, int hmask, int id)
-{
-    int h = (int)(((unsigned)id * 2654435761u) >> 7) & hmask;
-    int at = -1;
-    bool open = true;
-#pragma unroll 1
-    while (__any_sync(0xFFFFFFFFu, open)) {
-        const int kx = hkey[h];
-        at = open && kx == id ? h : at;
-        open = open && kx != id && kx != -1;
-        h = (h + 1) & hmask;
-    }
-    return at >= 0 ? hcnt[at] : 0u;
-}
-// the keys of a warp's candidates (0: none) with the penalties applied (Sampler.cs:263-287)
-__device__ __forceinline__ u64 fast_penalise(u64 key, const int *hkey, const unsigned *hcnt, int hmask, const RowPlan &rp, const float *pow_tab)
-{
-    key &= 0xFFFFFFFF7FFFFFFFull;
-    unsigned c = fast_occurrences(hkey, hcnt, hmask, fast_idx(key));
-    if (key == 0ull) c = 0u;  // reads as token 2^31 - 1
-    if (!__any_sync(0xFFFFFFFFu, c != 0u)) return key;
-    float x = key_val(key);
-    const int occ_all = (int)(c & 0xFFFFu), occ_w = (int)(c >> 16);
-    if (rp.rep != 1.0f && occ_w > 0) {
-        const float pw = pow_rep(pow_tab, rp.rep, occ_w);
-        x = x > 0.f ? __fdiv_rn(x, pw) : __fmul_rn(x, pw);
-    }
-    x = __fsub_rn(x, __fadd_rn(rp.pres, __fmul_rn(rp.freq, (float)occ_all)));
-    __syncwarp();
-    const uint32_t was = (uint32_t)(key >> 32), now = ord32(x);
-    return c != 0u ? ((u64)now << 32) | (key & 0x7FFFFFFFull) | (now != was ? 0x80000000ull : 0ull) : key;
-}
-
-// The sorted keys of one warp, with every run of equal lowered values put into the order of the raw logits.  Keys behind
-// the last one were dropped, so a run that reaches it may lack members; that, or a run beyond 32, is answered
-// with true: the general path.  `buf`: the 32 * KPL keys, in shared memory.
-template <int KPL, class Raw>
-__device__ __noinline__ bool order_by_raw(const Raw raw, u64 *buf, int k)
-{
-    constexpr int K2 = 32 * KPL;
-    const int lane = threadIdx.x & 31;
-    bool fail = false;
-    u64 r[KPL];
-    int to[KPL];
-#pragma unroll
-    for (int q = 0; q < KPL; q++) {
-        const int i = q * 32 + lane;
-        const u64 key = buf[i];
-        r[q] = key;
-        int at = i;
-        if ((key >> 31) & 1ull) {
-            int lo = i, hi = i;
-            while (lo > 0 && i - lo < 32 && (buf[lo - 1] >> 31) == (key >> 31)) lo--;
-            while (hi + 1 < K2 && hi - i < 32 && (buf[hi + 1] >> 31) == (key >> 31)) hi++;
-            if (lo < k && (hi == K2 - 1 || hi - lo >= 32)) {
-                fail = true;
-            } else if (lo < k && lo < hi) {
-                const uint32_t mine = ord32(__fadd_rn(raw(fast_idx(key)), 0.f));
-                at = lo;
-                for (int j = lo; j <= hi; j++) {
-                    if (j == i) continue;
-                    const uint32_t other = ord32(__fadd_rn(raw(fast_idx(buf[j])), 0.f));
-                    at += other > mine || (other == mine && j < i) ? 1 : 0;
-                }
-            }
-        }
-        to[q] = at;
-    }
-    __syncwarp();
-    if (__any_sync(0xFFFFFFFFu, fail)) return true;
-#pragma unroll
-    for (int q = 0; q < KPL; q++) buf[to[q]] = r[q];
-    __syncwarp();
-    return false;
-}
-
-// Where a row's hash of its history lies in the arena, and its slots
-__device__ __forceinline__ int *fast_hash_at(const RowPlan &rp, unsigned char *arena)
-{
-    return (int *)(arena + sizeof(FastShared) + (kThreads / 64) * 32 * (rp.top_k < 64 ? 2 : rp.top_k < 128 ? 4 : 8) * 8);
-}
-__device__ __forceinline__ int fast_hash_slots(const RowPlan &rp)
-{
-    int n = 64;
-    while (n < 2 * rp.hist_len) n <<= 1;
-    return n;
-}
-// One CTA, all threads: what the finish of a row needs besides its candidates, done while those are still being found.
-// Ends in a block barrier.
+// One CTA, all threads: what the finish of a row needs besides its candidates, done while those are still being found: the
+// hash of its history, token -> occurrences | inside the window << 16, behind the FastShared.
 __device__ __forceinline__ void finish_fast_begin(const RowPlan &rp, const int32_t *hist, unsigned char *arena)
 {
     const int tid = threadIdx.x;
-    if (tid == 0) ((FastShared *)arena)->fail = 0;
     if (rp.has_penalty) {
-        int *hkey = fast_hash_at(rp, arena);
         const int hslots = fast_hash_slots(rp);
+        int *hkey = (int *)(arena + sizeof(FastShared));
         unsigned *hcnt = (unsigned *)(hkey + hslots);
 #pragma unroll 1
         for (int t = tid; t < hslots; t += kThreads) { hkey[t] = -1; hcnt[t] = 0u; }
@@ -286,120 +146,196 @@ __device__ __forceinline__ void finish_fast_begin(const RowPlan &rp, const int32
     __syncthreads();
 }
 
-// One CTA, all threads, behind finish_fast_begin; `list`: cnt keys in device memory, `arena`: shared memory, (kThreads / 64) *
-// 32 * KPL * 8 bytes for the merges and, behind them, 8 bytes per slot of the history's hash.  False: nothing was written,
-// the general path has to do the row.  raw(id): the row's logit at token id.
-template <int KPL, class Raw>
-__device__ __forceinline__ bool finish_fast_k(const Raw &raw, const u64 *list, int cnt, const RowPlan &rp, const float *pow_tab,
-                                              float uniform, unsigned char *arena, FastShared &fs, FinishOut *out)
+// The penalised values of a warp's candidates (Sampler.cs:263-287), as ordered bits; key 0: none.  Whole warps call it, and the
+// warp leaves the lookup's loop together, when the last of its lanes is done: with a loop that each lane left by itself
+// the lane that had found its token stayed apart from the others through the shuffles behind it, and a warp's
+// candidates were lost (rows of 262,144 bf16 logits behind 700-token histories: once in 400 to 9,000 steps, a
+// `__syncwarp` notwithstanding).  A lane's keys are looked up side by side.
+template <int U>
+__device__ __forceinline__ void fast_penalise(const u64 (&key)[U], uint32_t (&pv)[U], const int *hkey, const unsigned *hcnt, int hmask,
+                                              const RowPlan &rp, const float *pow_tab)
 {
-    constexpr int K2 = 32 * KPL, W = kThreads / 32;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    u64 *merge = (u64 *)arena;
-    const int *hkey = (const int *)(arena + (W / 2) * K2 * 8);
-    const int hslots = fast_hash_slots(rp);
-    const unsigned *hcnt = (const unsigned *)(hkey + hslots);
-    const bool pen = rp.has_penalty != 0;
-    u64 r[KPL], nx[KPL];
+    int h[U], at[U];
+    unsigned open = 0u;
 #pragma unroll
-    for (int q = 0; q < KPL; q++) {
-        const int i = warp * K2 + q * 32 + lane;
-        r[q] = i < cnt ? __ldcg(list + i) : 0ull;
-    }
-    const int lists = (cnt + K2 - 1) / K2;
-    if (pen) {
-#pragma unroll
-        for (int q = 0; q < KPL; q++) r[q] = fast_penalise(r[q], hkey, hcnt, hslots - 1, rp, pow_tab);
-    }
-    warp_sort<KPL>(r);
-#pragma unroll 1
-    for (int l = warp + W; l < lists; l += W) {
-#pragma unroll
-        for (int q = 0; q < KPL; q++) {
-            const int i = l * K2 + q * 32 + lane;
-            nx[q] = i < cnt ? __ldcg(list + i) : 0ull;
-        }
-        if (pen) {
-#pragma unroll
-            for (int q = 0; q < KPL; q++) nx[q] = fast_penalise(nx[q], hkey, hcnt, hslots - 1, rp, pow_tab);
-        }
-        warp_sort<KPL>(nx);
-        u64 rev[KPL];
-#pragma unroll
-        for (int q = 0; q < KPL; q++) rev[q] = __shfl_xor_sync(0xFFFFFFFFu, nx[KPL - 1 - q], 31);
-        warp_best<KPL>(r, rev);
+    for (int q = 0; q < U; q++) {
+        pv[q] = (uint32_t)(key[q] >> 32);
+        h[q] = (int)(((unsigned)key_idx(key[q]) * 2654435761u) >> 7) & hmask;
+        at[q] = -1;
+        open |= key[q] != 0ull ? 1u << q : 0u;
     }
 #pragma unroll 1
-    for (int w = W / 2; w > 0; w >>= 1) {
-        if (w < lists) {  // the warps from `lists` on hold nothing
-            if (warp >= w && warp < 2 * w) {
+    while (__any_sync(0xFFFFFFFFu, open != 0u)) {
 #pragma unroll
-                for (int q = 0; q < KPL; q++) merge[(size_t)(warp - w) * K2 + q * 32 + lane] = r[q];
-            }
-            __syncthreads();
-            if (warp < w) {
-                u64 rev[KPL];
-#pragma unroll
-                for (int q = 0; q < KPL; q++) rev[q] = merge[(size_t)warp * K2 + K2 - 1 - (q * 32 + lane)];
-                warp_best<KPL>(r, rev);
-            }
-            __syncthreads();
+        for (int q = 0; q < U; q++) {
+            const int kx = hkey[h[q]], id = key_idx(key[q]);
+            at[q] = ((open >> q) & 1u) && kx == id ? h[q] : at[q];
+            open &= kx == id || kx == -1 ? ~(1u << q) : 0xFFFFFFFFu;
+            h[q] = (h[q] + 1) & hmask;
         }
     }
-    if (warp == 0) {
-        const int k = rp.top_k;
-        bool fail = false;
-        if (pen) {
-            bool tie = false;
 #pragma unroll
-            for (int q = 0; q < KPL; q++) {
-                // the key behind this one
-                u64 next = __shfl_down_sync(0xFFFFFFFFu, r[q], 1);
-                const u64 head = q + 1 < KPL ? __shfl_sync(0xFFFFFFFFu, r[q + 1 < KPL ? q + 1 : q], 0) : 0ull;
-                if (lane == 31) next = head;
-                tie |= q * 32 + lane < k && next != 0ull && (r[q] >> 31) == (next >> 31) && ((r[q] >> 31) & 1ull);
-            }
-            if (__any_sync(0xFFFFFFFFu, tie)) {
-#pragma unroll
-                for (int q = 0; q < KPL; q++) merge[q * 32 + lane] = r[q];
-                __syncwarp();
-                fail = order_by_raw<KPL>(raw, merge, k);
-#pragma unroll
-                for (int q = 0; q < KPL; q++) r[q] = merge[q * 32 + lane];
-            }
+    for (int q = 0; q < U; q++) {
+        if (!__any_sync(0xFFFFFFFFu, at[q] >= 0)) continue;
+        const unsigned c = at[q] >= 0 ? hcnt[at[q]] : 0u;
+        float x = key_val(key[q]);
+        const int occ_all = (int)(c & 0xFFFFu), occ_w = (int)(c >> 16);
+        if (rp.rep != 1.0f && occ_w > 0) {
+            const float pw = pow_rep(pow_tab, rp.rep, occ_w);
+            x = x > 0.f ? __fdiv_rn(x, pw) : __fmul_rn(x, pw);
         }
-#pragma unroll
-        for (int q = 0; q < KPL; q++) {
-            const int i = q * 32 + lane;
-            if (i < k) {
-                fs.vals[i] = r[q] ? key_val(r[q]) : -CUDART_INF_F;
-                fs.ids[i] = r[q] ? fast_idx(r[q]) : -1;
-            }
-        }
-        fail = __any_sync(0xFFFFFFFFu, fail);
+        x = __fsub_rn(x, __fadd_rn(rp.pres, __fmul_rn(rp.freq, (float)occ_all)));
         __syncwarp();
-        if (!fail) fast_draw(fs, rp, uniform, out);
-        else if (lane == 0) fs.fail = 1;
+        if (c != 0u) pv[q] = ord32(x);
     }
-    __syncthreads();
-    return fs.fail == 0;
 }
 
-template <class Raw>
-__device__ __forceinline__ bool finish_fast(const Raw &raw, const u64 *list, int cnt, const RowPlan &rp,
-                                            const float *pow_tab, float uniform, unsigned char *arena, FinishOut *out, int32_t *o_ids,
-                                            float *o_vals, float *o_probs)
+// One CTA, all threads, behind finish_fast_begin; `list`: cnt keys in device memory, `arena`: shared memory, the FastShared, the
+// history's hash, then 12 bytes per candidate; a list that does not fit is read and penalised again in every pass.
+// False: nothing was written, the general path has to do the row.
+__device__ __forceinline__ bool finish_fast(const u64 *list, int cnt, const RowPlan &rp, const float *pow_tab, float uniform,
+                                            unsigned char *arena, size_t arena_bytes, FinishOut *out, int32_t *o_ids, float *o_vals,
+                                            float *o_probs)
 {
+    constexpr int U = 4;
     FastShared &fs = *(FastShared *)arena;
-    arena += sizeof(FastShared);
     static_assert(sizeof(FastShared) % 16 == 0, "what follows is aligned");
-    bool ok;
-    if (rp.top_k < 64) ok = finish_fast_k<2>(raw, list, cnt, rp, pow_tab, uniform, arena, fs, out);
-    else if (rp.top_k < 128) ok = finish_fast_k<4>(raw, list, cnt, rp, pow_tab, uniform, arena, fs, out);
-    else ok = finish_fast_k<8>(raw, list, cnt, rp, pow_tab, uniform, arena, fs, out);
-    if (!ok) return false;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = rp.top_k, hslots = fast_hash_slots(rp);
+    const int *hkey = (const int *)(arena + sizeof(FastShared));
+    const unsigned *hcnt = (const unsigned *)(hkey + hslots);
+    const int room = (int)((arena_bytes - sizeof(FastShared) - (size_t)hslots * 8) / 12);
+    const bool stored = cnt <= room;
+    if (cnt < k) return false;
+    u64 *pk = (u64 *)(arena + sizeof(FastShared) + (size_t)hslots * 8);  // penalised value << 32 | raw logit, ordered bits
+    int *pt = (int *)(pk + room);
+    if (tid < 256) fs.hist[tid] = 0u;
+    if (tid < 8) fs.probs[(k + tid) & 255] = 0.f;  // behind the last, where the sums read
+    enum { kRange, kBinned, kTake };
+    int pass = kRange, shift = 0, want = k, above = 0;
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u, top = 0u;
 #pragma unroll 1
-    for (int t = threadIdx.x; t < rp.top_k; t += kThreads) {
+    for (;;) {
+        auto visit = [&](u64 x, int tok, int i) {
+            const uint32_t v = (uint32_t)(x >> 32);
+            if (pass == kRange) {
+                lo = min(lo, v);
+                hi = max(hi, v);
+                if (stored) { pk[i] = x; pt[i] = tok; }
+            } else if (pass == kBinned) {
+                const uint32_t d = (top - v) >> shift;
+                if (v <= top && d < 256u) atomicAdd(&fs.hist[d], 1u);
+            } else if (v >= top) {
+                const int slot = atomicAdd(&fs.n, 1);
+                fs.best[slot] = x;
+                fs.tok[slot] = tok;
+            }
+        };
+        if (pass == kRange || !stored) {
+#pragma unroll 1
+            for (int b = 0; b < cnt; b += U * kThreads) {
+                u64 key[U];
+                uint32_t pv[U];
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    const int i = b + q * kThreads + tid;
+                    key[q] = i < cnt ? __ldcg(list + i) : 0ull;
+                    pv[q] = (uint32_t)(key[q] >> 32);
+                }
+                if (rp.has_penalty) fast_penalise<U>(key, pv, hkey, hcnt, hslots - 1, rp, pow_tab);
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    const int i = b + q * kThreads + tid;
+                    if (i < cnt) visit((u64)pv[q] << 32 | (key[q] >> 32), key_idx(key[q]), i);
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int i = tid; i < cnt; i += kThreads) visit(pk[i], pt[i], i);
+        }
+        if (pass == kTake) break;
+        if (pass == kRange) {
+            const uint32_t l = __reduce_min_sync(0xFFFFFFFFu, lo), h = __reduce_max_sync(0xFFFFFFFFu, hi);
+            if (lane == 0) { fs.lo[warp] = l; fs.hi[warp] = h; }
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < kThreads / 32; w++) { lo = min(lo, fs.lo[w]); hi = max(hi, fs.hi[w]); }
+            // a window of 256 bins from the largest value downwards: value v in bin (top - v) >> shift
+            top = hi;
+            shift = max(24 - __clz((int)(hi - lo)), 0);
+            pass = kBinned;
+            continue;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (lane == 0) { fs.state = 2; fs.n = 0; }
+            __syncwarp();
+            unsigned h[8], sum = 0u;
+#pragma unroll
+            for (int j = 0; j < 8; j++) { h[j] = fs.hist[lane * 8 + j]; fs.hist[lane * 8 + j] = 0u; sum += h[j]; }
+            unsigned run = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned t = __shfl_up_sync(0xFFFFFFFFu, run, o);
+                if (lane >= o) run += t;
+            }
+            run -= sum;
+            if ((int)run < want && want <= (int)(run + sum)) {  // one lane
+                bool found = false;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    if (!found && want <= (int)(run + h[j])) {
+                        found = true;
+                        const int bin = lane * 8 + j, all = above + (int)(run + h[j]);
+                        const int state = all <= kFastM ? 1 : shift == 0 ? 2 : 0;
+                        // the bin's lower edge where the k best are fenced off, else its upper one: it is the next window
+                        fs.base = state == 1 ? top - min(top, (uint32_t)((((u64)bin + 1) << shift) - 1)) : top - ((uint32_t)bin << shift);
+                        fs.want = want - (int)run;
+                        fs.above = above + (int)run;
+                        fs.state = state;
+                    }
+                    run += found ? 0u : h[j];
+                }
+            }
+        }
+        __syncthreads();
+        const int state = fs.state;
+        if (state == 2) return false;  // more than kFastM candidates of one value at the cut
+        top = fs.base;
+        want = fs.want;
+        above = fs.above;
+        shift = max(shift - 8, 0);  // 256 bins inside that one
+        pass = state == 1 ? kTake : kBinned;
+    }
+    __syncthreads();
+    const int m = fs.n;
+    const float inv_t = rp.temperature == 1.0f ? 1.0f : __fdiv_rn(1.0f, rp.temperature);
+    const float mx = __fmul_rn(unord32(hi), inv_t);
+    for (int i = tid; i < m; i += kThreads) {
+        const u64 x = fs.best[i];
+        const int tok = fs.tok[i];
+        int rank = 0, same = 0;
+#pragma unroll 4
+        for (int j = 0; j < m; j++) {
+            const u64 y = fs.best[j];
+            rank += y > x ? 1 : 0;
+            same += y == x ? 1 : 0;
+        }
+        if (same > 1) {  // equal raw logits, equally penalised
+#pragma unroll 1
+            for (int j = 0; j < m; j++) rank += fs.best[j] == x && fs.tok[j] < tok ? 1 : 0;
+        }
+        if (rank < k) {
+            const float v = unord32((uint32_t)(x >> 32));
+            fs.vals[rank] = v;
+            fs.ids[rank] = tok;
+            fs.probs[rank] = isinf(v) && v < 0.f ? 0.f : (float)exp((double)__fsub_rn(__fmul_rn(v, inv_t), mx));
+        }
+    }
+    __syncthreads();
+    if (warp == 0) fast_draw(fs, rp, uniform, out);
+    __syncthreads();
+#pragma unroll 1
+    for (int t = tid; t < k; t += kThreads) {
         if (o_ids) o_ids[t] = fs.ids[t];
         if (o_vals) o_vals[t] = fs.vals[t];
         if (o_probs) o_probs[t] = fs.probs[t];
