@@ -11,7 +11,6 @@ namespace stg {
 
 struct FlatShared {
     FinishOut fout;
-    int ok;
 };
 
 // Rows the short finish does not take: a large top_k, a penalty that can raise a logit, and the second chance of a
@@ -148,15 +147,15 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
     // 47.2 -> 45.5.
     pdl_wait();
     tick(tk, 0);
-    if (threadIdx.x == 0) {
-        const FlatRow f = fr[row];
-        fs.ok = (f.cnt >= rp.sel && f.cnt <= f.cap && f.tau > -CUDART_INF_F) ? f.cnt : -1;
-    }
-    __syncthreads();
-    const int cnt = fs.ok;
+    u64 ahead[kFastU];  // within the list's capacity, however long it is
+    static_assert(kFastU * kThreads <= kFlatSlack, "a list has room for more");
+#pragma unroll
+    for (int q = 0; q < kFastU; q++) ahead[q] = fast ? __ldcg(a.cand + rp.cand_off + q * kThreads + threadIdx.x) : 0ull;
+    const int n_cand = __ldcg(&fr[row].cnt);
+    const int cnt = n_cand >= rp.sel && n_cand <= fr[row].cap && fr[row].tau > -CUDART_INF_F ? n_cand : -1;
     // a list that holds the N best (and, with no penalty that raises a logit, may hold any number more)
     if (fast && cnt > 0 &&
-        finish_fast(a.cand + rp.cand_off, cnt, rp, ptab, u, arena, (size_t)cap * 16, &fs.fout,
+        finish_fast(a.cand + rp.cand_off, ahead, cnt, rp, ptab, u, arena, (size_t)cap * 16, &fs.fout,
                     a.topk_ids ? a.topk_ids + o : nullptr, a.topk_logits ? a.topk_logits + o : nullptr,
                     a.topk_probs ? a.topk_probs + o : nullptr)) {
         tick(tk, 4);

@@ -17,6 +17,7 @@ namespace stg {
 constexpr int kFastK = 256;       // largest top_k
 constexpr int kFastM = 512;       // candidates put in order at most
 constexpr int kFastRoom = 1024;   // candidates there is room for at least
+constexpr int kFastU = kThreads >= 512 ? 2 : 3;  // candidates a thread takes at a time
 
 struct FastShared {
     float vals[256], probs[256], pre[256];
@@ -192,12 +193,13 @@ __device__ __forceinline__ void fast_penalise(const u64 (&key)[U], uint32_t (&pv
 
 // One CTA, all threads, behind finish_fast_begin; `list`: cnt keys in device memory, `arena`: shared memory, the FastShared, the
 // history's hash, then 12 bytes per candidate; a list that does not fit is read and penalised again in every pass.
-// False: nothing was written, the general path has to do the row.
-__device__ __forceinline__ bool finish_fast(const u64 *list, int cnt, const RowPlan &rp, const float *pow_tab, float uniform,
+// False: nothing was written, the general path has to do the row.  `ahead`: entries tid + q kThreads of the list, loaded before
+// its length was known.
+__device__ __forceinline__ bool finish_fast(const u64 *list, const u64 (&ahead)[kFastU], int cnt, const RowPlan &rp, const float *pow_tab, float uniform,
                                             unsigned char *arena, size_t arena_bytes, FinishOut *out, int32_t *o_ids, float *o_vals,
                                             float *o_probs)
 {
-    constexpr int U = 4;
+    constexpr int U = kFastU;
     FastShared &fs = *(FastShared *)arena;
     static_assert(sizeof(FastShared) % 16 == 0, "what follows is aligned");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = rp.top_k, hslots = fast_hash_slots(rp);
@@ -238,7 +240,7 @@ __device__ __forceinline__ bool finish_fast(const u64 *list, int cnt, const RowP
 #pragma unroll
                 for (int q = 0; q < U; q++) {
                     const int i = b + q * kThreads + tid;
-                    key[q] = i < cnt ? __ldcg(list + i) : 0ull;
+                    key[q] = i >= cnt ? 0ull : b == 0 ? ahead[q] : __ldcg(list + i);
                     pv[q] = (uint32_t)(key[q] >> 32);
                 }
                 if (rp.has_penalty) fast_penalise<U>(key, pv, hkey, hcnt, hslots - 1, rp, pow_tab);
@@ -313,16 +315,11 @@ __device__ __forceinline__ bool finish_fast(const u64 *list, int cnt, const RowP
     for (int i = tid; i < m; i += kThreads) {
         const u64 x = fs.best[i];
         const int tok = fs.tok[i];
-        int rank = 0, same = 0;
-#pragma unroll 4
-        for (int j = 0; j < m; j++) {
+        int rank = 0;
+#pragma unroll 8
+        for (int j = 0; j < m; j++) {  // no branches: bf16 logits tie in droves
             const u64 y = fs.best[j];
-            rank += y > x ? 1 : 0;
-            same += y == x ? 1 : 0;
-        }
-        if (same > 1) {  // equal raw logits, equally penalised
-#pragma unroll 1
-            for (int j = 0; j < m; j++) rank += fs.best[j] == x && fs.tok[j] < tok ? 1 : 0;
+            rank += (int)(y > x) | ((int)(y == x) & (int)(fs.tok[j] < tok));
         }
         if (rank < k) {
             const float v = unord32((uint32_t)(x >> 32));
