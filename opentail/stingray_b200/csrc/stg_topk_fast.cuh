@@ -6,7 +6,9 @@
 // order by counting, each by a thread, which also computes its exp; then one warp runs the filters and the draw of
 // Sampler.cs:296-349.  Equal values share a bin, so ties at the k-th are all there to be ordered.
 //
-// Bound: latency of a dozen dependent steps, six block barriers.
+// Bound: latency of a dozen dependent steps, six block barriers: 6 us for a lone row of 549 candidates (2.4 of them the loads and
+// the history's lookups, 1.4 the ranks and exps, 1.3 the draw), 11 where four CTAs share an SM.  A register sort of every
+// warp's share and a tree of merges in its place: 16 there, and 96 rows of bf16 logits took 45.5 us a step, now 34.8.
 #pragma once
 #include <math_constants.h>
 
