@@ -737,6 +737,10 @@ __device__ __forceinline__ void plan_bins(RowSh &sh, unsigned char *dyn, float t
     __syncthreads();
     const int c_lo = max(sh.cut_lo, 0);
     const bool open = sh.cut_lo < 0;  // the mass never reaches top_p: every survivor stays
+    // How near top_p a bin's sums have to lie for its elements to be handed over with the first.  Of a top_p near 1 they all do,
+    // tens of thousands of them: there the bin in which the exact sum meets top_p is asked for when it is known (4 of 14 such
+    // rows, of top_p 0.9998 and above, are no longer redone, which takes 0.8 to 6 ms).
+    const double near = fmin(1.0 / 16384.0, (1.0 - tp) / 64.0);
     double before = im - tm;
     int ac = ic - tc;
     uint32_t eb[2] = {0u, 0u};
@@ -746,7 +750,7 @@ __device__ __forceinline__ void plan_bins(RowSh &sh, unsigned char *dyn, float t
         // the estimate is good to some 1e-5, and the sum to come drifts by as much
         const double lo = before * (1.0 - 1.0 / 16384.0), hi = (before + lm[j]) * (1.0 + 1.0 / 16384.0);
         const int e_lo = exp_of_double(lo);
-        const bool order = lc[j] > 0 && (e_lo != exp_of_double(hi) || (lo <= tp && hi >= tp));
+        const bool order = lc[j] > 0 && (e_lo != exp_of_double(hi) || (before * (1.0 - near) <= tp && (before + lm[j]) * (1.0 + near) >= tp));
         const uint32_t v = b < c_lo ? 0u : (order ? (uint32_t)kBinOrder : (uint32_t)e_lo);
         eb[(7 - j) >> 2] |= v << (8 * ((7 - j) & 3));
         before += lm[j];

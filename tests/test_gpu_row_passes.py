@@ -94,3 +94,15 @@ def test_top_k_at_the_sizes_of_the_register_sort(top_k, rows):
     p["repetition_penalty"] = np.resize([1.0, 1.1, 1.25], rows)
     p["presence_penalty"] = np.resize([0.25, 0.0, 0.5, 0.125], rows)
     _run(x, p, hist, max_top_k=512)
+
+
+def test_top_p_next_to_one():
+    """The cut lies where the sorted sum is nearly flat: tens of thousands of tokens within the estimate's error of it."""
+    from opentail.stingray_b200 import workloads as W
+
+    rows, vocab = 12, 151_936
+    rng = np.random.default_rng(21)
+    p = W._params(rows)
+    p["temperature"] = np.resize([0.7, 1.1, 0.4], rows)
+    p["top_p"] = np.resize([0.9997, 0.9999, 0.99995, 0.99999, 0.999999], rows)
+    _run(rng.normal(0, 2.5, (rows, vocab)).astype(np.float32), p)
