@@ -524,26 +524,15 @@ __device__ __forceinline__ void guess_tiles(RowSh &sh, const TilePrefix &p, int 
     __syncthreads();
 }
 
-// One warp: the composition of tile t (8 elements per lane in x, their sum about `ts`) under its guess, or what its kind
-// asks for, into rank 0's walk area.
-__device__ __forceinline__ void compose_tile(const RowSh &sh, WalkArea *wa, WalkArea *dst, const float x[8], int t, int t0, float ts)
+// One warp: the composition of tile t (8 elements per lane in x) under its guess, or what its kind asks for, into rank 0's
+// walk area.
+__device__ __forceinline__ void compose_tile(const RowSh &sh, WalkArea *wa, WalkArea *dst, const float x[8], int t, int t0)
 {
     const int lane = threadIdx.x & 31;
     const int k = sh.kind[t - t0], g = sh.guess[t - t0];
     int a0 = 0, a1 = 0;
     if (k == kTileRun) {
-        if (g >= 48 && g < 250 && ts < __uint_as_float((uint32_t)(g - 2) << 23)) {
-            tile_composite(x, g, a0, a1);
-        } else {
-            float any = x[0];
-#pragma unroll
-            for (int j = 1; j < 8; j++) any = fmaxf(any, x[j]);
-            if (__any_sync(0xFFFFFFFFu, any > 0.f)) {
-                const int2 r = composite_any(lane8(x), g);
-                a0 = r.x;
-                a1 = r.y;
-            }
-        }
+        tile_composite(x, g, a0, a1);
     } else if (k != kTileReplay || t == 0) {
         WalkCross *c = &dst->xs[k >= kTileSlot ? (k - kTileSlot) % (kWalkCross + 1) : k - 1];
         if (t != 0) {
@@ -579,7 +568,7 @@ __device__ __forceinline__ void summarise(RowSh &sh, WalkArea *wa, WalkArea *dst
     guess_tiles(sh, p, t0, t1, base * scale, scale, all * scale, target);
     for_tiles(t0 + (int)(threadIdx.x >> 5), t1, kRW, load, [&](int t, float (&x)[8]) {
         map(t, x);
-        compose_tile(sh, wa, dst, x, t, t0, sh.tile_sum[t - t0] * (float)scale);
+        compose_tile(sh, wa, dst, x, t, t0);
     });
     __syncthreads();
     runs_of_tiles(sh, wa, dst, t0, t1);
@@ -1349,7 +1338,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
 #pragma unroll
             for (int j = 0; j < 8; j++) x[j] = b + j < n ? expf(__fsub_rn(x[j], mx)) : 0.f;
             store_e(e, b, x);
-            compose_tile(sh, wa, dst, x, t, t0, sh.tile_sum[t - t0]);
+            compose_tile(sh, wa, dst, x, t, t0);
             if (want_topp && small_table) to_bins(x);
         }
     } else {
@@ -1370,7 +1359,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
 #pragma unroll
             for (int j = 0; j < 8; j++) x[j] = expf(__fsub_rn(x[j], mx));  // 0 beyond the row, whose logits read as -inf
             store_e(e, at, x);
-            compose_tile(sh, wa, dst, x, t, t0, sh.tile_sum[t - t0] * own);
+            compose_tile(sh, wa, dst, x, t, t0);
             if (want_topp && small_table) to_bins(x);
         }
     }

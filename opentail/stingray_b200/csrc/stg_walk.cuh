@@ -297,29 +297,47 @@ __device__ __forceinline__ int walk_kind(int t, int g, int g_next, int g_end)
     return g_next == g + 1 ? 1 + slot : kTileSlot + slot;
 }
 
-// composition of a tile (8 consecutive elements per lane) under binade g; every lane gets it.  The sum of the
-// tile is below 0.49 * 2^(g - 127) and g >= 48: adding 1.5 * 2^(g - 127) then rounds every element to the
-// unit of the running sum, to even on a tie, in one addition.
+__device__ __forceinline__ float max_or_nan(float a, float b)
+{
+    float y;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
+}
+
+// composition of a tile (8 consecutive elements per lane) under binade g; every lane gets it.  Where g >= 48 and no element
+// reaches 2^(g - 128), half of the binade, adding 1.5 * 2^(g - 127) rounds each of them to the unit of the running sum, to even
+// on a tie, in one addition.  Both are asked of the elements themselves: what a tile weighs is known beforehand, but only
+// about (estimate_tile, stg_row.cu), and an element too large for its guess has other increments than the addition shows.
 __device__ __forceinline__ void tile_composite(const float x[8], int g, int &r0, int &r1)
 {
-    const float c = __uint_as_float(((uint32_t)g << 23) | 0x400000u);
-    unsigned a = 0u;  // modulo 2^32
-    float m = 0.f;
+    if (g >= 48 && g < 250) {
+        const float c = __uint_as_float(((uint32_t)g << 23) | 0x400000u);
+        unsigned a = 0u;  // modulo 2^32
+        float m = 0.f, top = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {  // two elements to an instruction
-        const float2 v = make_float2(x[j], x[j + 1]), y = __fadd2_rn(v, make_float2(c, c)), z = __fadd2_rn(y, make_float2(-c, -c));
-        const float2 w = __ffma2_rn(z, make_float2(-1.f, -1.f), v);
-        a += __float_as_uint(y.x) + __float_as_uint(y.y);
-        m = fmaxf(m, fmaxf(fabsf(w.x), fabsf(w.y)));
+        for (int j = 0; j < 8; j += 2) {  // two elements to an instruction
+            const float2 v = make_float2(x[j], x[j + 1]), y = __fadd2_rn(v, make_float2(c, c)), z = __fadd2_rn(y, make_float2(-c, -c));
+            const float2 w = __ffma2_rn(z, make_float2(-1.f, -1.f), v);
+            a += __float_as_uint(y.x) + __float_as_uint(y.y);
+            m = fmaxf(m, fmaxf(fabsf(w.x), fabsf(w.y)));
+            top = max_or_nan(top, max_or_nan(y.x, y.y));
+        }
+        a -= 8u * __float_as_uint(c);
+        const bool odd = m == __uint_as_float((uint32_t)(g - 24) << 23) || !(top < __uint_as_float((uint32_t)(g + 1) << 23));
+        if (__ballot_sync(0xFFFFFFFFu, odd) == 0u) {
+            r0 = r1 = min((int)__reduce_add_sync(0xFFFFFFFFu, a), 1 << 28);  // at most 2^30, and two of them are to be added (sat_add)
+            return;
+        }
     }
-    a -= 8u * __float_as_uint(c);
-    if (__ballot_sync(0xFFFFFFFFu, m == __uint_as_float((uint32_t)(g - 24) << 23)) == 0u) {
-        r0 = r1 = (int)__reduce_add_sync(0xFFFFFFFFu, a);
-        return;
+    float any = x[0];
+#pragma unroll
+    for (int j = 1; j < 8; j++) any = fmaxf(any, x[j]);
+    r0 = r1 = 0;
+    if (__any_sync(0xFFFFFFFFu, any > 0.f)) {
+        const int2 r = composite_any(lane8(x), g);
+        r0 = r.x;
+        r1 = r.y;
     }
-    const int2 r = composite_any(lane8(x), g);
-    r0 = r.x;
-    r1 = r.y;
 }
 
 }  // namespace stg

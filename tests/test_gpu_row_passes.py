@@ -106,3 +106,119 @@ def test_top_p_next_to_one():
     p["temperature"] = np.resize([0.7, 1.1, 0.4], rows)
     p["top_p"] = np.resize([0.9997, 0.9999, 0.99995, 0.99999, 0.999999], rows)
     _run(rng.normal(0, 2.5, (rows, vocab)).astype(np.float32), p)
+
+
+# ---- temperatures so small that neighbouring logits lie far apart, or fall together, once scaled -------------------------------
+
+SMALL_T = [1e-7, 3e-7, 5e-7, 7e-7, 1e-6]
+# a softmax sum that is off by a tenth shows in where these cut; Normalize hides it from the probabilities themselves
+CUTS = [0.9, 0.35, 0.7, 1.0, 0.55]
+
+
+def _near_maximum(rng, temperature, count):
+    """(A, B, maximum) triples whose exp values are other than their distance in the unscaled logits says: behind A alone the
+    sum is in the binade expected, B looks like less than a quarter of that binade and is half of it or more."""
+    inv = np.float32(1.0) / np.float32(temperature)
+    m = rng.uniform(15.0, 31.0, 8000).astype(np.float32)
+    found = []
+    for i, j in ((0, 1), (1, 2), (2, 3)):  # units of A and B below the maximum
+        a, b = ((m.view(np.uint32) - np.uint32(k)).view(np.float32) for k in (i, j))
+        real = [np.exp((v * inv).astype(np.float64) - (m * inv)) for v in (a, b)]
+        seen = [np.exp((v.astype(np.float64) - m) * float(inv)) for v in (a, b)]
+        with np.errstate(divide="ignore"):
+            g = np.floor(np.log2(seen[0]))
+            hit = (np.floor(np.log2(real[0])) == g) & (real[1] >= 2.0 ** (g - 1)) & (seen[1] < 2.0 ** (g - 2)) & (real[0] > 1e-4)
+        found += [(a[t], b[t], m[t]) for t in np.flatnonzero(hit)[:count]]
+    assert len(found) >= count
+    return [found[t] for t in rng.permutation(len(found))[:count]]
+
+
+def _near_rows(temperature, rows, vocab, seed=31):
+    rng = np.random.default_rng(seed)
+    x = rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)
+    for r, (a, b, m) in enumerate(_near_maximum(rng, temperature, rows)):
+        x[r, 100] = a
+        x[r, 256 * int(rng.integers(2, vocab // 512)) + int(rng.integers(0, 256))] = b
+        x[r, 256 * int(rng.integers(vocab // 512, vocab // 256)) + int(rng.integers(0, 256))] = m
+    return x
+
+
+@pytest.mark.parametrize("temperature", SMALL_T)
+@pytest.mark.parametrize("vocab", [32_000, 151_936])
+def test_near_the_maximum_at_small_temperatures(temperature, vocab):
+    from opentail.stingray_b200 import workloads as W
+
+    rows = 24
+    p = W._params(rows)
+    p["temperature"] = temperature
+    p["top_p"] = np.resize(CUTS, rows)
+    _run(_near_rows(temperature, rows, vocab), p)
+
+
+def test_near_the_maximum_behind_penalties():
+    """bf16 logits that a repetition penalty leaves one unit away from unpenalised ones (31.875 / 1.2 beside 26.5625), at
+    temperatures that make the two equal."""
+    from opentail.stingray_b200 import workloads as W
+
+    rows, vocab = 24, 32_000
+    rng = np.random.default_rng(33)
+    x = rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)
+    p = W._params(rows)
+    p["repeat_last_n"] = 0
+    p["top_p"] = np.resize(CUTS, rows)
+    hist = []
+    bf16 = (np.arange(0x4180, 0x4280, dtype=np.uint32) << 16).view(np.float32)  # 16 .. 64
+    for r in range(rows):
+        rep = np.float32([1.05, 1.2, 1.3][r % 3])
+        q = bf16 / rep
+        plain = ((q.view(np.uint32) + 0x7FFF) >> 16 << 16).view(np.float32)
+        pick = rng.choice(np.flatnonzero((np.abs(q.view(np.int32) - plain.view(np.int32)) == 1) & (q > 14.0)))
+        t = rng.uniform(1e-7, 1e-6, 1000).astype(np.float32)
+        inv = np.float32(1.0) / t
+        t = t[(q[pick] * inv == plain[pick] * inv) & (abs(float(q[pick]) - float(plain[pick])) * inv > 2.0)][0]
+        p["repetition_penalty"][r], p["temperature"][r] = rep, t
+        # the larger one in tile 0 and near the row's end, the smaller one in between
+        low = 256 * int(rng.integers(2, 60)) + int(rng.integers(0, 256))
+        high = np.array([100, 256 * int(rng.integers(61, vocab // 256)) + int(rng.integers(0, 256))])
+        pen, raw = (np.array([low]), high) if q[pick] < plain[pick] else (high, np.array([low]))
+        x[r, pen], x[r, raw] = bf16[pick], plain[pick]
+        hist.append(np.concatenate([pen, rng.integers(0, 50, 20)]))
+    _run(W.to_bf16_bits(x), p, hist)
+
+
+@pytest.mark.parametrize("temperature", SMALL_T)
+def test_distributions_near_the_maximum(temperature):
+    import torch
+    from opentail.stingray_b200 import BatchSampler, workloads as W
+    from oracle import oracle as orc
+
+    rows, vocab = 12, 32_000
+    x = _near_rows(temperature, rows, vocab, seed=35)
+    p = W._params(rows)
+    p["temperature"] = temperature
+    p["top_p"] = np.resize(CUTS, rows)
+    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=1, max_top_k=8)
+    try:
+        u = torch.full((rows,), 0.7, device="cuda")
+        beside = bs.sample_with_distribution(torch.from_numpy(x).cuda(), p, uniforms=u)[1].cpu().numpy()
+        alone = bs.build_distribution(torch.from_numpy(x).cuda(), p).cpu().numpy()
+    finally:
+        bs.close()
+    for r in range(rows):
+        want = orc.build_filtered_distribution(x[r], orc.OrcParams(*[p[r][n].item() for n in p.dtype.names]))[0]
+        for got in (beside[r], alone[r]):
+            np.testing.assert_allclose(got, want, rtol=2e-5, atol=1e-30)
+
+
+@pytest.mark.parametrize("temperature", SMALL_T)
+def test_verification_near_the_maximum(temperature):
+    from opentail.stingray_b200 import workloads as W
+    from tests.test_gpu_spec_shard import _check_spec
+
+    n, L, vocab = 4, 2, 32_000
+    rng = np.random.default_rng(37)
+    rows = _near_rows(temperature, n * (2 * L + 1), vocab, seed=39)
+    target, draft = rows[: n * (L + 1)].reshape(n, L + 1, vocab), rows[n * (L + 1):].reshape(n, L, vocab)
+    p = W._params(n, temperature=temperature)
+    p["top_p"] = CUTS[:n]
+    _check_spec(W.SpecWorkload("near", target, draft, draft.argmax(2).astype(np.int32), p, rng.random((n, L + 2))))
