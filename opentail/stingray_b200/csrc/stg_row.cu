@@ -215,7 +215,11 @@ struct RowSrc {
     {
         if (scale) {
 #pragma unroll
-            for (int j = 0; j < 8; j++) x[j] = __fmul_rn(x[j], inv_t);
+            for (int j = 0; j < 8; j += 2) {  // two elements to an instruction
+                const float2 v = __fmul2_rn(make_float2(x[j], x[j + 1]), make_float2(inv_t, inv_t));
+                x[j] = v.x;
+                x[j + 1] = v.y;
+            }
         }
     }
 };
@@ -264,9 +268,13 @@ __device__ __forceinline__ float warp_sum_f(float v)
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
     return v;
 }
-// One warp: {maximum, sum of 2^((x - maximum) k2)} of a tile's elements (8 per lane), to *est, and the lane's maximum.  What the
-// tile will weigh against the row's maximum, before that is known: a guess, good to some 1e-6.
-__device__ __forceinline__ float estimate_tile(const float x[8], float k2, float2 *est)
+// One warp: {maximum, sum of exp(x - maximum)} of a tile's elements (8 per lane, scaled by 1 / T as the exp values will be), to *est,
+// and the lane's maximum.  What the tile will weigh against the row's maximum, before that is known: a guess, good to 1e-6
+// for what weighs something and 1e-5 for the rest.  Of the logits before they are scaled it is good for nothing where
+// 1 / T makes a unit of them large: at T = 1e-6 softmax sums were expected in the wrong binade, and 16 rows with logits
+// next to their maximum took 125 us instead of 76.
+constexpr float kLog2E = 1.44269504f;
+__device__ __forceinline__ float estimate_tile(const float x[8], float2 *est)
 {
     float m = x[0];
 #pragma unroll
@@ -275,7 +283,7 @@ __device__ __forceinline__ float estimate_tile(const float x[8], float k2, float
     float2 s2 = make_float2(0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {  // two elements to an instruction
-        const float2 v = __fmul2_rn(__fadd2_rn(make_float2(x[j], x[j + 1]), make_float2(-ref, -ref)), make_float2(k2, k2));
+        const float2 v = __fmul2_rn(__fadd2_rn(make_float2(x[j], x[j + 1]), make_float2(-ref, -ref)), make_float2(kLog2E, kLog2E));
         s2 = __fadd2_rn(s2, make_float2(exp2_approx(v.x), exp2_approx(v.y)));
     }
     const float s = warp_sum_f(s2.x + s2.y);
@@ -1128,11 +1136,10 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
     }
 
     // P1: the maximum, and for the tiles' sums of exp values estimates that need no maximum
-    const float k2 = src.inv_t * 1.44269504f;
     float2 *est = (float2 *)wa->comp;
     TilePrefix tp{0.0, 0.0, 0.0, 0.0};
     {
-        float best = -CUDART_INF_F, cmax = -CUDART_INF_F;  // cmax: unscaled, what the CTA's estimates are relative to
+        float best = -CUDART_INF_F, cmax = -CUDART_INF_F;  // cmax: what the CTA's estimates are relative to
         u64 key = 0ull, raw = 0ull;
         if (CLOSE && ids != nullptr) {
             float nx[8];
@@ -1183,8 +1190,8 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                 for (int j = 0; j < 8; j++)
                     if (x[j] > rbest) { rbest = x[j]; rbest_i = base + j; }
                 src.override_(x, base);
-                if (!greedy) cmax = fmaxf(cmax, estimate_tile(x, k2, est + t));
                 src.rescale(x);
+                if (!greedy) cmax = fmaxf(cmax, estimate_tile(x, est + t));
 #pragma unroll
                 for (int j = 0; j < 8; j++)
                     if (x[j] > best) { best = x[j]; best_i = base + j; }
@@ -1194,7 +1201,6 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
             raw = block_max_k(rbest_i >= 0 ? make_key(rbest, rbest_i) : 0ull, sh.red_k);
             cmax = block_max_f(cmax, sh.red_f);
         } else {
-            // unscaled: multiplying by 1 / T > 0 and rounding is monotonic, so the maximum is scaled at the end
             for (int t = t0 + warp; t < t1; t += 2 * kRW) {
                 float x[2][8];
                 unsigned bits[2];
@@ -1203,16 +1209,15 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                 const bool two = t + kRW < t1;
                 if (two) src.fetch(b1, x[1], bits[1]);
                 src.mask(x[0], bits[0], b0);
-                src.override_(x[0], b0);
-                cmax = fmaxf(cmax, estimate_tile(x[0], k2, est + t));
+                src.adjust(x[0], b0);
+                cmax = fmaxf(cmax, estimate_tile(x[0], est + t));
                 if (two) {
                     src.mask(x[1], bits[1], b1);
-                    src.override_(x[1], b1);
-                    cmax = fmaxf(cmax, estimate_tile(x[1], k2, est + t + kRW));
+                    src.adjust(x[1], b1);
+                    cmax = fmaxf(cmax, estimate_tile(x[1], est + t + kRW));
                 }
             }
             best = cmax = block_max_f(cmax, sh.red_f);
-            if (src.scale) best = __fmul_rn(best, src.inv_t);
             if (best > -CUDART_INF_F) key = make_key(best, 0);
         }
         if (!greedy && !(CLOSE && ids != nullptr)) {
@@ -1221,7 +1226,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                 const int i = 2 * tid + u;
                 if (t0 + i < t1) {
                     const float2 v = est[t0 + i];
-                    sh.tile_sum[i] = v.x > -CUDART_INF_F ? v.y * exp2_approx((v.x - cmax) * k2) : 0.f;
+                    sh.tile_sum[i] = v.x > -CUDART_INF_F ? v.y * exp2_approx((v.x - cmax) * kLog2E) : v.y;  // of nothing but -infinity 0
                 }
             }
             tp = tile_prefix(sh.tile_sum, t1 - t0, sh.red_d);
@@ -1289,7 +1294,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
             float x[8], acc = 0.f;
             load_e(e, b, x);
 #pragma unroll
-            for (int j = 0; j < 8; j++) acc += b + j < n ? exp2_approx((x[j] - mx) * 1.44269504f) : 0.f;
+            for (int j = 0; j < 8; j++) acc += b + j < n ? exp2_approx((x[j] - mx) * kLog2E) : 0.f;
             acc = warp_sum_f(acc);
             if (lane == 0) sh.tile_sum[t - t0] = acc;
         }
@@ -1304,7 +1309,7 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
         float cmax = -CUDART_INF_F;
         for (int r = 0; r < C; r++) cmax = fmaxf(cmax, sh.cmax[r]);
         for (int r = 0; r < C; r++) {
-            const float f = exp2_approx((sh.cmax[r] - cmax) * k2);
+            const float f = exp2_approx((sh.cmax[r] - cmax) * kLog2E);
             if (r == rank) { base = all; own = f; }
             all += sh.tot[0][r] * (double)f;
         }

@@ -222,3 +222,29 @@ def test_verification_near_the_maximum(temperature):
     p = W._params(n, temperature=temperature)
     p["top_p"] = CUTS[:n]
     _check_spec(W.SpecWorkload("near", target, draft, draft.argmax(2).astype(np.int32), p, rng.random((n, L + 2))))
+
+
+@pytest.mark.parametrize("top_p,min_p", [(1.0, 0.0), (0.9, 0.0), (0.9, 0.02)])
+def test_not_a_number_wherever_it_stands(top_p, min_p):
+    """A NaN logit among -infinities, a whole tile of them, and one among ordinary logits make the same of a row."""
+    import torch
+    from opentail.stingray_b200 import BatchSampler, workloads as W
+
+    rows, vocab = 16, 32_000
+    x = np.random.default_rng(4).normal(0, 2.5, (rows, vocab)).astype(np.float32)
+    x[:, 5120:5376] = x[:, 5400] = -np.inf
+    p = W._params(rows, temperature=0.8, top_p=top_p, min_p=min_p)
+    u = torch.from_numpy(W.uniforms24(np.random.default_rng(5), rows)).cuda()
+    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=1, max_top_k=8)
+    got = []
+    try:
+        for where in (slice(5400, 5401), slice(5200, 5201), slice(5120, 5376)):
+            y = x.copy()
+            y[:, where] = np.nan
+            out = bs.sample_rows(torch.from_numpy(y).cuda(), p, uniforms=u, want_probs=True)
+            got.append((out["tokens"].cpu().numpy(), out["probs"].cpu().numpy()))
+    finally:
+        bs.close()
+    for tokens, probs in got[1:]:
+        np.testing.assert_array_equal(tokens, got[0][0])
+        np.testing.assert_array_equal(probs, got[0][1])
