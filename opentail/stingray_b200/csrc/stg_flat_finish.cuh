@@ -155,7 +155,7 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
     const int cnt = n_cand >= rp.sel && n_cand <= fr[row].cap && fr[row].tau > -CUDART_INF_F ? n_cand : -1;
     // a list that holds the N best (and, with no penalty that raises a logit, may hold any number more)
     if (fast && cnt > 0 &&
-        finish_fast(a.cand + rp.cand_off, ahead, cnt, rp, ptab, u, arena, (size_t)cap * 16, &fs.fout,
+        finish_fast([&](int id) { return load_one<BF16>(rowp, id); }, a.cand + rp.cand_off, ahead, cnt, rp, ptab, u, arena, (size_t)cap * 16, &fs.fout,
                     a.topk_ids ? a.topk_ids + o : nullptr, a.topk_logits ? a.topk_logits + o : nullptr,
                     a.topk_probs ? a.topk_probs + o : nullptr)) {
         tick(tk, 4);
@@ -167,7 +167,7 @@ __device__ void flat_finish_row(const SampleArgs &a, FlatRow *fr, int row, int i
         }
         return;
     }
-    flat_finish_general<BF16>(a, fr, row, item, cap, arena, ctl, fs, rp, rowp, cnt);
+    flat_finish_general<BF16>(a, fr, row, item, cap, arena, ctl, fs, rp, rowp, fast ? -1 : cnt);
 }
 
 }  // namespace stg

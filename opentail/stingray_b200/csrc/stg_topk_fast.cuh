@@ -18,7 +18,6 @@ namespace stg {
 
 constexpr int kFastK = 256;       // largest top_k
 constexpr int kFastM = 512;       // candidates put in order at most
-constexpr int kFastRoom = 1024;   // candidates there is room for at least
 constexpr int kFastU = kThreads >= 512 ? 2 : 3;  // candidates a thread takes at a time
 
 struct FastShared {
@@ -116,7 +115,7 @@ __device__ __forceinline__ int fast_hash_slots(const RowPlan &rp)
 }
 __device__ __forceinline__ bool fast_eligible(const RowPlan &rp, size_t arena_bytes)
 {
-    return sizeof(FastShared) + (size_t)fast_hash_slots(rp) * 8 + kFastRoom * 12 <= arena_bytes && rp.top_k <= kFastK &&
+    return sizeof(FastShared) + (size_t)fast_hash_slots(rp) * 8 <= arena_bytes && rp.top_k <= kFastK &&
            (!rp.has_penalty || (rp.rep >= 1.0f && rp.pres >= 0.f && rp.freq >= 0.f));
 }
 
@@ -150,10 +149,10 @@ __device__ __forceinline__ void finish_fast_begin(const RowPlan &rp, const int32
 }
 
 // The penalised values of a warp's candidates (Sampler.cs:263-287), as ordered bits; key 0: none.  Whole warps call it, and the
-// warp leaves the lookup's loop together, when the last of its lanes is done: with a loop that each lane left by itself
-// the lane that had found its token stayed apart from the others through the shuffles behind it, and a warp's
-// candidates were lost (rows of 262,144 bf16 logits behind 700-token histories: once in 400 to 9,000 steps, a
-// `__syncwarp` notwithstanding).  A lane's keys are looked up side by side.
+// warp leaves the lookup's loop together, when the last of its lanes is done: with a loop that each lane left by itself a
+// warp's candidates were now and then lost in the register sort that followed then (rows of 262,144 bf16 logits behind
+// 700-token histories: once in 400 to 9,000 steps), for a reason that was not found.  A lane's keys are looked up side
+// by side.
 template <int U>
 __device__ __forceinline__ void fast_penalise(const u64 (&key)[U], uint32_t (&pv)[U], const int *hkey, const unsigned *hcnt, int hmask,
                                               const RowPlan &rp, const float *pow_tab)
@@ -193,11 +192,18 @@ __device__ __forceinline__ void fast_penalise(const u64 (&key)[U], uint32_t (&pv
     }
 }
 
+// penalised value << 32 | raw logit of a candidate there was no room for: the list holds its penalised value in the raw
+// logit's place, which raw(token) reads from the row again
+template <class Raw>
+__device__ __noinline__ u64 fast_reread(const Raw raw, u64 x) { return (x & ~0xFFFFFFFFull) | ord32(raw(key_idx(x))); }
+
 // One CTA, all threads, behind finish_fast_begin; `list`: cnt keys in device memory, `arena`: shared memory, the FastShared, the
-// history's hash, then 12 bytes per candidate; a list that does not fit is read and penalised again in every pass.
-// False: nothing was written, the general path has to do the row.  `ahead`: entries tid + q kThreads of the list, loaded before
-// its length was known.
-__device__ __forceinline__ bool finish_fast(const u64 *list, const u64 (&ahead)[kFastU], int cnt, const RowPlan &rp, const float *pow_tab, float uniform,
+// history's hash, then 12 bytes per candidate.  Of those that do not fit the penalised value goes back to the list, so that
+// all are looked up and penalised once.  (Penalised again in every pass: 300 rows behind 1,000 tokens took 193 us, and rows
+// of 1,500, whose hash leaves little room, took 1,100 on the general path.)  `ahead`: entries tid + q kThreads of the
+// list, loaded before its length was known.  False: nothing was written, the row has to be done from its logits.
+template <class Raw>
+__device__ __forceinline__ bool finish_fast(const Raw &raw, u64 *list, const u64 (&ahead)[kFastU], int cnt, const RowPlan &rp, const float *pow_tab, float uniform,
                                             unsigned char *arena, size_t arena_bytes, FinishOut *out, int32_t *o_ids, float *o_vals,
                                             float *o_probs)
 {
@@ -207,68 +213,65 @@ __device__ __forceinline__ bool finish_fast(const u64 *list, const u64 (&ahead)[
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, k = rp.top_k, hslots = fast_hash_slots(rp);
     const int *hkey = (const int *)(arena + sizeof(FastShared));
     const unsigned *hcnt = (const unsigned *)(hkey + hslots);
-    const int room = (int)((arena_bytes - sizeof(FastShared) - (size_t)hslots * 8) / 12);
-    const bool stored = cnt <= room;
-    if (cnt < k) return false;
+    const int room = (int)((arena_bytes - sizeof(FastShared) - (size_t)hslots * 8) / 12), held = min(cnt, room);
     u64 *pk = (u64 *)(arena + sizeof(FastShared) + (size_t)hslots * 8);  // penalised value << 32 | raw logit, ordered bits
     int *pt = (int *)(pk + room);
     if (tid < 256) fs.hist[tid] = 0u;
     if (tid < 8) fs.probs[(k + tid) & 255] = 0.f;  // behind the last, where the sums read
-    enum { kRange, kBinned, kTake };
-    int pass = kRange, shift = 0, want = k, above = 0;
-    uint32_t lo = 0xFFFFFFFFu, hi = 0u, top = 0u;
+    uint32_t lo = 0xFFFFFFFFu, hi = 0u;
+#pragma unroll 1
+    for (int b = 0; b < cnt; b += U * kThreads) {
+        u64 key[U];
+        uint32_t pv[U];
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+            const int i = b + q * kThreads + tid;
+            key[q] = i >= cnt ? 0ull : b == 0 ? ahead[q] : __ldcg(list + i);
+            pv[q] = (uint32_t)(key[q] >> 32);
+        }
+        if (rp.has_penalty) fast_penalise<U>(key, pv, hkey, hcnt, hslots - 1, rp, pow_tab);
+#pragma unroll
+        for (int q = 0; q < U; q++) {
+            const int i = b + q * kThreads + tid;
+            if (i < cnt) {
+                lo = min(lo, pv[q]);
+                hi = max(hi, pv[q]);
+                if (i < room) {
+                    pk[i] = (u64)pv[q] << 32 | (key[q] >> 32);
+                    pt[i] = key_idx(key[q]);
+                } else {
+                    __stcg(list + i, (u64)pv[q] << 32 | (uint32_t)key[q]);
+                }
+            }
+        }
+    }
+    {
+        const uint32_t l = __reduce_min_sync(0xFFFFFFFFu, lo), h = __reduce_max_sync(0xFFFFFFFFu, hi);
+        if (lane == 0) { fs.lo[warp] = l; fs.hi[warp] = h; }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; w++) { lo = min(lo, fs.lo[w]); hi = max(hi, fs.hi[w]); }
+    }
+    // A window of 256 bins from the largest value downwards, value v in bin (top - v) >> shift; then the same inside the bin that
+    // holds the k-th, until no more than kFastM candidates lie above its lower edge (to go on until 128 do gives nothing).
+    int shift = max(24 - __clz((int)(hi - lo)), 0), want = k, above = 0;
+    uint32_t top = hi;
+    // body(x, tok): x = penalised value << 32 | raw logit, of which the latter may be missing where it does not matter
+    auto for_all = [&](auto body) {
+#pragma unroll 1
+        for (int i = tid; i < held; i += kThreads) body(pk[i], pt[i], true);
+#pragma unroll 1
+        for (int i = held + tid; i < cnt; i += kThreads) {
+            const u64 x = __ldcg(list + i);
+            body(x, key_idx(x), false);
+        }
+    };
 #pragma unroll 1
     for (;;) {
-        auto visit = [&](u64 x, int tok, int i) {
-            const uint32_t v = (uint32_t)(x >> 32);
-            if (pass == kRange) {
-                lo = min(lo, v);
-                hi = max(hi, v);
-                if (stored) { pk[i] = x; pt[i] = tok; }
-            } else if (pass == kBinned) {
-                const uint32_t d = (top - v) >> shift;
-                if (v <= top && d < 256u) atomicAdd(&fs.hist[d], 1u);
-            } else if (v >= top) {
-                const int slot = atomicAdd(&fs.n, 1);
-                fs.best[slot] = x;
-                fs.tok[slot] = tok;
-            }
-        };
-        if (pass == kRange || !stored) {
-#pragma unroll 1
-            for (int b = 0; b < cnt; b += U * kThreads) {
-                u64 key[U];
-                uint32_t pv[U];
-#pragma unroll
-                for (int q = 0; q < U; q++) {
-                    const int i = b + q * kThreads + tid;
-                    key[q] = i >= cnt ? 0ull : b == 0 ? ahead[q] : __ldcg(list + i);
-                    pv[q] = (uint32_t)(key[q] >> 32);
-                }
-                if (rp.has_penalty) fast_penalise<U>(key, pv, hkey, hcnt, hslots - 1, rp, pow_tab);
-#pragma unroll
-                for (int q = 0; q < U; q++) {
-                    const int i = b + q * kThreads + tid;
-                    if (i < cnt) visit((u64)pv[q] << 32 | (key[q] >> 32), key_idx(key[q]), i);
-                }
-            }
-        } else {
-#pragma unroll 1
-            for (int i = tid; i < cnt; i += kThreads) visit(pk[i], pt[i], i);
-        }
-        if (pass == kTake) break;
-        if (pass == kRange) {
-            const uint32_t l = __reduce_min_sync(0xFFFFFFFFu, lo), h = __reduce_max_sync(0xFFFFFFFFu, hi);
-            if (lane == 0) { fs.lo[warp] = l; fs.hi[warp] = h; }
-            __syncthreads();
-#pragma unroll
-            for (int w = 0; w < kThreads / 32; w++) { lo = min(lo, fs.lo[w]); hi = max(hi, fs.hi[w]); }
-            // a window of 256 bins from the largest value downwards: value v in bin (top - v) >> shift
-            top = hi;
-            shift = max(24 - __clz((int)(hi - lo)), 0);
-            pass = kBinned;
-            continue;
-        }
+        for_all([&](u64 x, int, bool) {
+            const uint32_t v = (uint32_t)(x >> 32), d = (top - v) >> shift;
+            if (v <= top && d < 256u) atomicAdd(&fs.hist[d], 1u);
+        });
         __syncthreads();
         if (warp == 0) {
             if (lane == 0) { fs.state = 2; fs.n = 0; }
@@ -303,15 +306,25 @@ __device__ __forceinline__ bool finish_fast(const u64 *list, const u64 (&ahead)[
         }
         __syncthreads();
         const int state = fs.state;
-        if (state == 2) return false;  // more than kFastM candidates of one value at the cut
         top = fs.base;
+        if (state == 1) break;
+        if (state == 2) return false;  // more than kFastM candidates of one value at the cut
         want = fs.want;
         above = fs.above;
         shift = max(shift - 8, 0);  // 256 bins inside that one
-        pass = state == 1 ? kTake : kBinned;
     }
+    const u64 fence = (u64)top << 32;
+    for_all([&](u64 x, int tok, bool whole) {
+        if (x >= fence) {
+            const int slot = atomicAdd(&fs.n, 1);
+            if (slot < kFastM) {
+                fs.best[slot] = whole ? x : fast_reread(raw, (x & ~0xFFFFFFFFull) | (uint32_t)~tok);
+                fs.tok[slot] = tok;
+            }
+        }
+    });
     __syncthreads();
-    const int m = fs.n;
+    const int m = min(fs.n, kFastM);
     const float inv_t = rp.temperature == 1.0f ? 1.0f : __fdiv_rn(1.0f, rp.temperature);
     const float mx = __fmul_rn(unord32(hi), inv_t);
     for (int i = tid; i < m; i += kThreads) {

@@ -248,3 +248,56 @@ def test_not_a_number_wherever_it_stands(top_p, min_p):
     for tokens, probs in got[1:]:
         np.testing.assert_array_equal(tokens, got[0][0])
         np.testing.assert_array_equal(probs, got[0][1])
+
+
+# ---- the finish of the top-k rows: 8 rows take its 512-thread form, 300 the 256-thread form, 600 the full-size one ---------------
+
+
+@pytest.mark.parametrize("rows", [8, 300, 600])
+@pytest.mark.parametrize("length", [500, 1500, 1850])
+def test_top_k_candidate_lists_behind_long_histories(rows, length):
+    """Beside the hash of 1,025 tokens and more the 256-thread form has room for the values of some 3,500 candidates, in
+    registers and shared memory; the lists hold 2,000 to 9,000."""
+    from opentail.stingray_b200 import workloads as W
+
+    vocab = 32_000
+    rng = np.random.default_rng(length)
+    x = rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)
+    x[1::3] = np.round(x[1::3] * 16) / 16
+    p = W._params(rows, temperature=0.9, top_p=0.98, top_k=40, repeat_last_n=0)
+    p["repetition_penalty"] = np.resize([1.1, 1.0, 1.3], rows)
+    p["frequency_penalty"] = np.resize([0.0, 0.25], rows)
+    # every other history holds what would have been drawn
+    hist = [rng.integers(0, vocab, length) if r % 2 else rng.permutation(np.argsort(-x[r])[: 2 * length])[:length] for r in range(rows)]
+    _run(x, p, hist, max_top_k=64)
+
+
+def test_a_long_history_costs_no_second_selection():
+    """Rows whose hash leaves little room beside it were once selected anew from their lists, which took 5.7 times as long as
+    rows of two thirds of their history; here they may take twice as long."""
+    import torch
+    from opentail.stingray_b200 import BatchSampler, workloads as W
+
+    rows, vocab = 300, 32_000
+    rng = np.random.default_rng(41)
+    x = torch.from_numpy(rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)).cuda()
+    p = W._params(rows, temperature=0.9, top_p=0.98, top_k=40, repetition_penalty=1.1, repeat_last_n=0)
+    u = torch.from_numpy(W.uniforms24(rng, rows)).cuda()
+    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=2048, max_top_k=64)
+    best = {}
+    try:
+        for length in (1000, 1500):
+            kw = dict(history_ids=torch.from_numpy(rng.integers(0, vocab, rows * length).astype(np.int32)).cuda(),
+                      history_offsets=np.arange(rows + 1, dtype=np.int32) * length, uniforms=u)
+            out, times = None, []
+            for _ in range(20):
+                a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                a.record()
+                out = bs.sample_rows(x, p, out=out, **kw)
+                b.record()
+                torch.cuda.synchronize()
+                times.append(a.elapsed_time(b))
+            best[length] = min(times)
+    finally:
+        bs.close()
+    assert best[1500] < 2 * best[1000], best
