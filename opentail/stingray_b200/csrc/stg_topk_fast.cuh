@@ -31,7 +31,7 @@ struct FastShared {
     int shift;                 // bins of 2^shift values
     int want;                  // how many of the k best lie in the window
     int above;                 // candidates above the window
-    int state;                 // 0: another round, 1: fenced off, 2: too many equal values
+    int state;                 // 0: another round, 1: fenced off, 2: too many of one value
     int n, pad[2];
 };
 
@@ -254,8 +254,10 @@ __device__ __forceinline__ bool finish_fast(const Raw &raw, u64 *list, const u64
     }
     // A window of 256 bins from the largest value downwards, value v in bin (top - v) >> shift; then the same inside the bin that
     // holds the k-th, until no more than kFastM candidates lie above its lower edge (to go on until 128 do gives nothing).
-    int shift = max(24 - __clz((int)(hi - lo)), 0), want = k, above = 0;
-    uint32_t top = hi;
+    // Where more have one value at the cut, their raw logits are divided in the same way (`by` 1), and where those are
+    // equal too, their tokens (`by` 2), of which no two are the same.
+    int by = 0, shift = max(24 - __clz((int)(hi - lo)), 0), want = k, above = 0;
+    uint32_t top = hi, cut = 0u, cut_raw = 0u;
     // body(x, tok): x = penalised value << 32 | raw logit, of which the latter may be missing where it does not matter
     auto for_all = [&](auto body) {
 #pragma unroll 1
@@ -263,18 +265,21 @@ __device__ __forceinline__ bool finish_fast(const Raw &raw, u64 *list, const u64
 #pragma unroll 1
         for (int i = held + tid; i < cnt; i += kThreads) {
             const u64 x = __ldcg(list + i);
-            body(x, key_idx(x), false);
+            body(by == 0 ? x : fast_reread(raw, x), key_idx(x), by != 0);
         }
     };
+    // the value in question of a candidate at the cut
+    auto value = [&](u64 x, int tok) { return by == 0 ? (uint32_t)(x >> 32) : by == 1 ? (uint32_t)x : ~(uint32_t)tok; };
+    auto at_cut = [&](u64 x) { return by == 0 || ((uint32_t)(x >> 32) == cut && (by == 1 || (uint32_t)x == cut_raw)); };
 #pragma unroll 1
     for (;;) {
-        for_all([&](u64 x, int, bool) {
-            const uint32_t v = (uint32_t)(x >> 32), d = (top - v) >> shift;
-            if (v <= top && d < 256u) atomicAdd(&fs.hist[d], 1u);
+        for_all([&](u64 x, int tok, bool) {
+            const uint32_t v = value(x, tok), d = (top - v) >> shift;
+            if (at_cut(x) && v <= top && d < 256u) atomicAdd(&fs.hist[d], 1u);
         });
         __syncthreads();
         if (warp == 0) {
-            if (lane == 0) { fs.state = 2; fs.n = 0; }
+            if (lane == 0) { fs.state = 3; fs.n = 0; }
             __syncwarp();
             unsigned h[8], sum = 0u;
 #pragma unroll
@@ -308,14 +313,21 @@ __device__ __forceinline__ bool finish_fast(const Raw &raw, u64 *list, const u64
         const int state = fs.state;
         top = fs.base;
         if (state == 1) break;
-        if (state == 2) return false;  // more than kFastM candidates of one value at the cut
+        if (state == 3) return false;  // not met: the k-th lies in every window
         want = fs.want;
         above = fs.above;
         shift = max(shift - 8, 0);  // 256 bins inside that one
+        if (state == 2) {
+            if (by == 0) cut = top;
+            else cut_raw = top;
+            by++;
+            top = 0xFFFFFFFFu;
+            shift = 24;
+        }
     }
-    const u64 fence = (u64)top << 32;
+    const u64 fence = by == 0 ? (u64)top << 32 : (u64)cut << 32 | (by == 1 ? top : cut_raw);
     for_all([&](u64 x, int tok, bool whole) {
-        if (x >= fence) {
+        if (x >= fence && (by < 2 || x > fence || ~(uint32_t)tok >= top)) {
             const int slot = atomicAdd(&fs.n, 1);
             if (slot < kFastM) {
                 fs.best[slot] = whole ? x : fast_reread(raw, (x & ~0xFFFFFFFFull) | (uint32_t)~tok);

@@ -20,8 +20,10 @@ def _run(logits, params, hist=None, seed=5, max_top_k=8):
     w = W.SampleWorkload("s", np.ascontiguousarray(logits), params, W.uniforms24(rng, rows), ids, off, None)
     bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=2048, max_top_k=max_top_k)
     try:
-        stats = parity.compare(w, parity.run_gpu(bs, w, want_topk=int(params["top_k"].max())))
+        gpu = parity.run_gpu(bs, w, want_topk=int(params["top_k"].max()))
+        stats = parity.compare(w, gpu)
         assert stats["mismatch"] == stats["boundary_draws"] <= 1
+        return gpu["flags"].view(np.uint32)
     finally:
         bs.close()
 
@@ -260,7 +262,7 @@ def test_top_k_candidate_lists_behind_long_histories(rows, length):
     registers and shared memory; the lists hold 2,000 to 9,000."""
     from opentail.stingray_b200 import workloads as W
 
-    vocab = 32_000
+    vocab = 16_640
     rng = np.random.default_rng(length)
     x = rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)
     x[1::3] = np.round(x[1::3] * 16) / 16
@@ -301,3 +303,26 @@ def test_a_long_history_costs_no_second_selection():
     finally:
         bs.close()
     assert best[1500] < 2 * best[1000], best
+
+
+@pytest.mark.parametrize("rows", [8, 300, 600])
+@pytest.mark.parametrize("lowered,plain", [(0, 2000), (600, 600), (300, 600), (20, 491)])
+def test_top_k_cut_among_equal_candidates(rows, lowered, plain):
+    """Around and beyond the 512 candidates that are put in order: `plain` logits of 6.5 and `lowered` ones of 7.0 that a
+    presence penalty makes equal to them, which come first; among equals the lower token does."""
+    from opentail.stingray_b200 import workloads as W
+
+    vocab = 16_640
+    rng = np.random.default_rng(lowered + plain)
+    x = np.minimum(rng.normal(0, 2.0, (rows, vocab)), 6.0).astype(np.float32)
+    hist = []
+    for r in range(rows):
+        t = rng.permutation(vocab)[: 10 + lowered + plain + 1300]
+        x[r, t[:10]] = 8.0 + np.arange(10) / 8
+        x[r, t[10:10 + plain]] = 6.5
+        x[r, t[10 + plain:10 + plain + lowered]] = 7.0
+        x[r, t[10 + plain + lowered:]] = -1.0
+        hist.append(t[10 + plain:])
+    p = W._params(rows, temperature=0.9, top_p=1.0, top_k=40, presence_penalty=0.5, repeat_last_n=0)
+    # (of some rows in a hundred the list overflows, whose bound is the smallest of a few group maxima)
+    assert (_run(x, p, hist, max_top_k=64) >> 8 & 1).mean() < 0.05, "read a second time"
