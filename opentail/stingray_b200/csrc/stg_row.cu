@@ -1160,6 +1160,23 @@ __global__ void __launch_bounds__(kRT, 2) k_row(const __grid_constant__ SampleAr
                 const int at = first_id + tile_at[t - t0] + warp_scan_i(c) - c;
                 float *ep = e + at;
                 int32_t *ip = ids + at;
+                if (__reduce_max_sync(0xFFFFFFFFu, (unsigned)c) <= 2u) {  // few: one after the other (64 rows of 262,144 behind masks of 1 % 64 -> 58 us)
+                    unsigned left = bits;
+#pragma unroll 1
+                    while (__any_sync(0xFFFFFFFFu, left != 0u)) {
+                        const int j = __ffs(left) - 1;
+                        float v = x[0];
+#pragma unroll
+                        for (int q = 1; q < 8; q++) v = q == j ? x[q] : v;
+                        if (left) {
+                            best = fmaxf(best, v);
+                            *ep++ = v;
+                            *ip++ = base + j;
+                            left &= left - 1u;
+                        }
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
                     const unsigned on = (bits >> j) & 1u;

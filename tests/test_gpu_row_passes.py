@@ -252,6 +252,32 @@ def test_not_a_number_wherever_it_stands(top_p, min_p):
         np.testing.assert_array_equal(probs, got[0][1])
 
 
+@pytest.mark.parametrize("vocab", [32_000, 50_257])
+def test_masks_of_a_few_tokens_per_lane(vocab):
+    """Rows closed up as they are read, eight tokens to a lane: none or one allowed in each, up to two (taken one after the
+    other), up to three and up to all of them (taken by predicate)."""
+    from opentail.stingray_b200 import BatchSampler, workloads as W
+
+    rows, words = 12, (vocab + 31) // 32
+    rng = np.random.default_rng(vocab)
+    allowed = np.zeros((rows, words * 32), bool)
+    for r in range(rows):
+        most = (1, 2, 3, 8)[r % 4]
+        pick = rng.permuted(np.tile(np.arange(8), (words * 4, 1)), axis=1)
+        n = rng.integers(0, most + 1, words * 4) * (rng.random(words * 4) < (0.02, 0.5, 1.0)[r % 3])
+        if r % 4 == 3:
+            n = np.where(rng.random(n.size) < 0.4, n, 0)
+        np.put_along_axis(allowed[r].reshape(-1, 8), pick, np.arange(8) < n[:, None], axis=1)
+    mask = np.packbits(allowed, axis=1, bitorder="little").view(np.uint32)
+    w = W.SampleWorkload("m", rng.normal(0, 2.5, (rows, vocab)).astype(np.float32), _params(rows), W.uniforms24(rng, rows), None, None, mask)
+    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=1, max_top_k=8)
+    try:
+        stats = parity.compare(w, parity.run_gpu(bs, w))
+        assert stats["mismatch"] == stats["boundary_draws"] <= 1
+    finally:
+        bs.close()
+
+
 # ---- the finish of the top-k rows: 8 rows take its 512-thread form, 300 the 256-thread form, 600 the full-size one ---------------
 
 
