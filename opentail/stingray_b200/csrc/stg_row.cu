@@ -735,9 +735,11 @@ __device__ __forceinline__ void plan_bins(RowSh &sh, unsigned char *dyn, float t
     const int c_lo = max(sh.cut_lo, 0);
     const bool open = sh.cut_lo < 0;  // the mass never reaches top_p: every survivor stays
     // How near top_p a bin's sums have to lie for its elements to be handed over with the first.  Of a top_p near 1 they all do,
-    // tens of thousands of them: there the bin in which the exact sum meets top_p is asked for when it is known (4 of 14 such
-    // rows, of top_p 0.9998 and above, are no longer redone, which takes 0.8 to 6 ms).
-    const double near = fmin(1.0 / 16384.0, (1.0 - tp) / 64.0);
+    // tens of thousands of them: there the bin in which the exact sum meets top_p is asked for when it is known, which takes
+    // another round over the row.  16 rows of 151,936, T = 1.1, with 2^-14 everywhere / (1 - top_p) / 16 / (1 - top_p) / 64: top_p
+    // 0.999 127 / 124 / 144 us, 0.9993 138 / 134 / 148, 0.9997 148 / 115 / 140, 0.9998 5,605 (all rows redone) / 199 / 193;
+    // T = 0.7: 0.999 117 / 113 / 103, 0.9993 130 / 119 / 128, 0.9997 172 / 138 / 126.
+    const double near = fmin(1.0 / 16384.0, (1.0 - tp) / 16.0);
     double before = im - tm;
     int ac = ic - tc;
     uint32_t eb[2] = {0u, 0u};

@@ -110,6 +110,17 @@ def test_top_p_next_to_one():
     _run(rng.normal(0, 2.5, (rows, vocab)).astype(np.float32), p)
 
 
+@pytest.mark.parametrize("top_p", [0.997, 0.999, 0.9995, 0.9997, 0.9998])
+def test_top_p_near_one_is_no_reason_to_redo_a_row(top_p):
+    from opentail.stingray_b200 import workloads as W
+
+    rows, vocab = 12, 151_936
+    p = W._params(rows, top_p=top_p)
+    p["temperature"] = np.resize([0.4, 0.7, 0.9, 1.1], rows)
+    flags = _run(np.random.default_rng(22).normal(0, 2.5, (rows, vocab)).astype(np.float32), p)
+    assert not (flags >> 8 & 1).any()
+
+
 # ---- temperatures so small that neighbouring logits lie far apart, or fall together, once scaled -------------------------------
 
 SMALL_T = [1e-7, 3e-7, 5e-7, 7e-7, 1e-6]
