@@ -118,6 +118,16 @@ __device__ __forceinline__ WalkOut row_walk(const WalkArea *w, const Get &get, i
         const uint32_t sb = __float_as_uint(o.s);
         const int eb = (int)(sb >> 23) & 255;  // the sum is >= 0
         if (eb == 255) break;                  // inf / NaN: nothing changes any more
+        if (sb == 0u) {
+            // Nothing yet: a run without a positive element leaves it so (under the lowest guess every positive one counts).
+            // Near-greedy rows are nothing else up to their maximum: 64 rows of 151,936 at T = 1e-5 516 -> 56 us.
+            const uint32_t d = w->desc[t];
+            const int2 v = w->tot[t];
+            if ((d & 0xFFFFu) == (1u | (kTileRun << 8)) && (v.x | v.y) == 0) {
+                t = (int)(d >> 16) + 1;
+                continue;
+            }
+        }
         int sint = (int)((sb & 0x7FFFFFu) | 0x800000u);
         bool replay = eb < 24;                 // sums that small have no summaries
         if (!replay) {
