@@ -4,7 +4,8 @@
 // in one 64-bit word, and its token.  The k best are fenced off by a histogram over the range of the penalised values, refined
 // inside the bin that holds the k-th until no more than kFastM candidates lie above its lower edge; those are put in
 // order by counting, each by a thread, which also computes its exp; then one warp runs the filters and the draw of
-// Sampler.cs:296-349.  Equal values share a bin, so ties at the k-th are all there to be ordered.
+// Sampler.cs:296-349.  Equal values share a bin, so ties at the k-th are all there to be ordered; more of them than that are
+// divided by their raw logits and tokens first.
 //
 // Bound: latency of a dozen dependent steps, six block barriers: 6 us for a lone row of 549 candidates (2.4 of them the loads and
 // the history's lookups, 1.4 the ranks and exps, 1.3 the draw), 11 where four CTAs share an SM.  A register sort of every

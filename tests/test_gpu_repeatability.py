@@ -61,9 +61,9 @@ def test_repeated_batches_in_random_order(own_stream):
 
 
 def test_penalised_top_k_rows_keep_every_candidate():
-    """Rows whose candidates are looked up in a long history and sorted in registers right behind that: three rows of the
-    sweep's batch 1, repeated.  Lanes that left the lookup one by one used to lose a warp's candidates once in
-    a few hundred to a few thousand steps."""
+    """Rows whose candidates are looked up in a long history: three rows of the sweep's batch 1, repeated.  With a lookup that
+    lanes left one by one, and a register sort behind it, a warp's candidates were lost once in a few hundred to a few
+    thousand steps."""
     import torch
     from opentail.stingray_b200 import BatchSampler, workloads as W
 
@@ -84,6 +84,39 @@ def test_penalised_top_k_rows_keep_every_candidate():
         for _ in range(10_000):
             out = bs.sample_rows(dev["logits"], w.params, out=out, **kw)
             differ += (out["topk_ids"] != first["topk_ids"]).any() | (out["probs"] != first["probs"]).any()
+        assert int(differ) == 0
+    finally:
+        bs.close()
+
+
+def test_full_rows_with_long_histories_repeat():
+    """Loops that lanes leave one by one ahead of warp-wide operations: the overrides of a lane's own tokens, and the rounding
+    ties of a wide nucleus.  Five thousand steps of rows full of both."""
+    import torch
+    from opentail.stingray_b200 import BatchSampler, workloads as W
+
+    rows, vocab, h = 6, 50_257, 1200
+    rng = np.random.default_rng(51)
+    x = rng.normal(0, 2.5, (rows, vocab)).astype(np.float32)
+    x[::2] = np.round(x[::2] * 8) / 8
+    p = W._params(rows, top_p=0.95, repetition_penalty=1.1, presence_penalty=0.25, repeat_last_n=0)
+    p["temperature"] = np.resize([1.0, 0.9, 1.2], rows)
+    # tokens side by side, so that a lane has several overrides
+    hist = np.concatenate([(rng.integers(0, vocab // 64, h) * 64 + rng.integers(0, 12, h)) % vocab for _ in range(rows)]).astype(np.int32)
+    w = W.SampleWorkload("s", x, p, W.uniforms24(rng, rows), hist, np.arange(rows + 1, dtype=np.int32) * h, None)
+    bs = BatchSampler(max_rows=rows, max_vocab=vocab, max_history=2048, max_top_k=8)
+    try:
+        dev = parity.to_device(w)
+        kw = dict(uniforms=dev["uniforms"], history_ids=dev["history_ids"], history_offsets=w.history_offsets,
+                  want_probs=True, want_flags=True)
+        out = bs.sample_rows(dev["logits"], w.params, **kw)
+        torch.cuda.synchronize()
+        parity.compare(w, {k: v.cpu().numpy() for k, v in out.items()})
+        first = {k: v.clone() for k, v in out.items()}
+        differ = torch.zeros(1, dtype=torch.int64, device="cuda")
+        for _ in range(5_000):
+            out = bs.sample_rows(dev["logits"], w.params, out=out, **kw)
+            differ += (out["tokens"] != first["tokens"]).any() | (out["probs"] != first["probs"]).any() | (out["flags"] != first["flags"]).any()
         assert int(differ) == 0
     finally:
         bs.close()

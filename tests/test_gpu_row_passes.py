@@ -79,9 +79,9 @@ def test_tiles_of_very_different_weight(vocab):
 
 @pytest.mark.parametrize("top_k", [63, 64, 127, 128, 255, 256])
 @pytest.mark.parametrize("rows", [8, 300])
-def test_top_k_at_the_sizes_of_the_register_sort(top_k, rows):
-    """Where the sort takes twice as many keys and the history's hash, filled ahead of the candidates, lies elsewhere: logits in
-    steps of 1/4, penalised in small steps, half of the tokens near the cut in the history."""
+def test_top_k_with_ties_and_penalties_around_the_cut(top_k, rows):
+    """Logits in steps of 1/4, penalised in small steps, 20 to 90 % of the tokens near the cut in the history; top_k up to the
+    largest the short finish takes."""
     from opentail.stingray_b200 import workloads as W
 
     vocab = 32_000
